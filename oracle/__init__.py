@@ -34,7 +34,7 @@ _D = ctypes.c_double
 def build(reference: bool = True) -> None:
     """Compile the restatement, and the reference shim when the reference sources exist."""
     subprocess.run(["make", "-s", "-C", str(HERE), "all"], check=True)
-    if reference and REFERENCE_SRC.is_dir():
+    if reference and (REFERENCE_SRC / "src" / "core" / "scene.cpp").is_file():
         subprocess.run(["make", "-s", "-C", str(HERE), "ref", f"REF={REFERENCE_SRC}"], check=True)
         # quarry's own callers against the engine's header and library (drop-in check); they
         # link libquarry_b200.so, so the engine is built first
