@@ -12,8 +12,8 @@
 //   reset headers -> centroid bounds -> 30-bit Morton codes (each in its scene's bounds)
 //   -> radix sort on the code (4 passes), then a stable sort on the scene index (1 pass):
 //      the scenes' slots come out contiguous, each in (code, index) order
-//   -> code / local-index gather -> Karras emit -> bottom-up boxes with atomic visit flags
-//   -> depths -> [4-wide: even-depth flags, one scan, per-scene rebase, emit]
+//   -> code / local-index gather -> block-boundary masks -> leaves, links, boxes and depths in
+//      one pass (qk_lbvh.cuh) -> [4-wide: even-depth flags, one scan, per-scene rebase, emit]
 //
 // Queries.  Persistent kernels: a grid of SMs x blocks_per_sm blocks whose warps take
 // `chunks_per_fetch` 32-query chunks at a time from a global counter until the chunk table
@@ -29,6 +29,7 @@
 
 #include "qk_build.cuh"
 #include "qk_internal.cuh"
+#include "qk_lbvh.cuh"
 #include "qk_traverse.cuh"
 
 namespace qk {
@@ -147,6 +148,7 @@ __global__ __launch_bounds__(kBlock) void k_bt_morton(const BScene* __restrict__
         const uint32_t code = spread10(quant(c.x, lx, hx - lx)) |
                               (spread10(quant(c.y, ly, hy - ly)) << 1) |
                               (spread10(quant(c.z, lz, hz - lz)) << 2);
+        if (i < sc.t.n - 1) sc.t.flags[i] = 0;  // the tree pass's arrival words
         const int j = sc.prim_off + i;
         codes[j] = code;
         keep[j] = code;
@@ -188,95 +190,66 @@ __global__ __launch_bounds__(kBlock) void k_bt_gather(const BScene* __restrict__
     }
 }
 
-// ranges: one int2 per primitive of the batch (scene s's internal nodes at prim_off(s)); the
-// emit writes every internal node's slot range (first, count)
+// A chunk holds kBuildChunk / kLbvhSpan blocks of the tree pass.  Their boundary masks sit at
+// half the first primitive's index in the batch (a block starts two or more primitives after
+// the one before it), 16 bytes each, so they fill at most 8 bytes per primitive.
+constexpr int kChunkSpans = kBuildChunk / kLbvhSpan;
+
+__device__ __forceinline__ LbvhView bt_view(const BScene& sc, const uint32_t* codes_f,
+                                            const uint32_t* ids_f) {
+    const qk_tree& t = sc.t;
+    LbvhView v;
+    v.items = sc.in;
+    v.codes = codes_f + sc.prim_off;
+    v.ids = ids_f + sc.prim_off;
+    v.n = t.n;
+    v.nodes = static_cast<Node*>(t.nodes);
+    v.sorted = static_cast<float*>(t.items);
+    v.prim_ids = t.prim_ids;
+    v.slot_of = t.slot_of;
+    v.parent = t.parent;
+    v.depth = t.depth_arr;
+    v.bnodes = static_cast<BNode*>(t.bnodes);
+    v.leaves = static_cast<float4*>(t.leaves);
+    v.flags = t.flags;
+    return v;
+}
+
+// one warp per block of the tree pass: the masks at its left boundary
+__global__ __launch_bounds__(32 * kChunkSpans) void k_bt_carry(const BScene* __restrict__ tab,
+                                                               const int2* __restrict__ chunks,
+                                                               const uint32_t* __restrict__ codes_f,
+                                                               const uint32_t* __restrict__ ids_f,
+                                                               LbvhCarry* __restrict__ carry) {
+    const int2 ch = chunks[blockIdx.x];
+    const BScene& sc = tab[ch.x];
+    const int base = ch.y + static_cast<int>(threadIdx.x >> 5) * kLbvhSpan;
+    const int lane = threadIdx.x & 31;
+    if (base >= sc.t.n) return;
+    unsigned long long left = 0, right = 0;
+    if (base > 0) lbvh_boundary(bt_view(sc, codes_f, ids_f), base, lane, left, right);
+    if (lane != 0) return;
+    const int at = (sc.prim_off + base) / 2;
+    carry[at].left = left;
+    if (base > 0) carry[(sc.prim_off + base - kLbvhSpan) / 2].right = right;
+    if (base + kLbvhSpan >= sc.t.n) carry[at].right = 0;
+}
+
+// blockIdx.x / kChunkSpans: the chunk
 template <class Ops>
-__global__ __launch_bounds__(kBlock) void k_bt_emit(const BScene* __restrict__ tab,
-                                                    const int2* __restrict__ chunks,
-                                                    const uint32_t* __restrict__ codes_f,
-                                                    const uint32_t* __restrict__ ids_f,
-                                                    int2* __restrict__ ranges) {
-    __shared__ __align__(16) float stage[kBlock / 32][emit_stage_floats<Ops>()];
-    const int2 ch = chunks[blockIdx.x];
+__global__ __launch_bounds__(kLbvhSpan, 4) void k_bt_tree(const BScene* __restrict__ tab,
+                                                          const int2* __restrict__ chunks,
+                                                          const uint32_t* __restrict__ codes_f,
+                                                          const uint32_t* __restrict__ ids_f,
+                                                          const LbvhCarry* __restrict__ carry,
+                                                          Header* __restrict__ hdr) {
+    __shared__ __align__(16) LbvhShared sh;
+    const int2 ch = chunks[blockIdx.x / kChunkSpans];
     const BScene& sc = tab[ch.x];
-    const qk_tree& t = sc.t;
-    const int n = t.n;
-    const int end = min(n, ch.y + kBuildChunk);
-    const uint32_t* codes = codes_f + sc.prim_off;
-    const uint32_t* ids = ids_f + sc.prim_off;
-    for (int k0 = ch.y + (threadIdx.x & ~31); k0 < end; k0 += kBlock) {  // whole warps
-        emit_leaves_warp<Ops>(sc.in, n, ids, static_cast<Node*>(t.nodes),
-                              static_cast<float*>(t.items), t.prim_ids, t.slot_of,
-                              static_cast<float4*>(t.leaves), k0, min(32, end - k0),
-                              stage[threadIdx.x >> 5]);
-        const int k = k0 + (threadIdx.x & 31);
-        if (k < end)
-            emit_internal(n, codes, ids, static_cast<Node*>(t.nodes), t.parent,
-                          static_cast<BNode*>(t.bnodes), t.flags, k, ranges + sc.prim_off);
-    }
-}
-
-// Bottom-up boxes of every scene: a chunk's block starts the climbs at its kBuildChunk leaf
-// slots, and nodes whose range lies inside the chunk meet in shared memory (climb_ranged).
-__global__ __launch_bounds__(kBlock) void k_bt_bottom_up(const BScene* __restrict__ tab,
-                                                         const int2* __restrict__ chunks,
-                                                         const int2* __restrict__ ranges) {
-    __shared__ int arrivals[kBuildChunk];
-    const int2 ch = chunks[blockIdx.x];
-    const BScene& sc = tab[ch.x];
-    const qk_tree& t = sc.t;
-    const int n = t.n;
-    const int end = min(n, ch.y + kBuildChunk);
-    for (int i = threadIdx.x; i < kBuildChunk; i += kBlock) arrivals[i] = 0;
-    __syncthreads();
-    for (int k = ch.y + threadIdx.x; k < end; k += kBlock)
-        climb_ranged<kBuildChunk>(static_cast<Node*>(t.nodes), static_cast<BNode*>(t.bnodes),
-                                  t.parent, t.flags, n, k, ch.y, arrivals, ranges + sc.prim_off);
-}
-
-// depths in two passes, as the single-tree build (anchored_depth in qk_build.cuh): the
-// anchors of every chunk's internal nodes, then every other node and each scene's maximum
-__global__ __launch_bounds__(kBlock) void k_bt_depth_anchors(const BScene* __restrict__ tab,
-                                                             const int2* __restrict__ chunks,
-                                                             const int2* __restrict__ ranges_all) {
-    const int2 ch = chunks[blockIdx.x];
-    const BScene& sc = tab[ch.x];
-    const qk_tree& t = sc.t;
-    const int n = t.n;
-    const int2* ranges = ranges_all + sc.prim_off;
-    const int end = min(n - 1, ch.y + kBuildChunk);
-    for (int k = ch.y + threadIdx.x; k < end; k += kBlock)
-        if (depth_anchor(ranges, k, n)) t.depth_arr[k] = chain_depth(t.parent, k, 2 * n - 1);
-}
-
-__global__ __launch_bounds__(kBlock) void k_bt_depth(const BScene* __restrict__ tab,
-                                                     const int2* __restrict__ chunks,
-                                                     const int2* __restrict__ ranges_all,
-                                                     Header* __restrict__ hdr) {
-    const int2 ch = chunks[blockIdx.x];
-    const BScene& sc = tab[ch.x];
-    const qk_tree& t = sc.t;
-    const int n = t.n;
-    const int m = 2 * n - 1;
-    const int2* ranges = ranges_all + sc.prim_off;
-    const int end = min(n, ch.y + kBuildChunk);
-    int dmax = 0;
-    for (int k = ch.y + threadIdx.x; k < end; k += kBlock) {
-        if (k < n - 1) {
-            int d;
-            if (depth_anchor(ranges, k, n)) {
-                d = t.depth_arr[k];
-            } else {
-                d = anchored_depth(t.parent, ranges, t.depth_arr, n, k, m);
-                t.depth_arr[k] = d;
-            }
-            dmax = max(dmax, d);
-        }
-        const int d = anchored_depth(t.parent, ranges, t.depth_arr, n, n - 1 + k, m);
-        t.depth_arr[n - 1 + k] = d;
-        dmax = max(dmax, d);
-    }
-    block_max_to(dmax, &hdr[ch.x].max_depth);
+    const int base = ch.y + static_cast<int>(blockIdx.x % kChunkSpans) * kLbvhSpan;
+    if (base >= sc.t.n) return;  // the whole block
+    lbvh_block<Ops>(bt_view(sc, codes_f, ids_f), base, carry[(sc.prim_off + base) / 2],
+                    &hdr[ch.x].max_depth, sh);
 }
 
 __global__ __launch_bounds__(kBlock) void k_bt_wide_flags(const BScene* __restrict__ tab,
@@ -805,12 +778,11 @@ int batch_build_impl(qk_batch* b, cudaStream_t s) {
     // idx_f = codes_s; gather codes into codes, local ids into idx_s
     k_bt_gather<<<C, kBlock, 0, s>>>(b->d_tab, b->d_chunks, keep, codes_s, codes, idx_s);
     // keep and idx are free after the gather: their 2N uint32 (adjacent, 256-byte aligned) hold
-    // the N int2 slot ranges
-    int2* ranges = reinterpret_cast<int2*>(keep);
-    k_bt_emit<Ops><<<C, kBlock, 0, s>>>(b->d_tab, b->d_chunks, codes, idx_s, ranges);
-    k_bt_bottom_up<<<C, kBlock, 0, s>>>(b->d_tab, b->d_chunks, ranges);
-    k_bt_depth_anchors<<<C, kBlock, 0, s>>>(b->d_tab, b->d_chunks, ranges);
-    k_bt_depth<<<C, kBlock, 0, s>>>(b->d_tab, b->d_chunks, ranges, b->d_hdr);
+    // the boundary masks
+    auto* carry = reinterpret_cast<LbvhCarry*>(keep);
+    k_bt_carry<<<C, 32 * kChunkSpans, 0, s>>>(b->d_tab, b->d_chunks, codes, idx_s, carry);
+    k_bt_tree<Ops><<<C * kChunkSpans, kLbvhSpan, 0, s>>>(b->d_tab, b->d_chunks, codes, idx_s, carry,
+                                                         b->d_hdr);
     if (b->flags & QK_WIDE) {
         k_bt_wide_flags<<<C, kBlock, 0, s>>>(b->d_tab, b->d_chunks);
         e = scan_exclusive(b->flags_field, b->wide_id_field, static_cast<int>(b->flag_span), false,

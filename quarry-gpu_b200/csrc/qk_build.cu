@@ -5,20 +5,19 @@
 //   2. 30-bit Morton code of the quantized centroid, value = scene index
 //   3. stable radix sort on the code (equal codes keep index order = the reference's
 //      64-bit (code << 32 | index) key order)
-//   4. emit: one thread per slot writes the leaf (payload, canonical leaf node, prim id,
-//      inverse map) and, for slot < n-1, the internal node found by the Karras split
-//      search over the 64-bit keys
-//   5. bottom-up boxes in ONE launch: each leaf thread climbs its parent chain; an atomic
-//      visit counter per internal node lets the second arriving child compute the union
-//      (both children final) and carry on, the first one stops.  min/max is exact, so the
-//      boxes equal the reference's level-by-level refit bit for bit.  The same pass writes
-//      the 64-byte traversal node (both child boxes inline).
-//   6. depth of every node by walking its parent chain; the maximum is read back once.
+//   4. one pass over the leaves writes the leaf arrays and meets siblings bottom-up: links,
+//      boxes, traversal nodes, parents and depths (qk_lbvh.cuh).  min/max is exact, so the
+//      boxes equal the reference's level-by-level refit bit for bit.
+//
+// The SAH builder and topology edits bring their own links and leaves; their boxes come from a
+// climb of every leaf's parent chain on visit counters (the second arriving child computes the
+// union and carries on), their depths from the parent chains.
 #include <algorithm>
 #include <cstdio>
 
 #include "qk_internal.cuh"
 #include "qk_build.cuh"
+#include "qk_lbvh.cuh"
 
 namespace qk {
 
@@ -95,9 +94,11 @@ template <class Ops>
 __global__ __launch_bounds__(kBlock) void k_morton(const float* __restrict__ items, int n,
                                                    const Header* __restrict__ h,
                                                    uint32_t* __restrict__ codes,
-                                                   uint32_t* __restrict__ idx) {
+                                                   uint32_t* __restrict__ idx,
+                                                   int* __restrict__ flags) {
     const int i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= n) return;
+    if (i < n - 1) flags[i] = 0;  // the tree pass's arrival words
     const float lx = unord_f(h->lo[0]), ly = unord_f(h->lo[1]), lz = unord_f(h->lo[2]);
     const float hx = unord_f(h->hi[0]), hy = unord_f(h->hi[1]), hz = unord_f(h->hi[2]);
     const float3 c = Ops::centroid(items + static_cast<size_t>(i) * Ops::kFloats);
@@ -106,20 +107,26 @@ __global__ __launch_bounds__(kBlock) void k_morton(const float* __restrict__ ite
     idx[i] = static_cast<uint32_t>(i);
 }
 
+// masks of every block boundary (lbvh_boundary in qk_lbvh.cuh): warp b takes the boundary left
+// of block b
+__global__ __launch_bounds__(kBlock) void k_lbvh_carry(LbvhView v, int blocks,
+                                                       LbvhCarry* __restrict__ carry) {
+    const int b = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (b >= blocks) return;
+    unsigned long long left = 0, right = 0;
+    if (b > 0) lbvh_boundary(v, b * kLbvhSpan, lane, left, right);
+    if (lane != 0) return;
+    carry[b].left = left;
+    if (b > 0) carry[b - 1].right = right;
+    if (b == blocks - 1) carry[b].right = 0;
+}
+
 template <class Ops>
-__global__ __launch_bounds__(kBlock) void k_emit(
-    const float* __restrict__ items, int n, const uint32_t* __restrict__ codes,
-    const uint32_t* __restrict__ ids, Node* __restrict__ nodes, float* __restrict__ sorted,
-    int* __restrict__ prim_ids, int* __restrict__ slot_of, int* __restrict__ parent,
-    BNode* __restrict__ bnodes, float4* __restrict__ leaves, int* __restrict__ flags,
-    int2* __restrict__ ranges) {
-    __shared__ __align__(16) float stage[kBlock / 32][emit_stage_floats<Ops>()];
-    const int k0 = blockIdx.x * kBlock + (threadIdx.x & ~31);
-    if (k0 >= n) return;  // whole warps
-    emit_leaves_warp<Ops>(items, n, ids, nodes, sorted, prim_ids, slot_of, leaves, k0,
-                          min(32, n - k0), stage[threadIdx.x >> 5]);
-    const int k = k0 + (threadIdx.x & 31);
-    if (k < n) emit_internal(n, codes, ids, nodes, parent, bnodes, flags, k, ranges);
+__global__ __launch_bounds__(kLbvhSpan, 4) void k_lbvh_tree(LbvhView v,
+                                                            const LbvhCarry* __restrict__ carry,
+                                                            Header* __restrict__ h) {
+    __shared__ __align__(16) LbvhShared sh;
+    lbvh_block<Ops>(v, blockIdx.x * kLbvhSpan, carry[blockIdx.x], &h->max_depth, sh);
 }
 
 // (first slot, leaves) of every internal node of a tree whose subtrees cover ordered
@@ -472,24 +479,10 @@ __global__ __launch_bounds__(kBlock) void k_check_wide(const Node* __restrict__ 
     if (bad) atomicAdd(&err[6], 1);
 }
 
-// Boxes (bottom-up), traversal nodes and depths of a tree whose links and leaves are set;
-// shared by the LBVH and SAH builders and topology edits.  `ranges` (one int2 per internal
-// node) holds the slot ranges when ranges_ready (the LBVH emit writes them), else they are
-// derived first.  Reads the maximum depth back (syncs).
-int finish_tree(qk_tree* t, Header* h, int2* ranges, bool ranges_ready, cudaStream_t s) {
-    const int n = t->n;
-    Node* nodes = static_cast<Node*>(t->nodes);
-    if (!ranges_ready) k_ranges_descent<<<blocks_for(n - 1), kBlock, 0, s>>>(nodes, n, ranges);
-    k_bottom_up_ranged<kUpSpan><<<blocks_for(n, kUpSpan), kUpSpan, 0, s>>>(nodes, static_cast<BNode*>(t->bnodes),
-                                                        t->parent, t->flags, n, ranges);
-    stage_mark(kMarkBoxes, s);
-    cudaMemsetAsync(&h->max_depth, 0, sizeof(int), s);
-    k_depth_anchors<<<blocks_for(n - 1), kBlock, 0, s>>>(t->parent, ranges, n, t->depth_arr);
-    k_depth<<<blocks_for(2 * n - 1), kBlock, 0, s>>>(t->parent, ranges, n, t->depth_arr, h);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_status(e, "tree boxes");
+// reads the maximum depth back into the tree (syncs); no 4-wide nodes yet
+int finish_depth(qk_tree* t, const Header* h, cudaStream_t s) {
     int depth = 0;
-    e = cudaMemcpyAsync(&depth, &h->max_depth, sizeof(int), cudaMemcpyDeviceToHost, s);
+    cudaError_t e = cudaMemcpyAsync(&depth, &h->max_depth, sizeof(int), cudaMemcpyDeviceToHost, s);
     stage_mark(kMarkEnd, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_status(e, "build depth readback");
@@ -498,6 +491,24 @@ int finish_tree(qk_tree* t, Header* h, int2* ranges, bool ranges_ready, cudaStre
     t->wide_leaf = 0;
     if (depth >= kStack) return fail(QK_ERR_DEPTH, "tree depth %d exceeds %d", depth, kStack - 1);
     return QK_OK;
+}
+
+// Boxes (bottom-up), traversal nodes and depths of a tree whose links and leaves are set;
+// shared by the SAH builder and topology edits.  `ranges`: one int2 per internal node of
+// scratch.  Reads the maximum depth back (syncs).
+int finish_tree(qk_tree* t, Header* h, int2* ranges, cudaStream_t s) {
+    const int n = t->n;
+    Node* nodes = static_cast<Node*>(t->nodes);
+    k_ranges_descent<<<blocks_for(n - 1), kBlock, 0, s>>>(nodes, n, ranges);
+    k_bottom_up_ranged<kUpSpan><<<blocks_for(n, kUpSpan), kUpSpan, 0, s>>>(nodes, static_cast<BNode*>(t->bnodes),
+                                                        t->parent, t->flags, n, ranges);
+    stage_mark(kMarkBoxes, s);
+    cudaMemsetAsync(&h->max_depth, 0, sizeof(int), s);
+    k_depth_anchors<<<blocks_for(n - 1), kBlock, 0, s>>>(t->parent, ranges, n, t->depth_arr);
+    k_depth<<<blocks_for(2 * n - 1), kBlock, 0, s>>>(t->parent, ranges, n, t->depth_arr, h);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_status(e, "tree boxes");
+    return finish_depth(t, h, s);
 }
 
 template <class Ops>
@@ -511,27 +522,38 @@ int build_lbvh(qk_tree* t, const void* items_v, void* ws, cudaStream_t s) {
     uint32_t* codes_s = c.take<uint32_t>(n);
     uint32_t* idx_s = c.take<uint32_t>(n);
     void* sort_ws = c.take<char>(sort_ws_bytes(n));
-    Node* nodes = static_cast<Node*>(t->nodes);
-    BNode* bn = static_cast<BNode*>(t->bnodes);
-
     k_header_init<<<1, 32, 0, s>>>(h);
     const int grid = min(blocks_for(n), 148 * 8);
     k_centroid_bounds<Ops><<<grid, kBlock, 0, s>>>(items, n, h);
-    k_morton<Ops><<<blocks_for(n), kBlock, 0, s>>>(items, n, h, codes, idx);
+    k_morton<Ops><<<blocks_for(n), kBlock, 0, s>>>(items, n, h, codes, idx, t->flags);
     stage_mark(kMarkMorton, s);
     cudaError_t e = sort_pairs(codes, idx, codes_s, idx_s, n, 30, sort_ws, s);
     if (e != cudaSuccess) return cuda_status(e, "build sort");
     stage_mark(kMarkSort, s);
-    int2* ranges = build_ranges(ws, t->kind, n, QK_BUILD_LBVH);
-    // leaves (the scatter into leaf order) and internal nodes in one pass
-    k_emit<Ops><<<blocks_for(n), kBlock, 0, s>>>(items, n, codes_s, idx_s, nodes,
-                                                  static_cast<float*>(t->items), t->prim_ids,
-                                                  t->slot_of, t->parent, bn,
-                                                  static_cast<float4*>(t->leaves), t->flags, ranges);
+    LbvhView v;
+    v.items = items;
+    v.codes = codes_s;
+    v.ids = idx_s;
+    v.n = n;
+    v.nodes = static_cast<Node*>(t->nodes);
+    v.sorted = static_cast<float*>(t->items);
+    v.prim_ids = t->prim_ids;
+    v.slot_of = t->slot_of;
+    v.parent = t->parent;
+    v.depth = t->depth_arr;
+    v.bnodes = static_cast<BNode*>(t->bnodes);
+    v.leaves = static_cast<float4*>(t->leaves);
+    v.flags = t->flags;
+    // 16 bytes per block of 256 leaves, in the builders' 8 bytes per primitive of range scratch
+    auto* carry = reinterpret_cast<LbvhCarry*>(build_ranges(ws, t->kind, n, QK_BUILD_LBVH));
+    const int blocks = blocks_for(n, kLbvhSpan);
+    k_lbvh_carry<<<blocks_for(blocks, kBlock / 32), kBlock, 0, s>>>(v, blocks, carry);
+    k_lbvh_tree<Ops><<<blocks, kLbvhSpan, 0, s>>>(v, carry, h);
     stage_mark(kMarkTopo, s);
+    stage_mark(kMarkBoxes, s);  // the same pass
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_status(e, "build kernels");
-    return finish_tree(t, h, ranges, true, s);
+    return finish_depth(t, h, s);
 }
 
 template <class Ops>
@@ -611,7 +633,7 @@ int validate_impl(const qk_tree* t, const void* items, int* err, void* ws, cudaS
 }  // namespace
 
 int finish_tree_boxes(qk_tree* t, Header* h, int2* ranges, cudaStream_t s) {
-    return finish_tree(t, h, ranges, false, s);
+    return finish_tree(t, h, ranges, s);
 }
 
 // workspace of the builders themselves; the bottom-up ranges follow it
@@ -655,8 +677,7 @@ int build_tree(qk_tree* t, int builder, int bins, const void* items, void* ws, s
         cudaMemsetAsync(t->flags, 0, sizeof(int) * static_cast<size_t>(t->n - 1), s);
         const int st = build_sah(t, bins, builder == QK_BUILD_SAH4 ? 4 : 1, items, ws, s);
         if (st != QK_OK) return st;
-        return finish_tree(t, static_cast<Header*>(ws), build_ranges(ws, t->kind, t->n, builder),
-                           false, s);
+        return finish_tree(t, static_cast<Header*>(ws), build_ranges(ws, t->kind, t->n, builder), s);
     }
     switch (t->kind) {
         case kTri: return build_lbvh<TriOps>(t, items, ws, s);

@@ -1,6 +1,6 @@
-// qk_build.cuh -- device code shared by the single-tree builder (qk_build.cu) and the
-// batched builder (qk_batch.cu): Morton quantisation, the Karras emit of one slot, the
-// bottom-up climb of one leaf and the 4-wide node of one even-depth internal node.
+// qk_build.cuh -- device code shared by the builders (qk_build.cu, qk_sah.cu, qk_topo.cu,
+// qk_batch.cu): Morton quantisation, the staged leaf writer, the bottom-up climb of one leaf,
+// depths along parent chains and the 4-wide node of one even-depth internal node.
 #pragma once
 
 #include "qk_internal.cuh"
@@ -26,14 +26,6 @@ __device__ __forceinline__ uint32_t quant(float v, float lo, float extent) {
 // 64-bit key of slot j: (code << 32) | scene index
 __device__ __forceinline__ uint64_t key64(const uint32_t* codes, const uint32_t* ids, int j) {
     return (static_cast<uint64_t>(codes[j]) << 32) | ids[j];
-}
-
-// common-prefix length of keys a and b; -1 outside [0, n)
-__device__ __forceinline__ int cpl(const uint32_t* codes, const uint32_t* ids, int n, uint64_t ka,
-                                   int b) {
-    if (b < 0 || b >= n) return -1;
-    const uint64_t x = ka ^ key64(codes, ids, b);
-    return x == 0 ? 64 : __clzll(x);
 }
 
 __device__ __forceinline__ void write_box(Node* nd, Box b) {
@@ -114,8 +106,8 @@ __device__ __forceinline__ void store_leaves_warp(const float (&it)[Ops::kFloats
     __syncwarp();
 }
 
-// Leaves k0 .. k0 + m - 1 (m <= 32) of the LBVH over sorted (code, id) pairs, by the whole
-// warp: each lane gathers one primitive, then store_leaves_warp writes them.
+// Leaves k0 .. k0 + m - 1 (m <= 32) of a tree whose slot order is `ids`, by the whole warp: each
+// lane gathers one primitive, then store_leaves_warp writes them.
 template <class Ops>
 __device__ __forceinline__ void emit_leaves_warp(
     const float* __restrict__ items, int n, const uint32_t* __restrict__ ids,
@@ -129,50 +121,6 @@ __device__ __forceinline__ void emit_leaves_warp(
     for (int j = 0; j < Ops::kFloats; ++j)
         it[j] = ok ? items[static_cast<size_t>(src) * Ops::kFloats + j] : 0.0f;
     store_leaves_warp<Ops>(it, src, n, nodes, sorted, prim_ids, slot_of, leaves, k0, m, stage);
-}
-
-// Internal node k (k < n - 1) of the LBVH over sorted (code, id) pairs, its children's parent
-// links, its slot range (with `ranges`) and its arrival counter; parent[0] = -1 for k = 0.
-__device__ __forceinline__ void emit_internal(int n, const uint32_t* __restrict__ codes,
-                                              const uint32_t* __restrict__ ids,
-                                              Node* __restrict__ nodes, int* __restrict__ parent,
-                                              BNode* __restrict__ bnodes, int* __restrict__ flags,
-                                              int k, int2* __restrict__ ranges = nullptr) {
-    if (k == 0) parent[0] = -1;
-    if (k >= n - 1) return;
-
-    // internal node k (Karras 2012): direction, range end by exponential + binary search,
-    // then the split as the last index whose prefix with the first exceeds the node's
-    const uint64_t kk = key64(codes, ids, k);
-    const int dir = cpl(codes, ids, n, kk, k + 1) > cpl(codes, ids, n, kk, k - 1) ? 1 : -1;
-    const int dmin = cpl(codes, ids, n, kk, k - dir);
-    int lmax = 2;
-    while (cpl(codes, ids, n, kk, k + lmax * dir) > dmin) lmax *= 2;
-    int l = 0;
-    for (int t = lmax / 2; t > 0; t /= 2) {
-        if (cpl(codes, ids, n, kk, k + (l + t) * dir) > dmin) l += t;
-    }
-    const int j = k + l * dir;
-    const int first = min(k, j), last = max(k, j);
-    if (ranges) ranges[k] = make_int2(first, last - first + 1);
-    const int dnode = cpl(codes, ids, n, kk, j);
-    const uint64_t kf = key64(codes, ids, first);
-    int split = first;
-    int step = last - first;
-    do {
-        step = (step + 1) >> 1;
-        const int cand = split + step;
-        if (cand < last && cpl(codes, ids, n, kf, cand) > dnode) split = cand;
-    } while (step > 1);
-    const int left = split == first ? (n - 1 + split) : split;
-    const int right = split + 1 == last ? (n - 1 + split + 1) : split + 1;
-    *reinterpret_cast<int2*>(&nodes[k].left) = make_int2(left, right);
-    parent[left] = k;
-    parent[right] = k;
-    const int lref = left >= n - 1 ? ~(left - (n - 1)) : left;
-    const int rref = right >= n - 1 ? ~(right - (n - 1)) : right;
-    bnodes[k].v3 = make_float4(__int_as_float(lref), __int_as_float(rref), 0.0f, 0.0f);
-    flags[k] = 0;
 }
 
 __device__ __forceinline__ Box load_box_cg(const Node* nd) {
