@@ -135,8 +135,7 @@ __global__ __launch_bounds__(kBlock) void k_bt_morton(const BScene* __restrict__
                                                       const int2* __restrict__ chunks,
                                                       const Header* __restrict__ hdr,
                                                       uint32_t* __restrict__ codes,
-                                                      uint32_t* __restrict__ keep,
-                                                      uint32_t* __restrict__ idx) {
+                                                      uint32_t* __restrict__ keep) {
     const int2 ch = chunks[blockIdx.x];
     const BScene& sc = tab[ch.x];
     const Header& h = hdr[ch.x];
@@ -152,7 +151,6 @@ __global__ __launch_bounds__(kBlock) void k_bt_morton(const BScene* __restrict__
         const int j = sc.prim_off + i;
         codes[j] = code;
         keep[j] = code;
-        idx[j] = static_cast<uint32_t>(j);
     }
 }
 
@@ -586,8 +584,7 @@ __global__ __launch_bounds__(kBlock) void k_bq_keys(const BScene* __restrict__ t
                                                     const int* __restrict__ q_off,
                                                     const float* __restrict__ pos, int stride,
                                                     int scene_bits, int axis_bits,
-                                                    uint32_t* __restrict__ keys,
-                                                    uint32_t* __restrict__ idx) {
+                                                    uint32_t* __restrict__ keys) {
     const int c = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
     if (c >= nchunks) return;
     const int2 ch = chunks[c];
@@ -612,7 +609,6 @@ __global__ __launch_bounds__(kBlock) void k_bq_keys(const BScene* __restrict__ t
     for (int b = axis_bits - 1; b >= 0; --b)
         code = (code << 3) | (((q3[2] >> b) & 1u) << 2) | (((q3[1] >> b) & 1u) << 1) | ((q3[0] >> b) & 1u);
     keys[i] = (static_cast<uint32_t>(s) << (3 * axis_bits)) | code;
-    idx[i] = static_cast<uint32_t>(i);
 }
 
 }  // namespace
@@ -662,6 +658,7 @@ struct qk_batch_plan {
     unsigned long long* d_stats = nullptr;
     qk::Header* d_hdr = nullptr;
     uint32_t *keys = nullptr, *idx = nullptr, *keys_s = nullptr, *idx_s = nullptr;
+    const uint32_t* order = nullptr;  // the sorted queries (idx or idx_s), set by each query
     void* sort_ws = nullptr;
     int* counts = nullptr;
     void* scan_ws = nullptr;
@@ -768,20 +765,23 @@ int batch_build_impl(qk_batch* b, cudaStream_t s) {
     uint32_t* idx_s = b->bufs[4];
     k_bt_reset<<<blocks_for(S, 128), 128, 0, s>>>(b->d_hdr, S);
     k_bt_bounds<Ops><<<C, kBlock, 0, s>>>(b->d_tab, b->d_chunks, b->d_hdr);
-    k_bt_morton<Ops><<<C, kBlock, 0, s>>>(b->d_tab, b->d_chunks, b->d_hdr, codes, keep, idx);
-    cudaError_t e = sort_pairs(codes, idx, codes_s, idx_s, N, 30, b->sort_ws, s);
+    k_bt_morton<Ops><<<C, kBlock, 0, s>>>(b->d_tab, b->d_chunks, b->d_hdr, codes, keep);
+    SortedPairs by_code, by_scene;
+    cudaError_t e = sort_pairs(codes, idx, codes_s, idx_s, N, 30, b->sort_ws, s, &by_code, true);
     if (e != cudaSuccess) return cuda_status(e, "batch code sort");
     // second, stable pass on the scene: sorted (code, index) stays in order inside a scene
-    k_bt_scene_key<<<blocks_for(N), kBlock, 0, s>>>(b->d_prim_off, S, idx_s, N, codes);
-    e = sort_pairs(codes, idx_s, idx, codes_s, N, scene_bits_for(S), b->sort_ws, s);
+    uint32_t* free_vals = by_code.vals == idx ? idx_s : idx;
+    k_bt_scene_key<<<blocks_for(N), kBlock, 0, s>>>(b->d_prim_off, S, by_code.vals, N, codes_s);
+    e = sort_pairs(codes_s, by_code.vals, codes, free_vals, N, scene_bits_for(S), b->sort_ws, s,
+                   &by_scene);
     if (e != cudaSuccess) return cuda_status(e, "batch scene sort");
-    // idx_f = codes_s; gather codes into codes, local ids into idx_s
-    k_bt_gather<<<C, kBlock, 0, s>>>(b->d_tab, b->d_chunks, keep, codes_s, codes, idx_s);
+    // the order is in idx or idx_s: gather codes into codes, local ids into codes_s
+    k_bt_gather<<<C, kBlock, 0, s>>>(b->d_tab, b->d_chunks, keep, by_scene.vals, codes, codes_s);
     // keep and idx are free after the gather: their 2N uint32 (adjacent, 256-byte aligned) hold
     // the boundary masks
     auto* carry = reinterpret_cast<LbvhCarry*>(keep);
-    k_bt_carry<<<C, 32 * kChunkSpans, 0, s>>>(b->d_tab, b->d_chunks, codes, idx_s, carry);
-    k_bt_tree<Ops><<<C * kChunkSpans, kLbvhSpan, 0, s>>>(b->d_tab, b->d_chunks, codes, idx_s, carry,
+    k_bt_carry<<<C, 32 * kChunkSpans, 0, s>>>(b->d_tab, b->d_chunks, codes, codes_s, carry);
+    k_bt_tree<Ops><<<C * kChunkSpans, kLbvhSpan, 0, s>>>(b->d_tab, b->d_chunks, codes, codes_s, carry,
                                                          b->d_hdr);
     if (b->flags & QK_WIDE) {
         k_bt_wide_flags<<<C, kBlock, 0, s>>>(b->d_tab, b->d_chunks);
@@ -888,7 +888,7 @@ int launch_bq(const Q& q, const qk_batch_plan* p, const qk_batch_tune& tune, cud
     a.chunks = p->d_chunks;
     a.nchunks = p->nchunks;
     a.q_off = p->d_qoff;
-    a.order = (p->flags & QK_ORDER_MORTON) ? p->idx_s : nullptr;
+    a.order = (p->flags & QK_ORDER_MORTON) ? p->order : nullptr;
     a.counter = p->d_counter;
     a.per_fetch = tune.chunks_per_fetch;
     a.short_stack = tune.short_stack;
@@ -909,7 +909,7 @@ int launch_bq_split(const Q& q, const qk_batch_plan* p, const qk_batch_tune& tun
     a.chunks = p->d_chunks;
     a.nchunks = p->nchunks;
     a.q_off = p->d_qoff;
-    a.order = (p->flags & QK_ORDER_MORTON) ? p->idx_s : nullptr;
+    a.order = (p->flags & QK_ORDER_MORTON) ? p->order : nullptr;
     a.counter = p->d_counter;
     a.per_fetch = tune.chunks_per_fetch;
     a.short_stack = 0;
@@ -1373,10 +1373,12 @@ int qk_batch_query(qk_batch_plan* p, const qk_batch_io* io, const qk_batch_tune*
         const int stride = p->op == QK_OP_RAY ? 8 : 3;
         k_bq_keys<<<blocks_for(p->nchunks, kBlock / 32), kBlock, 0, s>>>(
             p->b->d_tab, p->d_chunks, p->nchunks, p->d_qoff, static_cast<const float*>(io->input),
-            stride, sb, ab, p->keys, p->idx);
+            stride, sb, ab, p->keys);
+        SortedPairs by;
         const cudaError_t e = sort_pairs(p->keys, p->idx, p->keys_s, p->idx_s, p->total,
-                                         sb + 3 * ab, p->sort_ws, s);
+                                         sb + 3 * ab, p->sort_ws, s, &by, true);
         if (e != cudaSuccess) return cuda_status(e, "batched query order");
+        p->order = by.vals;
     }
     const bool wide = (p->flags & QK_WIDE) != 0;
     if (t.split) {

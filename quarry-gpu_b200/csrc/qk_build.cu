@@ -94,7 +94,6 @@ template <class Ops>
 __global__ __launch_bounds__(kBlock) void k_morton(const float* __restrict__ items, int n,
                                                    const Header* __restrict__ h,
                                                    uint32_t* __restrict__ codes,
-                                                   uint32_t* __restrict__ idx,
                                                    int* __restrict__ flags) {
     const int i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= n) return;
@@ -104,7 +103,6 @@ __global__ __launch_bounds__(kBlock) void k_morton(const float* __restrict__ ite
     const float3 c = Ops::centroid(items + static_cast<size_t>(i) * Ops::kFloats);
     codes[i] = spread10(quant(c.x, lx, hx - lx)) | (spread10(quant(c.y, ly, hy - ly)) << 1) |
                (spread10(quant(c.z, lz, hz - lz)) << 2);
-    idx[i] = static_cast<uint32_t>(i);
 }
 
 // masks of every block boundary (lbvh_boundary in qk_lbvh.cuh): warp b takes the boundary left
@@ -525,15 +523,16 @@ int build_lbvh(qk_tree* t, const void* items_v, void* ws, cudaStream_t s) {
     k_header_init<<<1, 32, 0, s>>>(h);
     const int grid = min(blocks_for(n), 148 * 8);
     k_centroid_bounds<Ops><<<grid, kBlock, 0, s>>>(items, n, h);
-    k_morton<Ops><<<blocks_for(n), kBlock, 0, s>>>(items, n, h, codes, idx, t->flags);
+    k_morton<Ops><<<blocks_for(n), kBlock, 0, s>>>(items, n, h, codes, t->flags);
     stage_mark(kMarkMorton, s);
-    cudaError_t e = sort_pairs(codes, idx, codes_s, idx_s, n, 30, sort_ws, s);
+    SortedPairs order;
+    cudaError_t e = sort_pairs(codes, idx, codes_s, idx_s, n, 30, sort_ws, s, &order, true);
     if (e != cudaSuccess) return cuda_status(e, "build sort");
     stage_mark(kMarkSort, s);
     LbvhView v;
     v.items = items;
-    v.codes = codes_s;
-    v.ids = idx_s;
+    v.codes = order.keys;
+    v.ids = order.vals;
     v.n = n;
     v.nodes = static_cast<Node*>(t->nodes);
     v.sorted = static_cast<float*>(t->items);

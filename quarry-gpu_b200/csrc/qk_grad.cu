@@ -288,12 +288,10 @@ __global__ __launch_bounds__(kBlock) void k_segment_sum(const uint32_t* __restri
     for (int ch = 0; ch < channels && ch < 10; ++ch) out[static_cast<size_t>(k) * channels + ch] = static_cast<float>(acc[ch]);
 }
 
-__global__ void k_shift_keys(const int* __restrict__ keys, int count, uint32_t* __restrict__ k32,
-                             uint32_t* __restrict__ idx) {
+__global__ void k_shift_keys(const int* __restrict__ keys, int count, uint32_t* __restrict__ k32) {
     const int i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= count) return;
     k32[i] = static_cast<uint32_t>(keys[i] + 1);
-    idx[i] = static_cast<uint32_t>(i);
 }
 
 struct GradWs {
@@ -326,12 +324,13 @@ int segment_sum_impl(const int* keys, const V* vals, int count, int channels, in
         cudaMemsetAsync(out, 0, sizeof(float) * static_cast<size_t>(nseg) * channels, s);
         return QK_OK;
     }
-    k_shift_keys<<<blocks_for(count), kBlock, 0, s>>>(keys, count, g.k32, g.idx);
+    k_shift_keys<<<blocks_for(count), kBlock, 0, s>>>(keys, count, g.k32);
     int bits = 1;
     while (bits < 32 && (1ull << bits) <= static_cast<unsigned long long>(nseg)) ++bits;
-    cudaError_t e = sort_pairs(g.k32, g.idx, g.k32s, g.idxs, count, bits, g.sort_ws, s);
+    SortedPairs by;
+    cudaError_t e = sort_pairs(g.k32, g.idx, g.k32s, g.idxs, count, bits, g.sort_ws, s, &by, true);
     if (e != cudaSuccess) return cuda_status(e, "gradient sort");
-    k_segment_sum<V><<<blocks_for(nseg), kBlock, 0, s>>>(g.k32s, g.idxs, vals, count, channels, nseg, out);
+    k_segment_sum<V><<<blocks_for(nseg), kBlock, 0, s>>>(by.keys, by.vals, vals, count, channels, nseg, out);
     e = cudaGetLastError();
     return e == cudaSuccess ? QK_OK : cuda_status(e, "segment sum");
 }

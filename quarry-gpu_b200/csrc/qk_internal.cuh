@@ -109,8 +109,14 @@ struct Header {
 
 // ---- sort / scan (qk_sort.cu) ----
 size_t sort_ws_bytes(int n);
+// where a sort left its result
+struct SortedPairs {
+    const uint32_t* keys;
+    const uint32_t* vals;
+};
 cudaError_t sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout,
-                       int n, int bits, void* ws, cudaStream_t s);
+                       int n, int bits, void* ws, cudaStream_t s, SortedPairs* sorted = nullptr,
+                       bool iota = false);
 size_t scan_ws_bytes(int n);
 // exclusive scan of n ints; writes the total to out[n] when write_total is set
 cudaError_t scan_exclusive(const int* in, int* out, int n, bool write_total, void* ws,

@@ -119,8 +119,7 @@ __global__ void k_bounds_reset(Header* h, int fixed_unit) {
 __global__ __launch_bounds__(kBlock) void k_pos_keys(const float* __restrict__ p, int stride,
                                                     int offset, int count,
                                                     const Header* __restrict__ h,
-                                                    uint32_t* __restrict__ keys,
-                                                    uint32_t* __restrict__ idx) {
+                                                    uint32_t* __restrict__ keys) {
     const int i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= count) return;
     const float* q = p + static_cast<size_t>(i) * stride + offset;
@@ -128,7 +127,6 @@ __global__ __launch_bounds__(kBlock) void k_pos_keys(const float* __restrict__ p
     const float hx = unord_f(h->hi[0]), hy = unord_f(h->hi[1]), hz = unord_f(h->hi[2]);
     keys[i] = spread10q(quantize10(q[0], lx, hx)) | (spread10q(quantize10(q[1], ly, hy)) << 1) |
               (spread10q(quantize10(q[2], lz, hz)) << 2);
-    idx[i] = static_cast<uint32_t>(i);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1240,10 +1238,12 @@ const uint32_t* make_order(const float* pos, int stride, int offset, int count, 
         const int grid = min(blocks_for(count), 148 * 4);
         k_pos_bounds<<<grid, kBlock, 0, s>>>(pos + offset, stride, count, o.h);
     }
-    k_pos_keys<<<blocks_for(count), kBlock, 0, s>>>(pos, stride, offset, count, o.h, o.keys, o.idx);
-    const cudaError_t e = sort_pairs(o.keys, o.idx, o.keys_s, o.idx_s, count, 30, o.sort_ws, s);
+    k_pos_keys<<<blocks_for(count), kBlock, 0, s>>>(pos, stride, offset, count, o.h, o.keys);
+    SortedPairs sorted;
+    const cudaError_t e = sort_pairs(o.keys, o.idx, o.keys_s, o.idx_s, count, 30, o.sort_ws, s,
+                                     &sorted, true);
     if (e != cudaSuccess) *status = cuda_status(e, "order sort");
-    return o.idx_s;
+    return sorted.vals;
 }
 
 // lanes per query of the split schedules: QK_TUNE_SPLIT a warp, QK_TUNE_SPLIT8 / 4 groups of

@@ -745,10 +745,12 @@ int update_impl(const qk_tree* old_t, qk_tree* new_t, const qk_topo_edit* ed, in
         k_topo_extra_rank<<<blocks_for(n_extra), kBlock, 0, s>>>(w.cut_mark, n_extra, w.ext_key);
         int bits = 1;
         while (bits < 32 && (1ll << bits) < plan.cuts) ++bits;
-        err = sort_pairs(w.ext_key, w.ext_val, w.ext_key_s, w.ext_val_s, n_extra, bits, w.sort_ws, s);
+        SortedPairs ext;
+        err = sort_pairs(w.ext_key, w.ext_val, w.ext_key_s, w.ext_val_s, n_extra, bits, w.sort_ws, s,
+                         &ext);
         if (err != cudaSuccess) return cuda_status(err, "topology extra sort");
         k_topo_stage_extra<Ops><<<blocks_for(n_extra), kBlock, 0, s>>>(
-            e, *old_t, w.ext_key_s, w.ext_val_s, w.cut_list, w.range, w.wslot, w.del_flag,
+            e, *old_t, ext.keys, ext.vals, w.cut_list, w.range, w.wslot, w.del_flag,
             w.st_items, w.st_id, w.cen, w.plo, w.phi, w.order, eerr);
     }
     stage_mark(kMarkRelayout, s);
