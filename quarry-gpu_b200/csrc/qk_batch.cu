@@ -448,6 +448,8 @@ struct QRay {
     __device__ bool enabled() const { return true; }
     __device__ __forceinline__ void run(const BScene& sc, int, int q, Stack& st, Trav& tv) const {
         const RayPre R = prepare_ray(__ldg(rays + 2 * q), __ldg(rays + 2 * q + 1));
+        __shared__ float4 tails[256];
+        const RayTail tail(tails + threadIdx.x, R);
         int best_id;
         // rays with no parallel axis and vertical rays take traversals compiled for their
         // RayPre::mode; others the general one
@@ -455,16 +457,16 @@ struct QRay {
         const BNode* bn = static_cast<const BNode*>(sc.t.bnodes);
         const float4* lv = static_cast<const float4*>(sc.t.leaves);
         if (kWide) {
-            out[q] = R.mode == 0 ? ray_wide_one<false, 0>(wn, lv, R, max_iter_of(sc.t), st, tv, best_id)
-                   : R.mode == 3 ? ray_wide_one<false, 3>(wn, lv, R, max_iter_of(sc.t), st, tv, best_id)
-                                 : ray_wide_one<false, -1>(wn, lv, R, max_iter_of(sc.t), st, tv, best_id);
+            out[q] = R.mode == 0 ? ray_wide_one<false, 0>(wn, lv, R, tail, max_iter_of(sc.t), st, tv, best_id)
+                   : R.mode == 3 ? ray_wide_one<false, 3>(wn, lv, R, tail, max_iter_of(sc.t), st, tv, best_id)
+                                 : ray_wide_one<false, -1>(wn, lv, R, tail, max_iter_of(sc.t), st, tv, best_id);
         } else {
             const Box rb = root_box(static_cast<const Node*>(sc.t.nodes));
             out[q] = R.mode == 0
-                         ? ray_bin_one<Stack, false, 0>(bn, lv, rb, R, max_iter_of(sc.t), st, tv, best_id)
+                         ? ray_bin_one<Stack, false, 0, true>(bn, lv, rb, R, tail, max_iter_of(sc.t), st, tv, best_id)
                      : R.mode == 3
-                         ? ray_bin_one<Stack, false, 3>(bn, lv, rb, R, max_iter_of(sc.t), st, tv, best_id)
-                         : ray_bin_one<Stack, false, -1>(bn, lv, rb, R, max_iter_of(sc.t), st, tv, best_id);
+                         ? ray_bin_one<Stack, false, 3, true>(bn, lv, rb, R, tail, max_iter_of(sc.t), st, tv, best_id)
+                         : ray_bin_one<Stack, false, -1, true>(bn, lv, rb, R, tail, max_iter_of(sc.t), st, tv, best_id);
         }
     }
 };
@@ -569,7 +571,7 @@ struct QRadiusPool {
                                                  static_cast<const float4*>(sc.t.leaves), p, r2,
                                                  sink, max_iter_of(sc.t), st, tv);
         else
-            found = radius_bin_visit<Ops, true, Stack, false>(
+            found = radius_bin_visit<Ops, true, Stack, false, false>(
                 static_cast<const BNode*>(sc.t.bnodes), static_cast<const float4*>(sc.t.leaves),
                 root_box(static_cast<const Node*>(sc.t.nodes)), p, r2, sink, max_iter_of(sc.t), st,
                 tv);

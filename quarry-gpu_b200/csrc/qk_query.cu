@@ -377,12 +377,14 @@ __global__ __launch_bounds__(kBlock, kMinBlocks) void k_ray_bin(const BNode* __r
                                                    int max_iter, unsigned long long* __restrict__ stats,
                                                    const Node* __restrict__ lnodes = nullptr) {
     cudaGridDependencySynchronize();  // the order, when the ordering kernels launched it early
-    const int i = blockIdx.x * kBlock + threadIdx.x;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = i < count;
     Trav tv;
+    __shared__ float4 tails[kBlock];
     if (active) {
         const int r = order ? static_cast<int>(order[i]) : i;
         const RayPre R = prepare_ray(__ldg(rays + 2 * r), __ldg(rays + 2 * r + 1));
+        const RayTail tail(tails + threadIdx.x, R);
         int best_id;
         if constexpr (kShort > 0) {
             // the top kShort entries of every thread's stack in shared memory
@@ -393,20 +395,21 @@ __global__ __launch_bounds__(kBlock, kMinBlocks) void k_ray_bin(const BNode* __r
             st.skey = sk + threadIdx.x;
             st.sh = kShort;
             st.stride = kBlock;
-            out[r] = ray_bin_one(bn, leaves, root_box(nodes), R, max_iter, st, tv, best_id);
+            out[r] = ray_bin_one(bn, leaves, root_box(nodes), R, tail, max_iter, st, tv, best_id);
         } else {
             LocalStack<kStack> st;
+            constexpr bool kVec256 = !kLeaf4;
             // rays with no parallel axis and vertical rays (x and y parallel), tmin / tmax not
             // NaN, run traversals compiled for their mode (RayPre::mode); others the general one
             const Box rb = root_box(nodes);
             if (R.mode == 0)
-                out[r] = ray_bin_one<LocalStack<kStack>, kLeaf4, 0>(bn, leaves, rb, R, max_iter,
+                out[r] = ray_bin_one<LocalStack<kStack>, kLeaf4, 0, kVec256>(bn, leaves, rb, R, tail, max_iter,
                                                                     st, tv, best_id, lnodes);
             else if (R.mode == 3)
-                out[r] = ray_bin_one<LocalStack<kStack>, kLeaf4, 3>(bn, leaves, rb, R, max_iter,
+                out[r] = ray_bin_one<LocalStack<kStack>, kLeaf4, 3, kVec256>(bn, leaves, rb, R, tail, max_iter,
                                                                     st, tv, best_id, lnodes);
             else
-                out[r] = ray_bin_one<LocalStack<kStack>, kLeaf4, -1>(bn, leaves, rb, R, max_iter,
+                out[r] = ray_bin_one<LocalStack<kStack>, kLeaf4, -1, kVec256>(bn, leaves, rb, R, tail, max_iter,
                                                                      st, tv, best_id, lnodes);
         }
         if (ids) ids[r] = best_id;
@@ -432,6 +435,8 @@ __global__ __launch_bounds__(kBlock, kMinBlocks) void k_ray_bin_dyn(
     int r = -1;
     bool done = false;
     RayPre R;
+    __shared__ float4 tails[kBlock];
+    RayTail tail(tails + threadIdx.x, RayPre{});
     float best = 0.0f, bound = 0.0f;
     bool any = false;
     int best_id = -1;
@@ -454,6 +459,7 @@ __global__ __launch_bounds__(kBlock, kMinBlocks) void k_ray_bin_dyn(
                 } else {
                     r = order ? static_cast<int>(order[k]) : k;
                     R = prepare_ray(__ldg(rays + 2 * r), __ldg(rays + 2 * r + 1));
+                    tail = RayTail(tails + threadIdx.x, R);
                     best = R.tmax;
                     bound = best * kMarginMul + kMarginAdd;
                     any = false;
@@ -489,12 +495,12 @@ __global__ __launch_bounds__(kBlock, kMinBlocks) void k_ray_bin_dyn(
             ntests += static_cast<int>(hl) + static_cast<int>(hr);
             if (hl && lref < 0) {
                 ++ttests;
-                test_tri(R, leaves, ~lref, best, bound, any, best_id);
+                test_tri(R, tail, leaves, ~lref, best, bound, any, best_id);
                 hl = false;
             }
             if (hr && rref < 0) {
                 ++ttests;
-                test_tri(R, leaves, ~rref, best, bound, any, best_id);
+                test_tri(R, tail, leaves, ~rref, best, bound, any, best_id);
                 hr = false;
             }
             if (hl && hr) {
@@ -543,17 +549,19 @@ __global__ __launch_bounds__(kBlock) void k_ray_wide(const WideNode* __restrict_
                                                     unsigned long long* __restrict__ out,
                                                     int* __restrict__ ids,
                                                     int max_iter, unsigned long long* __restrict__ stats) {
-    const int i = blockIdx.x * kBlock + threadIdx.x;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = i < count;
     Trav tv;
+    __shared__ float4 tails[kBlock];
     if (active) {
         const int r = order ? static_cast<int>(order[i]) : i;
         const RayPre R = prepare_ray(__ldg(rays + 2 * r), __ldg(rays + 2 * r + 1));
+        const RayTail tail(tails + threadIdx.x, R);
         LocalStack<kStackWide> st;
         int best_id;
-        out[r] = R.mode == 0 ? ray_wide_one<kRange, 0>(wn, leaves, R, max_iter, st, tv, best_id)
-               : R.mode == 3 ? ray_wide_one<kRange, 3>(wn, leaves, R, max_iter, st, tv, best_id)
-                             : ray_wide_one<kRange, -1>(wn, leaves, R, max_iter, st, tv, best_id);
+        out[r] = R.mode == 0 ? ray_wide_one<kRange, 0>(wn, leaves, R, tail, max_iter, st, tv, best_id)
+               : R.mode == 3 ? ray_wide_one<kRange, 3>(wn, leaves, R, tail, max_iter, st, tv, best_id)
+                             : ray_wide_one<kRange, -1>(wn, leaves, R, tail, max_iter, st, tv, best_id);
         if (ids) ids[r] = best_id;
     }
     flush_stats<kStats>(active, tv.nodes, tv.leaves, tv.overflow, stats);
@@ -563,6 +571,10 @@ __global__ __launch_bounds__(kBlock) void k_ray_wide(const WideNode* __restrict_
 // queries in blocks of 256 would occupy only some of the 148 SMs, and these latency-bound
 // traversals run faster spread over all of them; large batches keep 256.
 inline int query_block(int count) { return count <= 148 * 512 ? 64 : kBlock; }
+// the same for the lane-group kernels, counted in threads
+inline int split_block(int count, int lanes) {
+    return static_cast<long long>(count) * lanes <= 148 * 2048 ? 64 : kBlock;
+}
 
 // ---------------------------------------------------------------------------------------
 // heavy-query tail (QK_TUNE_TAIL, point clouds).  A point near the centre of a spherical shell
@@ -695,7 +707,7 @@ __global__ __launch_bounds__(kBlock) void k_radius_bin(
         const int write = kFill ? offsets[q] : 0;
         const int end = kFill ? offsets[q + 1] : 0;  // never write past this query's segment
         LocalStack<kStack> st;
-        const int found = radius_bin_one<Ops, kFill, LocalStack<kStack>, kLeaf4>(
+        const int found = radius_bin_one<Ops, kFill, LocalStack<kStack>, kLeaf4, true>(
             bn, leaves, root_box(nodes), p, r2, write, end, keys, max_iter, st, tv, lnodes);
         if (!kFill) counts[q] = found;
     }
@@ -723,7 +735,7 @@ __global__ __launch_bounds__(kBlock) void k_radius_count_pool(
         PoolSink sink{pool.stash + static_cast<size_t>(q) * kRadiusStash, pool.keys, pool.next,
                       pool.taken, pool.chunks, pool.first + q, 0, -1};
         LocalStack<kStack> st;
-        counts[q] = radius_bin_visit<Ops, true, LocalStack<kStack>, kLeaf4>(
+        counts[q] = radius_bin_visit<Ops, true, LocalStack<kStack>, kLeaf4, true>(
             bn, leaves, root_box(nodes), p, r2, sink, max_iter, st, tv, lnodes);
     }
     flush_stats<kStats>(active, tv.nodes, tv.leaves, tv.overflow, stats);
@@ -743,7 +755,7 @@ __global__ __launch_bounds__(kBlock) void k_radius_fill_lost(
     const float3 p = f3(pts[3 * q], pts[3 * q + 1], pts[3 * q + 2]);
     Trav tv;
     LocalStack<kStack> st;
-    radius_bin_one<Ops, true, LocalStack<kStack>, kLeaf4>(bn, leaves, root_box(nodes), p, r2, begin,
+    radius_bin_one<Ops, true, LocalStack<kStack>, kLeaf4, true>(bn, leaves, root_box(nodes), p, r2, begin,
                                                           end, keys, max_iter, st, tv, lnodes);
 }
 
@@ -794,7 +806,7 @@ __global__ __launch_bounds__(kBlock) void k_closest_split(const BNode* __restric
                                                          int max_iter,
                                                          unsigned long long* __restrict__ stats,
                                                          TailList tail = TailList{}) {
-    if (static_cast<long long>(blockIdx.x * kBlock + (threadIdx.x & ~31u)) / G >= count)
+    if (static_cast<long long>(blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) / G >= count)
         return;  // whole warps past the last query
     bool valid;
     int lane;
@@ -818,7 +830,7 @@ __global__ __launch_bounds__(kBlock) void k_knn_split(const BNode* __restrict__ 
                                                      uint2* __restrict__ out, int max_iter,
                                                      unsigned long long* __restrict__ stats,
                                                      TailList tail = TailList{}) {
-    if (static_cast<long long>(blockIdx.x * kBlock + (threadIdx.x & ~31u)) / G >= count)
+    if (static_cast<long long>(blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) / G >= count)
         return;  // whole warps past the last query
     bool valid;
     int lane;
@@ -853,7 +865,7 @@ __global__ __launch_bounds__(kTailBatch) void k_tail_scan(const float4* __restri
     for (int slot = begin; slot < end; ++slot) {
         int id;
         const float d2 = Ops::dist2(p, leaves, slot, id);
-        tab.insert(d2, id, K);
+        tab.insert(d2, id);
     }
     uint2* dst = tail.partial + static_cast<size_t>(hl) * kTailCands + static_cast<size_t>(ti) * K;
 #pragma unroll
@@ -876,7 +888,7 @@ __global__ __launch_bounds__(kBlock) void k_tail_merge(TailList tail, int ncand,
     const uint2* cand = tail.partial + static_cast<size_t>(hl) * kTailCands;
     for (int c = lane; c < ncand; c += 32) {
         const uint2 v = cand[c];
-        if (v.y != 0x7fffffffu) tab.insert(__uint_as_float(v.x), static_cast<int>(v.y), K);
+        if (v.y != 0x7fffffffu) tab.insert(__uint_as_float(v.x), static_cast<int>(v.y));
     }
     for (int r = 0; r < k; ++r) {
         float bd = tab.d[0];
@@ -934,7 +946,7 @@ __global__ __launch_bounds__(kBlock) void k_radius_split(
     const uint32_t* __restrict__ order, int count, float r2, int* __restrict__ counts,
     int* __restrict__ lane_counts, const int* __restrict__ offsets,
     unsigned long long* __restrict__ keys, int max_iter, unsigned long long* __restrict__ stats) {
-    if (static_cast<long long>(blockIdx.x * kBlock + (threadIdx.x & ~31u)) / G >= count)
+    if (static_cast<long long>(blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) / G >= count)
         return;  // whole warps past the last query
     bool valid;
     int lane;
@@ -1257,13 +1269,14 @@ template <class Ops, bool kStats>
 void launch_closest_split(int lanes, const BNode* bn, const float4* leaves, const float* pts,
                           const uint32_t* order, int count, uint2* out, int max_iter,
                           unsigned long long* stats, const TailList& tail, cudaStream_t s) {
-    const int g = blocks_for(static_cast<long long>(count) * lanes);
+    const int sb = split_block(count, lanes);
+    const int g = blocks_for(static_cast<long long>(count) * lanes, sb);
     if (lanes == 4)
-        k_closest_split<Ops, kStats, 4><<<g, kBlock, 0, s>>>(bn, leaves, pts, order, count, out, max_iter, stats, tail);
+        k_closest_split<Ops, kStats, 4><<<g, sb, 0, s>>>(bn, leaves, pts, order, count, out, max_iter, stats, tail);
     else if (lanes == 8)
-        k_closest_split<Ops, kStats, 8><<<g, kBlock, 0, s>>>(bn, leaves, pts, order, count, out, max_iter, stats, tail);
+        k_closest_split<Ops, kStats, 8><<<g, sb, 0, s>>>(bn, leaves, pts, order, count, out, max_iter, stats, tail);
     else
-        k_closest_split<Ops, kStats, 32><<<g, kBlock, 0, s>>>(bn, leaves, pts, order, count, out, max_iter, stats, tail);
+        k_closest_split<Ops, kStats, 32><<<g, sb, 0, s>>>(bn, leaves, pts, order, count, out, max_iter, stats, tail);
 }
 
 // kNN keeps its table one entry per lane: at least k lanes (the next group size up)
@@ -1277,13 +1290,14 @@ void launch_knn_split(int lanes, const BNode* bn, const float4* leaves, const fl
                       const uint32_t* order, int count, int k, int stride, uint2* out,
                       int max_iter, unsigned long long* stats, const TailList& tail,
                       cudaStream_t s) {
-    const int g = blocks_for(static_cast<long long>(count) * lanes);
+    const int sb = split_block(count, lanes);
+    const int g = blocks_for(static_cast<long long>(count) * lanes, sb);
     if (lanes == 4)
-        k_knn_split<Ops, kStats, 4><<<g, kBlock, 0, s>>>(bn, leaves, pts, order, count, k, stride, out, max_iter, stats, tail);
+        k_knn_split<Ops, kStats, 4><<<g, sb, 0, s>>>(bn, leaves, pts, order, count, k, stride, out, max_iter, stats, tail);
     else if (lanes == 8)
-        k_knn_split<Ops, kStats, 8><<<g, kBlock, 0, s>>>(bn, leaves, pts, order, count, k, stride, out, max_iter, stats, tail);
+        k_knn_split<Ops, kStats, 8><<<g, sb, 0, s>>>(bn, leaves, pts, order, count, k, stride, out, max_iter, stats, tail);
     else
-        k_knn_split<Ops, kStats, 32><<<g, kBlock, 0, s>>>(bn, leaves, pts, order, count, k, stride, out, max_iter, stats, tail);
+        k_knn_split<Ops, kStats, 32><<<g, sb, 0, s>>>(bn, leaves, pts, order, count, k, stride, out, max_iter, stats, tail);
 }
 
 template <class Ops>
@@ -1416,16 +1430,17 @@ int radius_launch(const qk_tree* t, const float* pts, int count, float r2, int* 
     if ((flags & kSplitFlags) && !(flags & QK_WIDE)) {
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
         const int lanes = split_lanes(flags);
-        const int gs = blocks_for(static_cast<long long>(count) * lanes);
+        const int sb = split_block(count, lanes);
+        const int gs = blocks_for(static_cast<long long>(count) * lanes, sb);
         if (lanes == 4) {
-            if (stats) k_radius_split<Ops, kFill, true, 4><<<gs, kBlock, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
-            else k_radius_split<Ops, kFill, false, 4><<<gs, kBlock, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
+            if (stats) k_radius_split<Ops, kFill, true, 4><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
+            else k_radius_split<Ops, kFill, false, 4><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
         } else if (lanes == 8) {
-            if (stats) k_radius_split<Ops, kFill, true, 8><<<gs, kBlock, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
-            else k_radius_split<Ops, kFill, false, 8><<<gs, kBlock, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
+            if (stats) k_radius_split<Ops, kFill, true, 8><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
+            else k_radius_split<Ops, kFill, false, 8><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
         } else {
-            if (stats) k_radius_split<Ops, kFill, true, 32><<<gs, kBlock, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
-            else k_radius_split<Ops, kFill, false, 32><<<gs, kBlock, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
+            if (stats) k_radius_split<Ops, kFill, true, 32><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
+            else k_radius_split<Ops, kFill, false, 32><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
         }
     } else if (flags & QK_WIDE) {
         const WideNode* wn = static_cast<const WideNode*>(t->wide);
@@ -1505,15 +1520,17 @@ int ray_query(const qk_tree* t, const void* rays, int count, uint64_t* out, int*
     auto* res = reinterpret_cast<unsigned long long*>(out);
     auto* stt = reinterpret_cast<unsigned long long*>(stats);
     const float4* leaves = static_cast<const float4*>(t->leaves);
-    const int g = blocks_for(count);
+    const int rb = query_block(count);
+    const int g = blocks_for(count, rb);
+    const int g256 = blocks_for(count);  // the short stack's shared arrays are sized for 256 threads
     if (flags & QK_WIDE) {
         const WideNode* wn = static_cast<const WideNode*>(t->wide);
         if (t->wide_leaf == 4) {
-            if (stt) k_ray_wide<true, true><<<g, kBlock, 0, s>>>(wn, leaves, r4, order, count, res, ids, t->n * 2 + 64, stt);
-            else k_ray_wide<false, true><<<g, kBlock, 0, s>>>(wn, leaves, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            if (stt) k_ray_wide<true, true><<<g, rb, 0, s>>>(wn, leaves, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            else k_ray_wide<false, true><<<g, rb, 0, s>>>(wn, leaves, r4, order, count, res, ids, t->n * 2 + 64, stt);
         } else {
-            if (stt) k_ray_wide<true><<<g, kBlock, 0, s>>>(wn, leaves, r4, order, count, res, ids, t->n * 2 + 64, stt);
-            else k_ray_wide<false><<<g, kBlock, 0, s>>>(wn, leaves, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            if (stt) k_ray_wide<true><<<g, rb, 0, s>>>(wn, leaves, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            else k_ray_wide<false><<<g, rb, 0, s>>>(wn, leaves, r4, order, count, res, ids, t->n * 2 + 64, stt);
         }
     } else if (flags & QK_TUNE_DYNAMIC) {
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
@@ -1535,34 +1552,38 @@ int ray_query(const qk_tree* t, const void* rays, int count, uint64_t* out, int*
     } else {
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
         const Node* nodes = static_cast<const Node*>(t->nodes);
+        // the plain kernels read nodes in 256-bit loads; nodes a caller placed off a 32-byte
+        // boundary go to the short-stack kernels, which keep 128-bit loads (same results)
+        if (!(flags & QK_TUNE_LEAF4) && reinterpret_cast<uintptr_t>(bn) % 32 != 0)
+            flags |= QK_TUNE_SHORT_STACK;
         if ((flags & QK_TUNE_HIGH_OCC) && (flags & QK_TUNE_SHORT_STACK)) {
-            if (stt) k_ray_bin<true, 5, 8><<<g, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
-            else k_ray_bin<false, 5, 8><<<g, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            if (stt) k_ray_bin<true, 5, 8><<<g256, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            else k_ray_bin<false, 5, 8><<<g256, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
         } else if (flags & QK_TUNE_SHORT_STACK) {
-            if (stt) k_ray_bin<true, 1, 8><<<g, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
-            else k_ray_bin<false, 1, 8><<<g, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            if (stt) k_ray_bin<true, 1, 8><<<g256, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            else k_ray_bin<false, 1, 8><<<g256, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
         } else if ((flags & QK_TUNE_HIGH_OCC) && (flags & QK_TUNE_LEAF4)) {
-            if (stt) k_ray_bin<true, 5, 0, true><<<g, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
-            else k_ray_bin<false, 5, 0, true><<<g, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
+            if (stt) k_ray_bin<true, 5, 0, true><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
+            else k_ray_bin<false, 5, 0, true><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
         } else if (flags & QK_TUNE_LEAF4) {
-            if (stt) k_ray_bin<true, 1, 0, true><<<g, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
-            else k_ray_bin<false, 1, 0, true><<<g, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
+            if (stt) k_ray_bin<true, 1, 0, true><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
+            else k_ray_bin<false, 1, 0, true><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
         } else if (order) {
             // the previous kernel in the stream wrote the order: start while it drains
             const Node* no_leaf4 = nullptr;
             if (flags & QK_TUNE_HIGH_OCC) {
-                if (stt) launch_pdl(k_ray_bin<true, 5>, dim3(g), dim3(kBlock), s, bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, no_leaf4);
-                else launch_pdl(k_ray_bin<false, 5>, dim3(g), dim3(kBlock), s, bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, no_leaf4);
+                if (stt) launch_pdl(k_ray_bin<true, 5>, dim3(g), dim3(rb), s, bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, no_leaf4);
+                else launch_pdl(k_ray_bin<false, 5>, dim3(g), dim3(rb), s, bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, no_leaf4);
             } else {
-                if (stt) launch_pdl(k_ray_bin<true, 1>, dim3(g), dim3(kBlock), s, bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, no_leaf4);
-                else launch_pdl(k_ray_bin<false, 1>, dim3(g), dim3(kBlock), s, bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, no_leaf4);
+                if (stt) launch_pdl(k_ray_bin<true, 1>, dim3(g), dim3(rb), s, bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, no_leaf4);
+                else launch_pdl(k_ray_bin<false, 1>, dim3(g), dim3(rb), s, bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, no_leaf4);
             }
         } else if (flags & QK_TUNE_HIGH_OCC) {
-            if (stt) k_ray_bin<true, 5><<<g, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
-            else k_ray_bin<false, 5><<<g, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            if (stt) k_ray_bin<true, 5><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            else k_ray_bin<false, 5><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
         } else {
-            if (stt) k_ray_bin<true, 1><<<g, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
-            else k_ray_bin<false, 1><<<g, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            if (stt) k_ray_bin<true, 1><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            else k_ray_bin<false, 1><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
         }
     }
     const cudaError_t e = cudaGetLastError();

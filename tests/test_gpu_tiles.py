@@ -1,0 +1,120 @@
+"""Sizes at which the engine's tiled kernels can go wrong, bit for bit against the oracle: the
+LBVH pass's blocks of 256 leaves, the radix sort's tiles of 4,096 keys, and the traversals'
+forms (node arrays off a 32-byte boundary, every kNN table size, early-ended ellipsoid tests)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import oracle
+from quarry import capi, workloads
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev(a, dtype=np.float32):
+    return capi.to_device(np.ascontiguousarray(a), dtype)
+
+
+def _points(n, seed, distinct):
+    """n points on `distinct` positions: few positions give runs of equal Morton codes, which only
+    their indices order."""
+    p = workloads.uniform_points(min(n, distinct), [0.0] * 3, [100.0] * 3, seed, 13)
+    return np.ascontiguousarray(p[np.random.default_rng(seed).integers(0, len(p), n)])
+
+
+@pytest.mark.parametrize("n", [2, 3, 31, 33, 255, 256, 257, 511, 513, 1025, 4096, 4097, 20001])
+@pytest.mark.parametrize("distinct", [1, 7, 1 << 30])
+def test_lbvh_block_edges(cuda, n, distinct):
+    pts = _points(n, n, distinct)
+    t, ref = capi.DeviceTree("point", pts), oracle.LBVH("point", pts)
+    assert t.nodes_bytes().tobytes() == ref.nodes.tobytes()
+    assert t.validate() == [0] * 8
+    first = t.host("bnodes", np.uint8).copy()
+    t.build()  # the arrival words are clean again
+    assert t.nodes_bytes().tobytes() == ref.nodes.tobytes()
+    assert np.array_equal(t.host("bnodes", np.uint8), first)
+
+
+@pytest.mark.parametrize("sizes", [[2, 2, 2], [2, 257, 3, 1024, 1025, 5], [300] * 40])
+def test_batched_lbvh_block_edges(cuda, sizes):
+    scenes = [_points(n, 100 + i, 50) for i, n in enumerate(sizes)]
+    b = capi.Batch("point", scenes)
+    b.build()
+    b.sync()
+    for i, s in enumerate(scenes):
+        v = b.view(i)
+        assert v.nodes_bytes().tobytes() == oracle.LBVH("point", s).nodes.tobytes()
+        assert v.validate() == [0] * 8
+
+
+@pytest.mark.parametrize("n", [1, 4095, 4096, 4097, 8192, 70001])
+@pytest.mark.parametrize("bits", [1, 8, 9, 16, 24, 30, 32])
+@pytest.mark.parametrize("spread", [1, 3, 1 << 32])
+def test_sort_tile_edges(cuda, n, bits, spread):
+    rng = np.random.default_rng(n + bits)
+    keys = (rng.integers(0, spread, n, dtype=np.uint64) & ((1 << bits) - 1)).astype(np.uint32)
+    vals = rng.integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32)
+    k, v = capi.sort_pairs(_dev(keys.view(np.int32), np.int32), _dev(vals.view(np.int32), np.int32),
+                           bits)
+    o = np.argsort(keys, kind="stable")
+    assert np.array_equal(k.cpu().numpy().view(np.uint32), keys[o])
+    assert np.array_equal(v.cpu().numpy().view(np.uint32), vals[o])
+
+
+def test_nodes_off_a_32_byte_boundary(cuda):
+    """Traversal and 4-wide nodes on a 16-byte boundary: every schedule gives the same bits."""
+    tris, _ = workloads.city(200, 3)
+    lo, hi = workloads.bounds_of(tris)
+    rays = _dev(workloads.cosine_rays(5000, float(lo[0]), float(hi[0]), float(lo[1]), float(hi[1]),
+                                      float(hi[2]) + 50.0, 3))
+    q = _dev(workloads.uniform_points(700, lo, hi, 3, 13))
+    t = capi.DeviceTree("tri", tris)
+    t.build_wide()
+    flags = [0, capi.QK_TUNE_HIGH_OCC, capi.QK_ORDER_COHERENT, capi.QK_WIDE]
+    want = [(t.raycast(rays, f).clone(), t.closest(q, f).clone(), t.knn(q, 8, f).clone())
+            for f in flags]
+    for name in ("bnodes", "wide"):
+        a = t.arrays[name]
+        moved = cuda.empty(a.numel() + 64, dtype=cuda.uint8, device="cuda")
+        at = 16 - moved.data_ptr() % 32 if moved.data_ptr() % 32 < 16 else 48 - moved.data_ptr() % 32
+        part = moved[at:at + a.numel()]
+        assert part.data_ptr() % 32 == 16
+        part.copy_(a)
+        t.arrays[name] = part
+        setattr(t.t, name, part.data_ptr())
+    for f, (r, c, k) in zip(flags, want):
+        assert cuda.equal(t.raycast(rays, f), r)
+        assert cuda.equal(t.closest(q, f), c)
+        assert cuda.equal(t.knn(q, 8, f), k)
+
+
+@pytest.mark.parametrize("kind", ["tri", "point", "gauss"])
+@pytest.mark.parametrize("k", [1, 3, 4, 5, 8, 11, 16, 17, 32])
+def test_knn_every_table(cuda, kind, k):
+    items = {"tri": lambda: workloads.terrain(12, 2), "point": lambda: _points(300, 5, 90),
+             "gauss": lambda: workloads.gaussians(300, 0.5, 20.0, 4)}[kind]()
+    c = items.reshape(len(items), -1)[:, :3]
+    q = workloads.uniform_points(403, c.min(0) - 5, c.max(0) + 5, 9, 13)
+    t, ref = capi.DeviceTree(kind, items), oracle.LBVH(kind, items)
+    t.build_wide()
+    want = ref.knn(q, k)
+    for f in (0, capi.QK_WIDE, capi.QK_TUNE_SPLIT4, capi.QK_TUNE_SPLIT8, capi.QK_TUNE_SPLIT):
+        assert np.array_equal(t.knn(_dev(q), k, f).cpu().numpy().view(np.uint32), want), f
+
+
+@pytest.mark.parametrize("smin,smax", [(0.05, 1.0), (1e-3, 30.0), (5.0, 5.0)])
+def test_ellipsoid_tests_end_early_with_the_same_bits(cuda, smin, smax):
+    """Needles, balls and plates: a test that stops once its distance is past the caller's limit
+    never changes a result (closest, kNN and radius against tests run to the end)."""
+    g = workloads.gaussians(1500, smin, smax, 8)
+    q = workloads.uniform_points(1500, [-20.0] * 3, [120.0] * 3, 8, 13)
+    t, ref = capi.DeviceTree("gauss", g), oracle.LBVH("gauss", g)
+    t.build_wide()
+    for f in (0, capi.QK_WIDE, capi.QK_TUNE_SPLIT):
+        assert np.array_equal(t.closest(_dev(q), f).cpu().numpy().view(np.uint32), ref.closest(q)), f
+        assert np.array_equal(t.knn(_dev(q), 6, f).cpu().numpy().view(np.uint32), ref.knn(q, 6)), f
+        off, keys = t.radius(_dev(q), 9.0, f)
+        woff, wkeys = ref.radius(q, 9.0)
+        assert np.array_equal(off.cpu().numpy().astype(np.int64), woff), f
+        assert np.array_equal(keys.cpu().numpy().view(np.uint64), wkeys), f
