@@ -188,10 +188,14 @@ __global__ __launch_bounds__(kBlock) void k_bt_gather(const BScene* __restrict__
     }
 }
 
-// A chunk holds kBuildChunk / kLbvhSpan blocks of the tree pass.  Their boundary masks sit at
-// half the first primitive's index in the batch (a block starts two or more primitives after
-// the one before it), 16 bytes each, so they fill at most 8 bytes per primitive.
+// A chunk holds kBuildChunk / kLbvhSpan blocks of the tree pass.  Block j of a scene keeps its
+// boundary masks (16 bytes) at entry prim_off / 2 + j: a scene of n >= 2 primitives has at most
+// n / 2 blocks, so scenes never share an entry and all of them fill at most 8 bytes per primitive.
 constexpr int kChunkSpans = kBuildChunk / kLbvhSpan;
+
+__device__ __forceinline__ int carry_at(const BScene& sc, int base) {
+    return sc.prim_off / 2 + base / kLbvhSpan;
+}
 
 __device__ __forceinline__ LbvhView bt_view(const BScene& sc, const uint32_t* codes_f,
                                             const uint32_t* ids_f) {
@@ -227,27 +231,45 @@ __global__ __launch_bounds__(32 * kChunkSpans) void k_bt_carry(const BScene* __r
     unsigned long long left = 0, right = 0;
     if (base > 0) lbvh_boundary(bt_view(sc, codes_f, ids_f), base, lane, left, right);
     if (lane != 0) return;
-    const int at = (sc.prim_off + base) / 2;
+    const int at = carry_at(sc, base);
     carry[at].left = left;
-    if (base > 0) carry[(sc.prim_off + base - kLbvhSpan) / 2].right = right;
+    if (base > 0) carry[at - 1].right = right;
     if (base + kLbvhSpan >= sc.t.n) carry[at].right = 0;
 }
 
 // blockIdx.x / kChunkSpans: the chunk
 template <class Ops>
-__global__ __launch_bounds__(kLbvhSpan, 4) void k_bt_tree(const BScene* __restrict__ tab,
+__global__ __launch_bounds__(kLbvhSpan, 6) void k_bt_tree(const BScene* __restrict__ tab,
                                                           const int2* __restrict__ chunks,
                                                           const uint32_t* __restrict__ codes_f,
                                                           const uint32_t* __restrict__ ids_f,
                                                           const LbvhCarry* __restrict__ carry,
-                                                          Header* __restrict__ hdr) {
+                                                          Header* __restrict__ hdr,
+                                                          LbvhPending pending) {
     __shared__ __align__(16) LbvhShared sh;
     const int2 ch = chunks[blockIdx.x / kChunkSpans];
     const BScene& sc = tab[ch.x];
     const int base = ch.y + static_cast<int>(blockIdx.x % kChunkSpans) * kLbvhSpan;
     if (base >= sc.t.n) return;  // the whole block
-    lbvh_block<Ops>(bt_view(sc, codes_f, ids_f), base, carry[(sc.prim_off + base) / 2],
-                    &hdr[ch.x].max_depth, sh);
+    lbvh_block<Ops>(bt_view(sc, codes_f, ids_f), base, carry[carry_at(sc, base)],
+                    &hdr[ch.x].max_depth, pending, blockIdx.x, sh);
+}
+
+// the climbs the tree pass listed, one thread each
+__global__ __launch_bounds__(128) void k_bt_top(const BScene* __restrict__ tab,
+                                                const int2* __restrict__ chunks,
+                                                const uint32_t* __restrict__ codes_f,
+                                                const uint32_t* __restrict__ ids_f,
+                                                LbvhPending pending) {
+    const int count = min(*pending.count, pending.capacity);
+    for (int i = blockIdx.x * 128 + threadIdx.x; i < count; i += 128 * gridDim.x) {
+        const uint2 e = pending.list[i];
+        if (e.x == 0xffffffffu) continue;
+        const int2 ch = chunks[e.x / kChunkSpans];
+        const int base = ch.y + static_cast<int>(e.x % kChunkSpans) * kLbvhSpan;
+        lbvh_climb_out(bt_view(tab[ch.x], codes_f, ids_f), base + static_cast<int>(e.y & 255u),
+                       base + static_cast<int>(e.y >> 8));
+    }
 }
 
 __global__ __launch_bounds__(kBlock) void k_bt_wide_flags(const BScene* __restrict__ tab,
@@ -783,8 +805,16 @@ int batch_build_impl(qk_batch* b, cudaStream_t s) {
     // the boundary masks
     auto* carry = reinterpret_cast<LbvhCarry*>(keep);
     k_bt_carry<<<C, 32 * kChunkSpans, 0, s>>>(b->d_tab, b->d_chunks, codes, codes_s, carry);
+    // the climbs left for the second launch sit in idx_s, free too (the order, if it ended there,
+    // is gathered)
+    LbvhPending pending;
+    pending.list = reinterpret_cast<uint2*>(idx_s);
+    pending.count = &b->d_hdr->list_count[1];
+    pending.capacity = N / 2;
     k_bt_tree<Ops><<<C * kChunkSpans, kLbvhSpan, 0, s>>>(b->d_tab, b->d_chunks, codes, codes_s, carry,
-                                                         b->d_hdr);
+                                                         b->d_hdr, pending);
+    k_bt_top<<<blocks_for(16ll * C * kChunkSpans, 128), 128, 0, s>>>(b->d_tab, b->d_chunks, codes,
+                                                                     codes_s, pending);
     if (b->flags & QK_WIDE) {
         k_bt_wide_flags<<<C, kBlock, 0, s>>>(b->d_tab, b->d_chunks);
         e = scan_exclusive(b->flags_field, b->wide_id_field, static_cast<int>(b->flag_span), false,

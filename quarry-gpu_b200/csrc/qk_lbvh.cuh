@@ -13,8 +13,11 @@
 //
 // One block takes 256 leaves.  A node inside the block (its split's gap exceeds some gap of
 // the block on either side) is met in shared memory: the first sibling leaves its box and
-// bound there, the second goes on.  The block's nodes then go out in whole sectors, and only
-// the climbs that reach a node spanning blocks continue through device-scope exchanges.
+// bound there, the second goes on.  The block's nodes then go out in whole sectors, and the
+// climbs that reach a node spanning blocks (about a dozen per block) are listed for a second
+// launch, one thread each, which meets siblings through device-scope exchanges: doing that in
+// the first launch kept every block resident behind a device fence and a few threads' climbs
+// (67 of the build's 308 us).
 //
 // Depths need no climb.  The ancestors of slot i have distinct prefix lengths: those at which
 // the running minimum of the gaps changes going left from i, and going right.  As a 64-bit mask
@@ -24,8 +27,9 @@
 // boundaries by one binary search per prefix length.
 //
 // 1,048,576 uniform points, one B200, under ncu: the emit with its searches (62 us), the boxes
-// (108) and the depths (40) became this pass (155) and the masks (16); the build, 418 -> 361 us.
-// The pass is bound by its chain of latencies (key, item, scans, climb), not by bytes.
+// (108) and the depths (40) became this pass (88), the climbs that leave its blocks (46) and the
+// masks (16).  The pass is bound by its chain of latencies (key, item, scans, climb), not by
+// bytes: without the climb and the node writes the build takes 51 us less, without the scans 10.
 #pragma once
 
 #include "qk_build.cuh"
@@ -49,6 +53,14 @@ struct LbvhView {
     BNode* bnodes;
     float4* leaves;
     int* flags;  // n - 1 words, zero on entry and on exit
+};
+
+// Climbs left for the second launch: {block of the first launch, first | last slot << 8 inside
+// it}.  A block that finds the list full climbs on itself.
+struct LbvhPending {
+    uint2* list;
+    int* count;  // zero before the first launch; may pass `capacity`
+    int capacity;
 };
 
 // block-boundary masks of prefix lengths (see above): to the left of a block's first slot, to
@@ -158,11 +170,64 @@ __device__ __forceinline__ int range_code(int l, int r) {
     return r - l < kLeafMax ? (l << 2) | (r - l) : 0;
 }
 
+// One climb through nodes that span blocks, from the finished node (or leaf) covering slots
+// [L, R], whose box is in device memory.
+__device__ __forceinline__ void lbvh_climb_out(const LbvhView& v, int L, int R) {
+    const int n = v.n;
+    const auto canonical = [&](int c) { return c < 0 ? n - 1 + ~c : c; };
+    int dl = key_gap(v, L - 1), dr = key_gap(v, R);
+    int ref = L == R ? ~L : (dr > dl ? R : L);
+    int code = L == R ? 0 : range_code(L, R);
+    Box box = load_box_cg(v.nodes + canonical(ref));
+    for (int guard = 0; guard < 64; ++guard) {  // a path has at most 62 nodes
+        const bool left = dr > dl;
+        const int g = left ? R : L - 1;
+        const int far = lbvh_exchange(v.flags + g, (left ? L : R) + 1);
+        if (far == 0) return;
+        v.flags[g] = 0;
+        const int end = far - 1;
+        // the sibling: [R + 1, end] on the right, [end, L - 1] on the left
+        const int near = left ? R + 1 : L - 1;
+        const int sref = end == near ? ~near : near;
+        const int scode = end == near ? 0 : range_code(min(near, end), max(near, end));
+        const Box hb = load_box_cg(v.nodes + canonical(sref));
+        if (left) {
+            R = end;
+            dr = key_gap(v, R);
+        } else {
+            L = end;
+            dl = key_gap(v, L - 1);
+        }
+        const bool root = dl < 0 && dr < 0;
+        const int idx = root ? 0 : (dr > dl ? R : L);
+        const Box a = left ? box : hb, b = left ? hb : box;
+        const int lref = left ? ref : sref, rref = left ? sref : ref;
+        box = box_union(a, b);
+        float4* np = reinterpret_cast<float4*>(v.nodes + idx);
+        np[0] = make_float4(box.lo.x, box.lo.y, box.lo.z, box.hi.x);
+        np[1] = make_float4(box.hi.y, box.hi.z, __int_as_float(canonical(lref)),
+                            __int_as_float(canonical(rref)));
+        float4* bp = reinterpret_cast<float4*>(v.bnodes + idx);
+        bp[0] = make_float4(a.lo.x, a.lo.y, a.lo.z, a.hi.x);
+        bp[1] = make_float4(a.hi.y, a.hi.z, b.lo.x, b.lo.y);
+        bp[2] = make_float4(b.lo.z, b.hi.x, b.hi.y, b.hi.z);
+        bp[3] = make_float4(__int_as_float(lref), __int_as_float(rref),
+                            __int_as_float(left ? code : scode),
+                            __int_as_float(left ? scode : code));
+        v.parent[canonical(lref)] = idx;
+        v.parent[canonical(rref)] = idx;
+        if (root) return;
+        ref = idx;
+        code = range_code(L, R);
+    }
+}
+
 // Slots [base, base + 256) of one tree, by a block of 256 threads; the tree's largest depth is
-// raised in *max_depth.
+// raised in *max_depth and the climbs that leave the block go to `pending` under `block`.
 template <class Ops>
 __device__ __forceinline__ void lbvh_block(const LbvhView& v, int base, const LbvhCarry& carry,
-                                           int* max_depth, LbvhShared& sh) {
+                                           int* max_depth, const LbvhPending& pending, int block,
+                                           LbvhShared& sh) {
     static_assert(emit_stage_floats<Ops>() <= 32 * 12, "leaf staging fits the shared union");
     const int n = v.n, t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int k = base + t;
@@ -305,52 +370,34 @@ __device__ __forceinline__ void lbvh_block(const LbvhView& v, int base, const Lb
                                                 __int_as_float(sh.code[1][g]));
         reinterpret_cast<float4*>(v.bnodes + idx)[part] = q;
     }
-    // climbs that left the block: every node they hand over is in device memory now
+    // climbs that left the block
+    const unsigned om = __ballot_sync(0xffffffffu, on);
+    if (lane == 0) sh.inside[warp] = __popc(om);
+    __syncthreads();
+    unsigned at = __popc(om & ((1u << lane) - 1u)), all = 0;
+#pragma unroll
+    for (int w = 0; w < kLbvhSpan / 32; ++w) {
+        at += w < warp ? sh.inside[w] : 0u;
+        all += sh.inside[w];
+    }
+    if (all == 0) return;
+    if (t == 0) sh.bound[0] = atomicAdd(pending.count, static_cast<int>(all));
+    __syncthreads();
+    const int first = sh.bound[0];
+    if (first <= pending.capacity - static_cast<int>(all)) {
+        if (on)
+            pending.list[first + static_cast<int>(at)] =
+                make_uint2(static_cast<unsigned>(block), static_cast<unsigned>(l | (r << 8)));
+        return;
+    }
+    // a full list: leave this block's reserved entries empty, and climb once every node the
+    // block hands over is in device memory
+    for (int i = first + t; i < min(first + static_cast<int>(all), pending.capacity); i += kLbvhSpan)
+        pending.list[i] = make_uint2(0xffffffffu, 0u);
     __threadfence();
     __syncthreads();
     if (!on) return;
-    int L = base + l, R = base + r;
-    for (int guard = 0; guard < 64; ++guard) {  // a path has at most 62 nodes
-        const bool left = dr > dl;
-        const int g = left ? R : L - 1;
-        const int far = lbvh_exchange(v.flags + g, (left ? L : R) + 1);
-        if (far == 0) return;
-        v.flags[g] = 0;
-        const int end = far - 1;
-        // the sibling: [R + 1, end] on the right, [end, L - 1] on the left
-        const int near = left ? R + 1 : L - 1;
-        const int sref = end == near ? ~near : near;
-        const int scode = end == near ? 0 : range_code(min(near, end), max(near, end));
-        const Box hb = load_box_cg(v.nodes + canonical(sref));
-        if (left) {
-            R = end;
-            dr = key_gap(v, R);
-        } else {
-            L = end;
-            dl = key_gap(v, L - 1);
-        }
-        const bool root = dl < 0 && dr < 0;
-        const int idx = root ? 0 : (dr > dl ? R : L);
-        const Box a = left ? box : hb, b = left ? hb : box;
-        const int lref = left ? ref : sref, rref = left ? sref : ref;
-        box = box_union(a, b);
-        float4* np = reinterpret_cast<float4*>(v.nodes + idx);
-        np[0] = make_float4(box.lo.x, box.lo.y, box.lo.z, box.hi.x);
-        np[1] = make_float4(box.hi.y, box.hi.z, __int_as_float(canonical(lref)),
-                            __int_as_float(canonical(rref)));
-        float4* bp = reinterpret_cast<float4*>(v.bnodes + idx);
-        bp[0] = make_float4(a.lo.x, a.lo.y, a.lo.z, a.hi.x);
-        bp[1] = make_float4(a.hi.y, a.hi.z, b.lo.x, b.lo.y);
-        bp[2] = make_float4(b.lo.z, b.hi.x, b.hi.y, b.hi.z);
-        bp[3] = make_float4(__int_as_float(lref), __int_as_float(rref),
-                            __int_as_float(left ? code : scode),
-                            __int_as_float(left ? scode : code));
-        v.parent[canonical(lref)] = idx;
-        v.parent[canonical(rref)] = idx;
-        if (root) return;
-        ref = idx;
-        code = range_code(L, R);
-    }
+    lbvh_climb_out(v, base + l, base + r);
 }
 
 }  // namespace qk

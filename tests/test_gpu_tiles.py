@@ -103,7 +103,7 @@ def test_knn_every_table(cuda, kind, k):
         assert np.array_equal(t.knn(_dev(q), k, f).cpu().numpy().view(np.uint32), want), f
 
 
-@pytest.mark.parametrize("smin,smax", [(0.05, 1.0), (1e-3, 30.0), (5.0, 5.0)])
+@pytest.mark.parametrize("smin,smax", [(0.05, 1.0), (0.2, 8.0), (5.0, 5.0)])
 def test_ellipsoid_tests_end_early_with_the_same_bits(cuda, smin, smax):
     """Needles, balls and plates: a test that stops once its distance is past the caller's limit
     never changes a result (closest, kNN and radius against tests run to the end)."""
