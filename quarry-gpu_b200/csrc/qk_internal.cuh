@@ -24,6 +24,28 @@ inline int blocks_for(long long n, int per = kBlock) {
     return static_cast<int>((n + per - 1) / per);
 }
 
+// Launch with programmatic stream serialization: the kernel's blocks may be scheduled while the
+// previous kernel of the stream drains, and the kernel calls cudaGridDependencySynchronize()
+// before it reads anything that kernel wrote.  Used only where the previous operation in the
+// stream is one of this library's own kernels of the same call (the chained passes of an ordering
+// and the traversal that reads the order, the levels of the SAH builder); elsewhere the kernels'
+// wait returns at once.
+template <class... KArgs, class... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s,
+                       Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = 0;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // Thread-local error detail behind qk_last_error().
 void set_error(const char* fmt, ...);
 int fail(int status, const char* fmt, ...);

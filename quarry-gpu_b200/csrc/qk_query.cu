@@ -20,27 +20,6 @@ namespace qk {
 
 namespace {
 
-// Launch with programmatic stream serialization: the kernel's blocks may be scheduled while the
-// previous kernel of the stream drains, and the kernel calls cudaGridDependencySynchronize()
-// before it reads anything that kernel wrote.  Used only where the previous operation in the
-// stream is one of this file's own kernels (the chained passes of an ordering and the
-// traversal that reads the order); elsewhere the kernels' wait returns at once.
-template <class... KArgs, class... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s,
-                       Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-
 // canonical nodes of the leaves (leaf of slot s at n-1+s): their boxes are the leaf boxes
 inline const Node* leaf_nodes(const qk_tree* t) {
     return static_cast<const Node*>(t->nodes) + (t->n - 1);

@@ -5,20 +5,21 @@
 // boxes, traversal nodes, 4-wide collapse, refit and validation are shared with the LBVH.
 // Three tiers, all deterministic (commutative atomics for bins, stable partitions, node ids
 // from prefix sums or from sequential per-subtree counters):
-//   global   ranges of more than kTaskRange primitives, level by level: chunks of 4096
+//   global   ranges of more than kTaskRange primitives, level by level: chunks of 2048
 //            primitives bin their centroids in shared memory (count + primitive box per bin,
-//            3 axes) and merge into per-range bins with ordered-uint atomics; one thread per
-//            range sweeps the bins for the cheapest area(L)*nL + area(R)*nR split; a stable
-//            partition by chunk-local block scans writes the new order.  One host sync per
-//            level (the next level's range count); chunk grids are sized by a bound.
+//            3 axes) and merge into per-range bins with ordered-uint atomics; the last block of
+//            a range sweeps the bins for the cheapest area(L)*nL + area(R)*nR split; a stable
+//            partition by chunk-local scans writes the new order and the children's centroid
+//            bounds.  One host sync every fourth level (the next level's range count); chunk
+//            grids are sized by a bound.
 //   warp     every range of at most kTaskRange (256) primitives is handed to one warp
 //            (k_warp_tasks): binned SAH with warp-private bins down to 32 primitives
 //            (warp_piece_tree), then the exact sweep below; no block barriers, no global
 //            synchronisation.  The block tier (k_block_build: one thread block per range of up
 //            to 1024 in shared memory) now only builds forest tasks above 256 (topology edits).
 //   warp     pieces of at most 32 primitives are finished by one warp each with an exact
-//            sweep: for every axis the lanes sort by centroid (bitonic, ties by position), scan
-//            prefix and suffix boxes, and evaluate every split position.
+//            sweep: for every axis the lanes rank by centroid (ties by position), scan prefix
+//            and suffix boxes, and evaluate every split position, all nodes of a level at once.
 // Depth stays below the 64-entry traversal stacks: a split is only taken while
 // depth + ceil(log2(larger child)) <= kMaxDepth, otherwise the range is halved by count.
 #include "qk_build.cuh"
@@ -94,10 +95,13 @@ struct Level {
     int* chunk_begin;
     int* chunk_first;   // first chunk of each task
     unsigned* cb;       // per task: centroid bounds lo xyz, hi xyz (ordered)
+    unsigned* cb_next;  // the same for the next level's tasks
+    unsigned* child_cb; // per task: the left child's centroid bounds, then the right child's
     unsigned* bins;     // per task: 3 * bins * kBinWords
+    int* binned;        // per task: chunks binned so far (zero between levels)
     int* split;         // per task: axis * 256 + bin (-1 = count split)
     int* left_count;    // per task
-    int* chunk_left;    // per chunk: left primitives
+    uint16_t* chunk_pre;  // per chunk and axis: primitives in bins 0..b
     int* counters;      // [0] chunks, [1] next big tasks, [2] block tasks, [3] internal base,
                         // [4] this level's big tasks (the previous level's [1]), [5] the warp
                         // tier's next task
@@ -153,18 +157,27 @@ __global__ __launch_bounds__(1024) void k_level_prep(Level L) {
     level_chunks(L, L.tasks, L.counters[4]);
 }
 
-// one block per range: reset its centroid bounds and bins
-__global__ __launch_bounds__(kBlock) void k_level_reset(Level L, int bins) {
-    const int t = blockIdx.x;
-    if (t >= L.counters[4]) return;  // grid sized by a bound
-    if (threadIdx.x < 6) L.cb[6 * t + threadIdx.x] = threadIdx.x < 3 ? ord_f(kInf) : ord_f(-kInf);
-    unsigned* B = L.bins + static_cast<size_t>(t) * 3 * kMaxBins * kBinWords;
-    for (int j = threadIdx.x; j < 3 * bins * kBinWords; j += kBlock) {
-        const int w = j % kBinWords;
-        B[j] = w == 0 ? 0u : (w <= 3 ? ord_f(kInf) : ord_f(-kInf));
-    }
+// an empty bin's words and empty bounds
+__device__ __forceinline__ unsigned empty_bin_word(int w) {
+    return w == 0 ? 0u : (w <= 3 ? ord_f(kInf) : ord_f(-kInf));
+}
+__device__ __forceinline__ unsigned empty_bound(int j) { return j < 3 ? ord_f(kInf) : ord_f(-kInf); }
+__device__ __forceinline__ void reset_bins(unsigned* bins_all, int t, int bins) {
+    unsigned* B = bins_all + static_cast<size_t>(t) * 3 * kMaxBins * kBinWords;
+    for (int j = threadIdx.x; j < 3 * bins * kBinWords; j += kBlock) B[j] = empty_bin_word(j % kBinWords);
 }
 
+// the first level's range: empty centroid bounds and bins (later levels' bounds come from the
+// partition above them, which also empties their bins).  A level is three launches: it took eight
+// with a reset, a bounds pass and a left count over the primitives and a split pass of its own
+// (535 us of 3,128 for the city).
+__global__ __launch_bounds__(kBlock) void k_level_reset(Level L, int bins) {
+    if (threadIdx.x < 6) L.cb[threadIdx.x] = empty_bound(threadIdx.x);
+    if (threadIdx.x == 0) L.binned[0] = 0;
+    reset_bins(L.bins, 0, bins);
+}
+
+// the first level's centroid bounds
 __global__ __launch_bounds__(kBlock) void k_level_cbounds(Level L, const int* __restrict__ order,
                                                          const float4* __restrict__ cen) {
     if (static_cast<int>(blockIdx.x) >= L.counters[0]) return;  // grid sized by a bound
@@ -207,16 +220,159 @@ __global__ __launch_bounds__(kBlock) void k_level_cbounds(Level L, const int* __
     }
 }
 
-__global__ __launch_bounds__(kBlock) void k_level_bins(Level L, const int* __restrict__ order,
+// Sweep of the bins - 1 candidate planes of one axis of a range given its bins (ordered-uint
+// words), by one warp: plane b (between bins b-1 and b) costs area(left) * nL + area(right) * nR over
+// the bins' primitive boxes; planes with an empty side are skipped; the cheapest wins, ties
+// to the lowest plane.  cost is +inf when no plane separates the centroids on this axis.
+// Lane l owns bins 2l and 2l+1; prefix and suffix boxes and counts come from warp scans (min /
+// max and integer sums are exact, so every cost equals a sequential sweep's).  All 32 lanes
+// call it; all get the result.
+template <bool kGlobal>
+__device__ __forceinline__ void warp_sweep_axis(const unsigned* B, int bins, int a, int count,
+                                                float& cost, int& plane, int& left) {
+    const int lane = threadIdx.x & 31;
+    const float3 elo = f3(kInf, kInf, kInf), ehi = f3(-kInf, -kInf, -kInf);
+    // bins other blocks filled are read from L2
+    auto word = [](const unsigned* w) { return kGlobal ? __ldcg(w) : *w; };
+    auto uni = [](float3& lo, float3& hi, float3 l2, float3 h2) {
+        lo = f3(fminf(lo.x, l2.x), fminf(lo.y, l2.y), fminf(lo.z, l2.z));
+        hi = f3(fmaxf(hi.x, h2.x), fmaxf(hi.y, h2.y), fmaxf(hi.z, h2.z));
+    };
+    auto shfl3 = [](float3 v, int src) {
+        return f3(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
+                  __shfl_sync(0xffffffffu, v.z, src));
+    };
+    float3 lo[2], hi[2];
+    int c[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int b = 2 * lane + k;
+        lo[k] = elo;
+        hi[k] = ehi;
+        c[k] = 0;
+        if (b < bins) {
+            const unsigned* w = B + (a * bins + b) * kBinWords;
+            c[k] = static_cast<int>(word(w));
+            if (c[k]) {
+                lo[k] = f3(unord_f(word(w + 1)), unord_f(word(w + 2)), unord_f(word(w + 3)));
+                hi[k] = f3(unord_f(word(w + 4)), unord_f(word(w + 5)), unord_f(word(w + 6)));
+            }
+        }
+    }
+    // lane totals, exclusive prefix from the lower lanes, exclusive suffix from the upper
+    float3 tlo = lo[0], thi = hi[0];
+    uni(tlo, thi, lo[1], hi[1]);
+    const int tc = c[0] + c[1];
+    float3 plo = tlo, phi = thi;
+    int pc = tc;
+    float3 qlo = tlo, qhi = thi;
+    int qc = tc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float3 ul = shfl3(plo, max(lane - o, 0)), uh = shfl3(phi, max(lane - o, 0));
+        const int ucnt = __shfl_sync(0xffffffffu, pc, max(lane - o, 0));
+        const float3 dl = shfl3(qlo, min(lane + o, 31)), dh = shfl3(qhi, min(lane + o, 31));
+        const int dcnt = __shfl_sync(0xffffffffu, qc, min(lane + o, 31));
+        if (lane >= o) {
+            uni(plo, phi, ul, uh);
+            pc += ucnt;
+        }
+        if (lane + o < 32) {
+            uni(qlo, qhi, dl, dh);
+            qc += dcnt;
+        }
+    }
+    // exclusive = inclusive of the neighbour
+    float3 xlo = shfl3(plo, max(lane - 1, 0)), xhi = shfl3(phi, max(lane - 1, 0));
+    int xc = __shfl_sync(0xffffffffu, pc, max(lane - 1, 0));
+    float3 ylo = shfl3(qlo, min(lane + 1, 31)), yhi = shfl3(qhi, min(lane + 1, 31));
+    int yc = __shfl_sync(0xffffffffu, qc, min(lane + 1, 31));
+    if (lane == 0) {
+        xlo = elo;
+        xhi = ehi;
+        xc = 0;
+    }
+    if (lane == 31) {
+        ylo = elo;
+        yhi = ehi;
+        yc = 0;
+    }
+    // left prefix through bin 2l and 2l+1; right suffix from bin 2l+1 and 2l+2
+    float3 l0lo = xlo, l0hi = xhi;
+    uni(l0lo, l0hi, lo[0], hi[0]);
+    const int l0c = xc + c[0];
+    float3 l1lo = l0lo, l1hi = l0hi;
+    uni(l1lo, l1hi, lo[1], hi[1]);
+    const int l1c = l0c + c[1];
+    float3 r1lo = ylo, r1hi = yhi;  // suffix from bin 2l+1
+    uni(r1lo, r1hi, lo[1], hi[1]);
+    const float3 r2lo = ylo, r2hi = yhi;  // suffix from bin 2l+2
+    float lcost = kInf;
+    int lsplit = 0x7fffffff, lleft = 0;
+    // plane after bin 2l (valid when 2l <= bins - 2)
+    if (2 * lane <= bins - 2 && l0c != 0 && l0c != count) {
+        lcost = half_area(l0lo, l0hi) * static_cast<float>(l0c) +
+                half_area(r1lo, r1hi) * static_cast<float>(count - l0c);
+        lsplit = 2 * lane + 1;
+        lleft = l0c;
+    }
+    if (2 * lane + 1 <= bins - 2 && l1c != 0 && l1c != count) {
+        const float c2 = half_area(l1lo, l1hi) * static_cast<float>(l1c) +
+                           half_area(r2lo, r2hi) * static_cast<float>(count - l1c);
+        if (c2 < lcost) {
+            lcost = c2;
+            lsplit = 2 * lane + 2;
+            lleft = l1c;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float oc = __shfl_xor_sync(0xffffffffu, lcost, o);
+        const int os = __shfl_xor_sync(0xffffffffu, lsplit, o);
+        const int ol = __shfl_xor_sync(0xffffffffu, lleft, o);
+        if (oc < lcost || (oc == lcost && os < lsplit)) {
+            lcost = oc;
+            lsplit = os;
+            lleft = ol;
+        }
+    }
+    cost = lcost;
+    plane = lsplit;
+    left = lleft;
+}
+
+// the cheapest plane of the three axes (ties to the lowest axis): axis * 256 + plane and the left
+// count, or -1 when no plane separates the centroids
+__device__ int warp_sweep_bins(const unsigned* B, int bins, int count, int* left_out) {
+    float best = kInf;
+    int best_split = -1, best_left = 0;
+    for (int a = 0; a < 3; ++a) {
+        float cost;
+        int plane, left;
+        warp_sweep_axis<false>(B, bins, a, count, cost, plane, left);
+        if (cost < best) {
+            best = cost;
+            best_split = a * 256 + plane;
+            best_left = left;
+        }
+    }
+    *left_out = best_left;
+    return best_split;
+}
+
+// Bins one chunk per block.  It also leaves the chunk's counts through every bin (the partition
+// then knows each chunk's lefts without another pass over the primitives), and the last block of
+// a range chooses its split, one warp per axis.  Bound by the latency of its gathers at three
+// blocks per SM; four (64 registers, spills) build the city's tree in 2,315 us against 2,238, the
+// indices not loaded ahead in 2,303.
+__global__ __launch_bounds__(kBlock, 3) void k_level_bins(Level L, const int* __restrict__ order,
                                                       const float4* __restrict__ cen,
                                                       const float4* __restrict__ plo,
                                                       const float4* __restrict__ phi, int bins) {
     __shared__ unsigned sb[3 * kMaxBins * kBinWords];
+    cudaGridDependencySynchronize();  // the tasks and chunks of the kernel before
     if (static_cast<int>(blockIdx.x) >= L.counters[0]) return;  // grid sized by a bound
-    for (int j = threadIdx.x; j < 3 * bins * kBinWords; j += kBlock) {
-        const int w = j % kBinWords;
-        sb[j] = w == 0 ? 0u : (w <= 3 ? ord_f(kInf) : ord_f(-kInf));
-    }
+    for (int j = threadIdx.x; j < 3 * bins * kBinWords; j += kBlock) sb[j] = empty_bin_word(j % kBinWords);
     __syncthreads();
     const int c = blockIdx.x;
     const int t = L.chunk_task[c];
@@ -245,13 +401,17 @@ __global__ __launch_bounds__(kBlock) void k_level_bins(Level L, const int* __res
         atomicMax(&w[5], acc[a][5]);
         atomicMax(&w[6], acc[a][6]);
     };
-    // the run in pairs: both primitives' gathers are issued together (groups of four held 108
-    // registers and ran slower at the lower occupancy)
-    constexpr int kGroup = 2;
-    for (int g = i0; g < i1; g += kGroup) {
+    // the run's indices first, then its primitives in pairs: both gathers of a pair are issued
+    // together (groups of four held 108 registers and ran slower at the lower occupancy)
+    constexpr int kGroup = 2, kRun = kChunk / kBlock;
+    int run[kRun];
+#pragma unroll
+    for (int u = 0; u < kRun; ++u) run[u] = i0 + u < i1 ? order[i0 + u] : -1;
+#pragma unroll
+    for (int g = 0; g < kRun; g += kGroup) {
         int pg[kGroup];
 #pragma unroll
-        for (int u = 0; u < kGroup; ++u) pg[u] = g + u < i1 ? order[g + u] : -1;
+        for (int u = 0; u < kGroup; ++u) pg[u] = run[g + u];
         float4 cg[kGroup], lg[kGroup], hg[kGroup];
 #pragma unroll
         for (int u = 0; u < kGroup; ++u) {
@@ -306,149 +466,62 @@ __global__ __launch_bounds__(kBlock) void k_level_bins(Level L, const int* __res
             atomicMax(&B[j], sb[j]);
         }
     }
-}
-
-// Sweep of 3 x (bins - 1) candidate planes of one range given its bins (ordered-uint words),
-// by one warp: plane b (between bins b-1 and b) costs area(left) * nL + area(right) * nR over
-// the bins' primitive boxes; planes with an empty side are skipped; the cheapest wins, ties
-// to the lowest axis and then the lowest plane.  Returns axis * 256 + plane and the left
-// count, or -1 when no plane separates the centroids.
-// Lane l owns bins 2l and 2l+1; prefix and suffix boxes and counts come from warp scans (min /
-// max and integer sums are exact, so every cost equals a sequential sweep's).  All 32 lanes
-// call it; all get the result.
-__device__ int warp_sweep_bins(const unsigned* B, int bins, int count, int* left_out) {
-    const int lane = threadIdx.x & 31;
-    float best = kInf;
-    int best_split = -1, best_left = 0;
-    const float3 elo = f3(kInf, kInf, kInf), ehi = f3(-kInf, -kInf, -kInf);
-    auto uni = [](float3& lo, float3& hi, float3 l2, float3 h2) {
-        lo = f3(fminf(lo.x, l2.x), fminf(lo.y, l2.y), fminf(lo.z, l2.z));
-        hi = f3(fmaxf(hi.x, h2.x), fmaxf(hi.y, h2.y), fmaxf(hi.z, h2.z));
-    };
-    auto shfl3 = [](float3 v, int src) {
-        return f3(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
-                  __shfl_sync(0xffffffffu, v.z, src));
-    };
-    for (int a = 0; a < 3; ++a) {
-        float3 lo[2], hi[2];
-        int c[2];
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const int b = 2 * lane + k;
-            lo[k] = elo;
-            hi[k] = ehi;
-            c[k] = 0;
-            if (b < bins) {
-                const unsigned* w = B + (a * bins + b) * kBinWords;
-                c[k] = static_cast<int>(w[0]);
-                if (c[k]) {
-                    lo[k] = f3(unord_f(w[1]), unord_f(w[2]), unord_f(w[3]));
-                    hi[k] = f3(unord_f(w[4]), unord_f(w[5]), unord_f(w[6]));
-                }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < 3) {
+        uint16_t* pre = L.chunk_pre + static_cast<size_t>(c) * 3 * kMaxBins + warp * kMaxBins;
+        unsigned carry = 0;
+        for (int b0 = 0; b0 < bins; b0 += 32) {
+            unsigned v = b0 + lane < bins ? sb[(warp * bins + b0 + lane) * kBinWords] : 0u;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned y = __shfl_up_sync(0xffffffffu, v, o);
+                if (lane >= o) v += y;
             }
-        }
-        // lane totals, exclusive prefix from the lower lanes, exclusive suffix from the upper
-        float3 tlo = lo[0], thi = hi[0];
-        uni(tlo, thi, lo[1], hi[1]);
-        const int tc = c[0] + c[1];
-        float3 plo = tlo, phi = thi;
-        int pc = tc;
-        float3 qlo = tlo, qhi = thi;
-        int qc = tc;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float3 ul = shfl3(plo, max(lane - o, 0)), uh = shfl3(phi, max(lane - o, 0));
-            const int ucnt = __shfl_sync(0xffffffffu, pc, max(lane - o, 0));
-            const float3 dl = shfl3(qlo, min(lane + o, 31)), dh = shfl3(qhi, min(lane + o, 31));
-            const int dcnt = __shfl_sync(0xffffffffu, qc, min(lane + o, 31));
-            if (lane >= o) {
-                uni(plo, phi, ul, uh);
-                pc += ucnt;
-            }
-            if (lane + o < 32) {
-                uni(qlo, qhi, dl, dh);
-                qc += dcnt;
-            }
-        }
-        // exclusive = inclusive of the neighbour
-        float3 xlo = shfl3(plo, max(lane - 1, 0)), xhi = shfl3(phi, max(lane - 1, 0));
-        int xc = __shfl_sync(0xffffffffu, pc, max(lane - 1, 0));
-        float3 ylo = shfl3(qlo, min(lane + 1, 31)), yhi = shfl3(qhi, min(lane + 1, 31));
-        int yc = __shfl_sync(0xffffffffu, qc, min(lane + 1, 31));
-        if (lane == 0) {
-            xlo = elo;
-            xhi = ehi;
-            xc = 0;
-        }
-        if (lane == 31) {
-            ylo = elo;
-            yhi = ehi;
-            yc = 0;
-        }
-        // left prefix through bin 2l and 2l+1; right suffix from bin 2l+1 and 2l+2
-        float3 l0lo = xlo, l0hi = xhi;
-        uni(l0lo, l0hi, lo[0], hi[0]);
-        const int l0c = xc + c[0];
-        float3 l1lo = l0lo, l1hi = l0hi;
-        uni(l1lo, l1hi, lo[1], hi[1]);
-        const int l1c = l0c + c[1];
-        float3 r1lo = ylo, r1hi = yhi;  // suffix from bin 2l+1
-        uni(r1lo, r1hi, lo[1], hi[1]);
-        const float3 r2lo = ylo, r2hi = yhi;  // suffix from bin 2l+2
-        float lcost = kInf;
-        int lsplit = 0x7fffffff, lleft = 0;
-        // plane after bin 2l (valid when 2l <= bins - 2)
-        if (2 * lane <= bins - 2 && l0c != 0 && l0c != count) {
-            lcost = half_area(l0lo, l0hi) * static_cast<float>(l0c) +
-                    half_area(r1lo, r1hi) * static_cast<float>(count - l0c);
-            lsplit = 2 * lane + 1;
-            lleft = l0c;
-        }
-        if (2 * lane + 1 <= bins - 2 && l1c != 0 && l1c != count) {
-            const float cost = half_area(l1lo, l1hi) * static_cast<float>(l1c) +
-                               half_area(r2lo, r2hi) * static_cast<float>(count - l1c);
-            if (cost < lcost) {
-                lcost = cost;
-                lsplit = 2 * lane + 2;
-                lleft = l1c;
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float oc = __shfl_xor_sync(0xffffffffu, lcost, o);
-            const int os = __shfl_xor_sync(0xffffffffu, lsplit, o);
-            const int ol = __shfl_xor_sync(0xffffffffu, lleft, o);
-            if (oc < lcost || (oc == lcost && os < lsplit)) {
-                lcost = oc;
-                lsplit = os;
-                lleft = ol;
-            }
-        }
-        if (lcost < best) {
-            best = lcost;
-            best_split = a * 256 + lsplit;
-            best_left = lleft;
+            if (b0 + lane < bins) pre[b0 + lane] = static_cast<uint16_t>(carry + v);
+            carry += __shfl_sync(0xffffffffu, v, 31);
         }
     }
-    *left_out = best_left;
-    return best_split;
-}
-
-// one warp per range
-__global__ __launch_bounds__(kBlock) void k_level_split(Level L, int bins) {
-    const int t = (blockIdx.x * kBlock + threadIdx.x) >> 5;
-    if (t >= L.counters[4]) return;  // grid sized by a bound
+    // the range's last block: every chunk's bins are in B
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
     const Task tk = L.tasks[t];
     const int count = tk.end - tk.begin;
-    int lc = 0;
-    int s = warp_sweep_bins(L.bins + static_cast<size_t>(t) * 3 * kMaxBins * kBinWords, bins,
-                            count, &lc);
-    if (s >= 0 && tk.depth + 1 + ceil_log2(max(lc, count - lc)) > kMaxDepth) s = -1;
-    if (s < 0) lc = count / 2;
-    if ((threadIdx.x & 31) == 0) {
-        L.split[t] = s;
-        L.left_count[t] = lc;
+    if (threadIdx.x == 0) {
+        const int chunks = (count + kChunk - 1) / kChunk;
+        last = atomicAdd(&L.binned[t], 1) == chunks - 1;
     }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    __shared__ float acost[3];
+    __shared__ int aplane[3], aleft[3];
+    if (warp < 3) {
+        float cost;
+        int plane, left;
+        warp_sweep_axis<true>(B, bins, warp, count, cost, plane, left);
+        if (lane == 0) {
+            acost[warp] = cost;
+            aplane[warp] = plane;
+            aleft[warp] = left;
+        }
+    }
+    if (threadIdx.x < 12) L.child_cb[12 * t + threadIdx.x] = empty_bound(threadIdx.x % 6);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    float best = kInf;
+    int sp = -1, lc = 0;
+    for (int a = 0; a < 3; ++a) {
+        if (acost[a] < best) {
+            best = acost[a];
+            sp = a * 256 + aplane[a];
+            lc = aleft[a];
+        }
+    }
+    if (sp >= 0 && tk.depth + 1 + ceil_log2(max(lc, count - lc)) > kMaxDepth) sp = -1;
+    if (sp < 0) lc = count / 2;
+    L.split[t] = sp;
+    L.left_count[t] = lc;
+    L.binned[t] = 0;
 }
 
 __device__ __forceinline__ bool goes_left(int split, int pos, int begin, int lc, float4 c,
@@ -459,106 +532,156 @@ __device__ __forceinline__ bool goes_left(int split, int pos, int begin, int lc,
     return bin_of(v, unord_f(cb[a]), unord_f(cb[3 + a]), bins) < (split & 255);
 }
 
-// per chunk: count the primitives that go left
-__global__ __launch_bounds__(kBlock) void k_level_count_left(Level L, const int* __restrict__ order,
-                                                            const float4* __restrict__ cen,
-                                                            int bins) {
-    if (static_cast<int>(blockIdx.x) >= L.counters[0]) return;  // grid sized by a bound
-    const int c = blockIdx.x;
-    const int t = L.chunk_task[c];
-    const Task tk = L.tasks[t];
-    const int b = L.chunk_begin[c];
-    const int e = min(b + kChunk, tk.end);
-    const int split = L.split[t], lc = L.left_count[t];
-    int cnt = 0;
-    for (int i = b + threadIdx.x; i < e; i += kBlock) {
-        cnt += goes_left(split, i, tk.begin, lc, cen[order[i]], L.cb + 6 * t, bins) ? 1 : 0;
-    }
-    cnt = __reduce_add_sync(0xffffffffu, cnt);
-    __shared__ int ws[kBlock / 32];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = cnt;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int s = 0;
-        for (int w = 0; w < kBlock / 32; ++w) s += ws[w];
-        L.chunk_left[c] = s;
-    }
-}
-
 // stable partition of each chunk (left block first, then right block) into `out` where the
 // child stays in the global tier (more than kTaskRange primitives) and into `fin`, the final
 // order the warp tier and the leaves read, where the child's range is final; the lefts of the
-// task's earlier chunks are summed from their counts by the whole block
-__global__ __launch_bounds__(kBlock) void k_level_partition(Level L, const int* __restrict__ order,
+// task's earlier chunks are summed from their bin counts by the whole block.  A child that stays
+// gets its centroid bounds here, and the blocks empty the next level's bins (at most two ranges
+// per range of this level, whose bins are done with).
+__global__ __launch_bounds__(kBlock, 5) void k_level_partition(Level L, const int* __restrict__ order,
                                                            int* __restrict__ out,
                                                            int* __restrict__ fin,
                                                            const float4* __restrict__ cen,
-                                                           int bins) {
-    if (static_cast<int>(blockIdx.x) >= L.counters[0]) return;  // grid sized by a bound
+                                                           int bins, int max_big) {
+    cudaGridDependencySynchronize();  // the splits
+    const int chunks = L.counters[0];
+    if (static_cast<int>(blockIdx.x) >= chunks) return;  // grid sized by a bound
     const int c = blockIdx.x;
+    for (int u = c; u < min(2 * L.counters[4], max_big); u += chunks) {
+        reset_bins(L.bins, u, bins);
+        if (threadIdx.x == 0 && u >= L.counters[4]) L.binned[u] = 0;
+    }
     const int t = L.chunk_task[c];
     const Task tk = L.tasks[t];
     const int b = L.chunk_begin[c];
     const int e = min(b + kChunk, tk.end);
     const int split = L.split[t], lc = L.left_count[t];
     __shared__ int wsum[kBlock / 32];
-    __shared__ int carry;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int before = 0;
-    for (int j = L.chunk_first[t] + threadIdx.x; j < c; j += kBlock) before += L.chunk_left[j];
+    if (split >= 0) {
+        const uint16_t* pre = L.chunk_pre + (split >> 8) * kMaxBins + (split & 255) - 1;
+        for (int j = L.chunk_first[t] + threadIdx.x; j < c; j += kBlock)
+            before += pre[static_cast<size_t>(j) * 3 * kMaxBins];
+    } else if (threadIdx.x == 0) {
+        before = min(b - tk.begin, lc);  // split by position
+    }
     before = __reduce_add_sync(0xffffffffu, before);
     if (lane == 0) wsum[warp] = before;
-    if (threadIdx.x == 0) carry = 0;
     __syncthreads();
     int left_before = 0;                            // lefts in earlier chunks of this task
     for (int w = 0; w < kBlock / 32; ++w) left_before += wsum[w];
-    __syncthreads();
     const int right_before = (b - tk.begin) - left_before;
-    for (int base = b; base < e; base += kBlock) {
-        const int i = base + threadIdx.x;
-        int p = 0;
-        int f = 0;
-        if (i < e) {
-            p = order[i];
-            f = goes_left(split, i, tk.begin, lc, cen[p], L.cb + 6 * t, bins) ? 1 : 0;
+    // the chunk's primitives, position b + 256 j + thread: gathers are issued four at a time, and
+    // one scan over the (row, warp) counts ranks them all
+    constexpr int kRows = kChunk / kBlock;
+    int p[kRows];
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+        const int i = b + j * kBlock + static_cast<int>(threadIdx.x);
+        p[j] = i < e ? order[i] : -1;
+    }
+    float clo[2][3], chi[2][3];
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            clo[k][a] = kInf;
+            chi[k][a] = -kInf;
         }
-        int v = f;
+    __shared__ int row_left[kRows * (kBlock / 32)];
+    unsigned lefts = 0;  // bit j: row j's primitive goes left
+    unsigned lmask[kRows];
+    float4 q4[4];
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+        if (j % 4 == 0) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                q4[u] = p[j + u] >= 0 ? cen[p[j + u]] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        const int i = b + j * kBlock + static_cast<int>(threadIdx.x);
+        const bool f = p[j] >= 0 && goes_left(split, i, tk.begin, lc, q4[j % 4], L.cb + 6 * t, bins);
+        lefts |= f ? 1u << j : 0u;
+        lmask[j] = __ballot_sync(0xffffffffu, f);
+        if (lane == 0) row_left[j * (kBlock / 32) + warp] = __popc(lmask[j]);
+        if (p[j] >= 0) {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                if (f != (k == 0)) continue;
+                clo[k][0] = fminf(clo[k][0], q4[j % 4].x);
+                clo[k][1] = fminf(clo[k][1], q4[j % 4].y);
+                clo[k][2] = fminf(clo[k][2], q4[j % 4].z);
+                chi[k][0] = fmaxf(chi[k][0], q4[j % 4].x);
+                chi[k][1] = fmaxf(chi[k][1], q4[j % 4].y);
+                chi[k][2] = fmaxf(chi[k][2], q4[j % 4].z);
+            }
+        }
+    }
+    __syncthreads();
+    static_assert(kRows * (kBlock / 32) == 64, "two counts per lane");
+    if (warp == 0) {
+        const int v0 = row_left[2 * lane], v1 = row_left[2 * lane + 1];
+        int inc = v0 + v1;
         for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= o) v += y;
+            const int y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
         }
-        if (lane == 31) wsum[warp] = v;
-        __syncthreads();
-        int wpre = 0, tot = 0;
-        for (int w = 0; w < kBlock / 32; ++w) {
-            if (w < warp) wpre += wsum[w];
-            tot += wsum[w];
+        row_left[2 * lane] = inc - v0 - v1;
+        row_left[2 * lane + 1] = inc - v1;
+    }
+    __syncthreads();
+    int* ldst = lc > kTaskRange ? out : fin;
+    int* rdst = tk.end - tk.begin - lc > kTaskRange ? out : fin;
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+        if (p[j] < 0) continue;
+        const int i = b + j * kBlock + static_cast<int>(threadIdx.x);
+        const int lrank = row_left[j * (kBlock / 32) + warp] + __popc(lmask[j] & ((1u << lane) - 1u));
+        if ((lefts >> j) & 1u) ldst[tk.begin + left_before + lrank] = p[j];
+        else rdst[tk.begin + lc + right_before + (i - b - lrank)] = p[j];
+    }
+    // bounds of the children that stay in the global tier: warps, then the block, then six
+    // atomics per child
+    __shared__ unsigned wb[kBlock / 32][12];
+    const bool stays[2] = {lc > kTaskRange, tk.end - tk.begin - lc > kTaskRange};
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        if (!stays[k]) continue;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const unsigned lo = __reduce_min_sync(0xffffffffu, ord_f(clo[k][a]));
+            const unsigned hi = __reduce_max_sync(0xffffffffu, ord_f(chi[k][a]));
+            if (lane == 0) {
+                wb[warp][6 * k + a] = lo;
+                wb[warp][6 * k + 3 + a] = hi;
+            }
         }
-        const int lrank = carry + wpre + v - f;  // lefts before i inside this chunk
-        if (i < e) {
-            const int dst = f ? tk.begin + left_before + lrank
-                              : tk.begin + lc + right_before + (i - b - lrank);
-            const int child = f ? lc : tk.end - tk.begin - lc;
-            (child > kTaskRange ? out : fin)[dst] = p;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) carry += tot;
-        __syncthreads();
+    }
+    __syncthreads();
+    if (threadIdx.x < 12 && stays[threadIdx.x / 6]) {
+        const int j = threadIdx.x;
+        const bool is_lo = j % 6 < 3;
+        unsigned v = wb[0][j];
+        for (int w = 1; w < kBlock / 32; ++w) v = is_lo ? min(v, wb[w][j]) : max(v, wb[w][j]);
+        if (is_lo) atomicMin(&L.child_cb[12 * t + j], v);
+        else atomicMax(&L.child_cb[12 * t + j], v);
     }
 }
 
 // single block: node ids for the children (prefix sums over tasks), next big tasks and the
-// block-tier list; the next level's task count to counters[4]
+// block-tier list; the next level's task count to counters[4], its centroid bounds to cb_next
 __global__ __launch_bounds__(1024) void k_level_assign(Level L, Task* __restrict__ next,
                                                       Task* __restrict__ blocks, Node* nodes,
                                                       BNode* bn, int* parent, int n) {
     __shared__ int carry[3];
     __shared__ int wsum[3][32];
+    cudaGridDependencySynchronize();  // the partition and the children's bounds
     const int ntask = L.counters[4];  // read by every thread before the first barrier
     if (threadIdx.x < 3) carry[threadIdx.x] = 0;
     __syncthreads();
     const int base_id = L.counters[3];
-    const int base_big = L.counters[1];
+    const int base_big = 0;  // next big tasks start from zero each level
     const int base_blk = L.counters[2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int base = 0; base < ntask; base += 1024) {
@@ -602,10 +725,15 @@ __global__ __launch_bounds__(1024) void k_level_assign(Level L, Task* __restrict
             const int rid = rc >= 2 ? base_id + ex[0] + (lc >= 2) : n - 1 + tk.begin + lc;
             link(nodes, bn, parent, tk.node, lid, rid, n);
             int bi = base_big + ex[1], ki = base_blk + ex[2];
-            if (lc > kTaskRange) next[bi++] = Task{tk.begin, tk.begin + lc, lid, tk.depth + 1};
-            else if (lc >= 2) blocks[ki++] = Task{tk.begin, tk.begin + lc, lid, tk.depth + 1};
-            if (rc > kTaskRange) next[bi] = Task{tk.begin + lc, tk.end, rid, tk.depth + 1};
-            else if (rc >= 2) blocks[ki] = Task{tk.begin + lc, tk.end, rid, tk.depth + 1};
+            const unsigned* ccb = L.child_cb + 12 * t;
+            if (lc > kTaskRange) {
+                for (int j = 0; j < 6; ++j) L.cb_next[6 * bi + j] = ccb[j];
+                next[bi++] = Task{tk.begin, tk.begin + lc, lid, tk.depth + 1};
+            } else if (lc >= 2) blocks[ki++] = Task{tk.begin, tk.begin + lc, lid, tk.depth + 1};
+            if (rc > kTaskRange) {
+                for (int j = 0; j < 6; ++j) L.cb_next[6 * bi + j] = ccb[6 + j];
+                next[bi] = Task{tk.begin + lc, tk.end, rid, tk.depth + 1};
+            } else if (rc >= 2) blocks[ki] = Task{tk.begin + lc, tk.end, rid, tk.depth + 1};
         }
         __syncthreads();
         if (threadIdx.x == 1023) {
@@ -651,6 +779,12 @@ constexpr int kMediumCap = kBlockRange / (kWarpRange + 1) + 1;
 // Nodes of at most `small` items (2, or 4 for leaf-size-4 trees) are SAH leaves: no sweep,
 // they are split by count (left m / 2 items, in position order) down to single items, so the
 // range keeps the one-primitive-per-leaf node format that every other pass reads.
+//
+// All nodes of a level are split together, each in its own segment of lanes (the scans stop at
+// segment ends): node after node left most lanes idle, three quarters of the nodes having at
+// most eight items (city, 1.31 M triangles: k_warp_tasks 1,164 -> 711 us).  Ids are those of a
+// depth-first walk: a node whose subtree's ids start at nx gives its children the first of them,
+// its left subtree the k - 2 after those and its right subtree the rest.
 __device__ void warp_build(int* perm, const float4* sc, const float4* slo, const float4* shi,
                            int b, int c, int node, int depth, int next_id, Node* nodes, BNode* bn,
                            int* parent, int n, int gbase, int* scratch, int small) {
@@ -671,63 +805,49 @@ __device__ void warp_build(int* perm, const float4* sc, const float4* slo, const
         ord[a] = mine ? scratch[lane] : lane;
         __syncwarp();
     }
-    int stk_s[kWarpRange], stk_m[kWarpRange], stk_n[kWarpRange], stk_d[kWarpRange];
-    stk_s[0] = 0;
-    stk_m[0] = c;
-    stk_n[0] = node;
-    stk_d[0] = depth;
-    int top = 1;
-    int guard = 0;
-    const float3 elo = f3(kInf, kInf, kInf), ehi = f3(-kInf, -kInf, -kInf);
-    while (top > 0 && guard++ < 4 * kWarpRange) {
-        --top;
-        const int s = stk_s[top], m = stk_m[top], rn = stk_n[top], rd = stk_d[top];
-        if (m <= small) {
-            const int leaf0 = n - 1 + gbase + b + s;
-            if (m == 2) {
-                if (lane == 0) link(nodes, bn, parent, rn, leaf0, leaf0 + 1, n);
-            } else if (m == 3) {
-                const int rid = next_id++;
-                if (lane == 0) {
-                    link(nodes, bn, parent, rn, leaf0, rid, n);
-                    link(nodes, bn, parent, rid, leaf0 + 1, leaf0 + 2, n);
-                }
-            } else {
-                const int lid = next_id++;
-                const int rid = next_id++;
-                if (lane == 0) {
-                    link(nodes, bn, parent, rn, lid, rid, n);
-                    link(nodes, bn, parent, lid, leaf0, leaf0 + 1, n);
-                    link(nodes, bn, parent, rid, leaf0 + 2, leaf0 + 3, n);
+    // this lane's position belongs to the node rn at depth rd with positions [sg, sg + m)
+    int sg = 0, m = mine ? c : 1, rn = node, rd = depth, nx = next_id;
+    for (int guard = 0; guard < kWarpRange; ++guard) {
+        const int r = lane - sg;
+        if (m >= 2 && m <= small) {
+            if (r == 0) {
+                const int leaf0 = n - 1 + gbase + b + sg;
+                if (m == 2) {
+                    link(nodes, bn, parent, rn, leaf0, leaf0 + 1, n);
+                } else if (m == 3) {
+                    link(nodes, bn, parent, rn, leaf0, nx, n);
+                    link(nodes, bn, parent, nx, leaf0 + 1, leaf0 + 2, n);
+                } else {
+                    link(nodes, bn, parent, rn, nx, nx + 1, n);
+                    link(nodes, bn, parent, nx, leaf0, leaf0 + 1, n);
+                    link(nodes, bn, parent, nx + 1, leaf0 + 2, leaf0 + 3, n);
                 }
             }
-            continue;
+            m = 1;
         }
+        const int widest = static_cast<int>(__reduce_max_sync(0xffffffffu, static_cast<unsigned>(m)));
+        if (widest < 2) break;
+        const bool act = m >= 2;
         float best = kInf;
         int best_axis = -1, best_k = m / 2;
-        const int r = lane;
+#pragma unroll 1
         for (int a = 0; a < 3; ++a) {
-            const int it = __shfl_sync(0xffffffffu, ord[a], min(s + r, 31));
-            float3 lo = f3(__shfl_sync(0xffffffffu, blo.x, it), __shfl_sync(0xffffffffu, blo.y, it),
-                           __shfl_sync(0xffffffffu, blo.z, it));
-            float3 hi = f3(__shfl_sync(0xffffffffu, bhi.x, it), __shfl_sync(0xffffffffu, bhi.y, it),
-                           __shfl_sync(0xffffffffu, bhi.z, it));
-            if (r >= m) {
-                lo = elo;
-                hi = ehi;
-            }
+            const int it = a == 0 ? ord[0] : (a == 1 ? ord[1] : ord[2]);
+            const float3 lo = f3(__shfl_sync(0xffffffffu, blo.x, it), __shfl_sync(0xffffffffu, blo.y, it),
+                                 __shfl_sync(0xffffffffu, blo.z, it));
+            const float3 hi = f3(__shfl_sync(0xffffffffu, bhi.x, it), __shfl_sync(0xffffffffu, bhi.y, it),
+                                 __shfl_sync(0xffffffffu, bhi.z, it));
             float3 plo = lo, phi = hi, qlo = lo, qhi = hi;
-            // scans over the node's m positions only (lanes >= m hold empty boxes): log2(m) steps
-            for (int o = 1; o < m; o <<= 1) {
+            for (int o = 1; o < widest; o <<= 1) {
                 const float3 ulo = f3(__shfl_up_sync(0xffffffffu, plo.x, o), __shfl_up_sync(0xffffffffu, plo.y, o), __shfl_up_sync(0xffffffffu, plo.z, o));
                 const float3 uhi = f3(__shfl_up_sync(0xffffffffu, phi.x, o), __shfl_up_sync(0xffffffffu, phi.y, o), __shfl_up_sync(0xffffffffu, phi.z, o));
                 const float3 dlo = f3(__shfl_down_sync(0xffffffffu, qlo.x, o), __shfl_down_sync(0xffffffffu, qlo.y, o), __shfl_down_sync(0xffffffffu, qlo.z, o));
                 const float3 dhi = f3(__shfl_down_sync(0xffffffffu, qhi.x, o), __shfl_down_sync(0xffffffffu, qhi.y, o), __shfl_down_sync(0xffffffffu, qhi.z, o));
-                if (lane >= o) {
+                if (r >= o) {
                     plo = f3(fminf(plo.x, ulo.x), fminf(plo.y, ulo.y), fminf(plo.z, ulo.z));
                     phi = f3(fmaxf(phi.x, uhi.x), fmaxf(phi.y, uhi.y), fmaxf(phi.z, uhi.z));
                 }
-                if (lane + o < 32) {
+                if (r + o < m) {
                     qlo = f3(fminf(qlo.x, dlo.x), fminf(qlo.y, dlo.y), fminf(qlo.z, dlo.z));
                     qhi = f3(fmaxf(qhi.x, dhi.x), fmaxf(qhi.y, dhi.y), fmaxf(qhi.z, dhi.z));
                 }
@@ -735,70 +855,61 @@ __device__ void warp_build(int* perm, const float4* sc, const float4* slo, const
             // plane after position r: left r + 1 items, right the rest
             const float3 rlo = f3(__shfl_down_sync(0xffffffffu, qlo.x, 1), __shfl_down_sync(0xffffffffu, qlo.y, 1), __shfl_down_sync(0xffffffffu, qlo.z, 1));
             const float3 rhi = f3(__shfl_down_sync(0xffffffffu, qhi.x, 1), __shfl_down_sync(0xffffffffu, qhi.y, 1), __shfl_down_sync(0xffffffffu, qhi.z, 1));
-            const int kl = r + 1;
-            float cost = kInf;
-            if (kl < m && rd + 1 + ceil_log2(max(kl, m - kl)) <= kMaxDepth) {
-                cost = half_area(plo, phi) * static_cast<float>(kl) +
-                       half_area(rlo, rhi) * static_cast<float>(m - kl);
+            float bc = kInf;
+            int bk = r + 1;
+            if (bk < m && rd + 1 + ceil_log2(max(bk, m - bk)) <= kMaxDepth) {
+                bc = half_area(plo, phi) * static_cast<float>(bk) +
+                     half_area(rlo, rhi) * static_cast<float>(m - bk);
             }
-            float bc = cost;
-            int bk = kl;
-            int span = 1;  // lanes holding candidates: below m, rounded up to a power of two
-            while (span < m) span <<= 1;
-            for (int o = span >> 1; o > 0; o >>= 1) {
-                const float oc = __shfl_xor_sync(0xffffffffu, bc, o);
-                const int ok = __shfl_xor_sync(0xffffffffu, bk, o);
-                if (oc < bc || (oc == bc && ok < bk)) {
+            // the segment's cheapest plane meets in its first lane
+            for (int o = 1; o < widest; o <<= 1) {
+                const float oc = __shfl_down_sync(0xffffffffu, bc, o);
+                const int ok = __shfl_down_sync(0xffffffffu, bk, o);
+                if (r + o < m && (oc < bc || (oc == bc && ok < bk))) {
                     bc = oc;
                     bk = ok;
                 }
             }
-            // lanes [0, span) hold the winner; every lane takes it from lane 0
-            bc = __shfl_sync(0xffffffffu, bc, 0);
-            bk = __shfl_sync(0xffffffffu, bk, 0);
+            bc = __shfl_sync(0xffffffffu, bc, sg);
+            bk = __shfl_sync(0xffffffffu, bk, sg);
             if (bc < best) {
                 best = bc;
                 best_axis = a;
                 best_k = bk;
             }
         }
-        const int axis = best_axis < 0 ? 0 : best_axis;
-        const int k = best_k;
-        // items of the left side (bit per item), then a stable partition of every order
-        const int ax_ord = axis == 0 ? ord[0] : (axis == 1 ? ord[1] : ord[2]);
-        const int it = __shfl_sync(0xffffffffu, ax_ord, min(s + r, 31));
-        const unsigned leftmask = __reduce_or_sync(0xffffffffu, (r < k) ? (1u << it) : 0u);
-        const bool inseg = lane >= s && lane < s + m;
-        const unsigned segmask = __ballot_sync(0xffffffffu, inseg);
+        const int k = best_k, kr = m - best_k;
+        // items of the left sides (bit per item), then a stable partition of every order
+        const int it = best_axis == 1 ? ord[1] : (best_axis == 2 ? ord[2] : ord[0]);
+        const unsigned leftmask = __reduce_or_sync(0xffffffffu, (act && r < k) ? (1u << it) : 0u);
+        const unsigned below_me = ((1u << lane) - 1u) & ~((1u << sg) - 1u);
+#pragma unroll
         for (int a = 0; a < 3; ++a) {
             const int item = ord[a];
-            const bool left = inseg && ((leftmask >> item) & 1u);
+            const bool left = act && ((leftmask >> item) & 1u);
             const unsigned lm = __ballot_sync(0xffffffffu, left);
-            const int below = __popc(lm & ((1u << lane) - 1u));
-            const int segbelow = __popc(segmask & ((1u << lane) - 1u));  // = lane - s in the segment
-            const int pos = left ? s + below : s + k + (segbelow - below);
-            if (inseg) scratch[pos] = item;
+            const int below = __popc(lm & below_me);
+            if (act) scratch[left ? sg + below : sg + k + (r - below)] = item;
             __syncwarp();
-            if (inseg) ord[a] = scratch[lane];
+            if (act) ord[a] = scratch[lane];
             __syncwarp();
         }
-        const int kr = m - k;
-        const int lid = k >= 2 ? next_id++ : n - 1 + gbase + b + s;
-        const int rid = kr >= 2 ? next_id++ : n - 1 + gbase + b + s + k;
-        if (lane == 0) link(nodes, bn, parent, rn, lid, rid, n);
-        if (kr >= 2 && top < kWarpRange) {
-            stk_s[top] = s + k;
-            stk_m[top] = kr;
-            stk_n[top] = rid;
-            stk_d[top] = rd + 1;
-            ++top;
-        }
-        if (k >= 2 && top < kWarpRange) {
-            stk_s[top] = s;
-            stk_m[top] = k;
-            stk_n[top] = lid;
-            stk_d[top] = rd + 1;
-            ++top;
+        if (act) {
+            const int leaf = n - 1 + gbase + b + sg;
+            const int lid = k >= 2 ? nx : leaf;
+            const int rid = kr >= 2 ? nx + (k >= 2 ? 1 : 0) : leaf + k;
+            if (r == 0) link(nodes, bn, parent, rn, lid, rid, n);
+            nx += (k >= 2 ? 1 : 0) + (kr >= 2 ? 1 : 0);
+            ++rd;
+            if (r < k) {
+                m = k;
+                rn = lid;
+            } else {
+                nx += max(k - 2, 0);
+                sg += k;
+                m = kr;
+                rn = rid;
+            }
         }
     }
     // leaf order: position p of the axis-0 order
@@ -1266,10 +1377,13 @@ SahWs carve_sah(Carve& c, int n) {
     w.L.chunk_begin = c.take<int>(max_chunks);
     w.L.chunk_first = c.take<int>(max_big);
     w.L.cb = c.take<unsigned>(6 * static_cast<size_t>(max_big));
+    w.L.cb_next = c.take<unsigned>(6 * static_cast<size_t>(max_big));
+    w.L.child_cb = c.take<unsigned>(12 * static_cast<size_t>(max_big));
     w.L.bins = c.take<unsigned>(static_cast<size_t>(max_big) * 3 * kMaxBins * kBinWords);
+    w.L.binned = c.take<int>(max_big);
     w.L.split = c.take<int>(max_big);
     w.L.left_count = c.take<int>(max_big);
-    w.L.chunk_left = c.take<int>(max_chunks);
+    w.L.chunk_pre = c.take<uint16_t>(static_cast<size_t>(max_chunks) * 3 * kMaxBins);
     w.L.counters = c.take<int>(8);
     return w;
 }
@@ -1317,7 +1431,11 @@ int build_sah_impl(qk_tree* t, int bins, int small, const void* items_v, void* w
     const int per_sync = clk ? 1 : kLevelsPerSync;
     const int max_big = n / (kTaskRange + 1) + 1;
     // the first level's chunk list; each level's k_level_assign writes the next one's
-    if (nbig > 0) k_level_prep<<<1, 1024, 0, s>>>(w.L);
+    if (nbig > 0) {
+        k_level_prep<<<1, 1024, 0, s>>>(w.L);
+        k_level_reset<<<1, kBlock, 0, s>>>(w.L, bins);
+        k_level_cbounds<<<n / kChunk + 2, kBlock, 0, s>>>(w.L, ord, w.cen);
+    }
     while (nbig > 0) {
         if (level >= kMaxDepth) return fail(QK_ERR_DEPTH, "SAH: too many levels");
         int bound = nbig;
@@ -1325,24 +1443,24 @@ int build_sah_impl(qk_tree* t, int bins, int small, const void* items_v, void* w
         cudaError_t e;
         for (int j = 0; j < batch; ++j, ++level) {
             w.L.tasks = cur;
-            k_level_reset<<<bound, kBlock, 0, s>>>(w.L, bins);
             // chunk kernels: grid sized by a bound on the chunk count (every task spans at most
-            // size / kChunk + 1 chunks); blocks beyond the count k_level_prep wrote return at once
+            // size / kChunk + 1 chunks); blocks beyond the count return at once.  Three launches
+            // a level, each scheduled while the one before drains.
             const int nch = n / kChunk + bound + 1;
-            // per-level stage times when a StageClock is installed: binning (centroid bounds +
-            // bins), split selection, partition (+ child assignment)
+            // per-level stage times when a StageClock is installed: binning with the split
+            // selection, partition (+ child assignment)
             if (clk) cudaEventRecord(clk->lv[0], s);
-            k_level_cbounds<<<nch, kBlock, 0, s>>>(w.L, ord, w.cen);
-            k_level_bins<<<nch, kBlock, 0, s>>>(w.L, ord, w.cen, w.plo, w.phi, bins);
-            if (clk) cudaEventRecord(clk->lv[1], s);
-            k_level_split<<<blocks_for(static_cast<long long>(bound) * 32), kBlock, 0, s>>>(w.L, bins);
-            if (clk) cudaEventRecord(clk->lv[2], s);
-            k_level_count_left<<<nch, kBlock, 0, s>>>(w.L, ord, w.cen, bins);
-            k_level_partition<<<nch, kBlock, 0, s>>>(w.L, ord, alt, w.orderF, w.cen, bins);
-            // next big tasks start from zero each level; block tasks accumulate
-            cudaMemsetAsync(w.L.counters + 1, 0, sizeof(int), s);
-            k_level_assign<<<1, 1024, 0, s>>>(w.L, nxt, w.blocks, nodes, bn, t->parent, n);
+            launch_pdl(k_level_bins, dim3(nch), dim3(kBlock), s, w.L, ord, w.cen, w.plo, w.phi, bins);
+            if (clk) {
+                cudaEventRecord(clk->lv[1], s);
+                cudaEventRecord(clk->lv[2], s);
+            }
+            launch_pdl(k_level_partition, dim3(nch), dim3(kBlock), s, w.L, ord, alt, w.orderF, w.cen,
+                       bins, max_big);
+            launch_pdl(k_level_assign, dim3(1), dim3(1024), s, w.L, nxt, w.blocks, nodes, bn,
+                       t->parent, n);
             if (clk) cudaEventRecord(clk->lv[3], s);
+            std::swap(w.L.cb, w.L.cb_next);
             Task* tmpt = cur;
             cur = nxt;
             nxt = tmpt;

@@ -118,3 +118,27 @@ def test_ellipsoid_tests_end_early_with_the_same_bits(cuda, smin, smax):
         woff, wkeys = ref.radius(q, 9.0)
         assert np.array_equal(off.cpu().numpy().astype(np.int64), woff), f
         assert np.array_equal(keys.cpu().numpy().view(np.uint64), wkeys), f
+
+
+@pytest.mark.parametrize("builder", ["sah", "sah4"])
+@pytest.mark.parametrize("n", [2, 3, 5, 31, 32, 33, 64, 255, 256, 257, 600, 2048, 2049, 4500, 30011])
+@pytest.mark.parametrize("distinct", [1, 9, 1 << 30])
+def test_sah_range_edges(cuda, builder, n, distinct):
+    """Ranges at the edges of the warp and global tiers, with and without planes that separate the
+    centroids: a sound tree, the same one each time, with the oracle's query results."""
+    pts = _points(n, n + 1, distinct)
+    t = capi.DeviceTree("point", pts, builder=builder)
+    assert t.validate() == [0] * 8
+    first = t.nodes_bytes().tobytes()
+    t.build()
+    assert t.nodes_bytes().tobytes() == first
+    q = workloads.uniform_points(200, [-5.0] * 3, [105.0] * 3, n, 13)
+    ref = oracle.LBVH("point", pts)
+    assert np.array_equal(t.knn(_dev(q), 5).cpu().numpy().view(np.uint32), ref.knn(q, 5))
+
+
+@pytest.mark.parametrize("bins", [4, 17, 32, 33, 64])
+def test_sah_bin_counts(cuda, bins):
+    tris, _ = workloads.city(700, 11)
+    t = capi.DeviceTree("tri", tris, builder="sah", sah_bins=bins)
+    assert t.validate() == [0] * 8
