@@ -233,16 +233,22 @@ __global__ __launch_bounds__(kBlock) void k_refit_leaves(const float* __restrict
     for (int j = 0; j < Ops::kVec4; ++j) leaves[static_cast<size_t>(k) * Ops::kVec4 + j] = pay[j];
 }
 
+// A dirty refit is two climbs of about log n levels by a few thousand threads, so it is bound by
+// the latency of one level: 64 threads per block spread them over the SMs, and both climbs load
+// what the next level needs (static during the pass) while this level's atomic waits.  1 % of a
+// 1 M-point cloud: 53.7 -> 49.7 us.
+constexpr int kDirtyBlock = 64;
+
 // Dirty refit, pass 1: write the moved leaves and mark ancestors.  flags[p] bit 0 / bit 1
 // record a dirty left / right child; a thread stops climbing at the first node another
 // thread already marked.  A repeated id (same leaf twice) is dropped via skip[].
 template <class Ops>
-__global__ __launch_bounds__(kBlock) void k_dirty_mark(
+__global__ __launch_bounds__(kDirtyBlock) void k_dirty_mark(
     const int* __restrict__ ids, const float* __restrict__ items, int count, int n,
     const int* __restrict__ slot_of, const int* __restrict__ parent, Node* __restrict__ nodes,
     float* __restrict__ sorted, float4* __restrict__ leaves, int* __restrict__ flags,
     int* __restrict__ skip, Header* __restrict__ h) {
-    const int i = blockIdx.x * kBlock + threadIdx.x;
+    const int i = blockIdx.x * kDirtyBlock + threadIdx.x;
     if (i >= count) return;
     const int id = ids[i];
     if (id < 0 || id >= n) {
@@ -251,10 +257,11 @@ __global__ __launch_bounds__(kBlock) void k_dirty_mark(
         return;
     }
     const int slot = slot_of[id];
-    int node = n - 1 + slot;
+    const int node = n - 1 + slot;
     int p = parent[node];
     // claim the leaf: the first thread to set the child bit of its parent owns it
     const int bit0 = nodes[p].left == node ? 1 : 2;
+    int pn = parent[p];
     const int old0 = atomicOr(&flags[p], bit0);
     if (old0 & bit0) {
         skip[i] = 1;
@@ -272,36 +279,43 @@ __global__ __launch_bounds__(kBlock) void k_dirty_mark(
 #pragma unroll
     for (int j = 0; j < Ops::kVec4; ++j) leaves[static_cast<size_t>(slot) * Ops::kVec4 + j] = pay[j];
     if (old0 != 0) return;  // parent already marked by the sibling
-    int guard = 0;
-    while (guard++ < 4096) {
-        node = p;
-        p = parent[node];
-        if (p < 0) return;
-        const int bit = nodes[p].left == node ? 1 : 2;
-        if (atomicOr(&flags[p], bit) != 0) return;
+    int left = pn >= 0 ? nodes[pn].left : 0;
+    for (int guard = 0; guard < 4096 && pn >= 0; ++guard) {
+        const int pnn = parent[pn];
+        const int old = atomicOr(&flags[pn], left == p ? 1 : 2);
+        const int left_n = pnn >= 0 ? nodes[pnn].left : 0;
+        if (old != 0) return;
+        p = pn;
+        pn = pnn;
+        left = left_n;
     }
 }
 
 // Dirty refit, pass 2: climb again; arrivals are counted in flags[p] >> 2 and the last of
-// the popcount(flags[p] & 3) dirty children finishes p, clears the word and continues.
-__global__ __launch_bounds__(kBlock) void k_dirty_merge(const int* __restrict__ ids, int count,
-                                                       int n, const int* __restrict__ slot_of,
-                                                       const int* __restrict__ parent,
-                                                       Node* __restrict__ nodes,
-                                                       BNode* __restrict__ bnodes,
-                                                       int* __restrict__ flags,
-                                                       const int* __restrict__ skip) {
-    const int i = blockIdx.x * kBlock + threadIdx.x;
+// the popcount(flags[p] & 3) dirty children finishes p, clears the word and continues.  A
+// thread carries its child's box; the sibling's is loaded with the arrival, and again after it
+// only where the sibling is dirty too (its box was then written by the thread that stopped).
+__global__ __launch_bounds__(kDirtyBlock) void k_dirty_merge(const int* __restrict__ ids, int count,
+                                                            int n, const int* __restrict__ slot_of,
+                                                            const int* __restrict__ parent,
+                                                            Node* __restrict__ nodes,
+                                                            BNode* __restrict__ bnodes,
+                                                            int* __restrict__ flags,
+                                                            const int* __restrict__ skip) {
+    const int i = blockIdx.x * kDirtyBlock + threadIdx.x;
     if (i >= count || skip[i]) return;
     auto links = [&](int v) { return *reinterpret_cast<const int2*>(&nodes[v].left); };
-    int p = parent[n - 1 + slot_of[ids[i]]];
+    int c = n - 1 + slot_of[ids[i]];
+    int p = parent[c];
     if (p < 0) return;
     int2 lr = links(p);
     int pn = parent[p];
-    const int2 none = make_int2(0, 0);
+    Box box = load_box_cg(nodes + c);
     for (int guard = 0; guard < 4096; ++guard) {
-        // the next level's parent and links (static) load while this arrival and box wait
-        int2 lrn = none;
+        const bool left = lr.x == c;
+        const int sib = left ? lr.y : lr.x;
+        Box sb = load_box_cg(nodes + sib);
+        int2 lrn = make_int2(0, 0);
         int pnn = -1;
         if (pn >= 0) {
             lrn = links(pn);
@@ -310,9 +324,12 @@ __global__ __launch_bounds__(kBlock) void k_dirty_merge(const int* __restrict__ 
         const int old = arrive_add(&flags[p], 4);
         const int need = __popc(old & 3);
         if ((old >> 2) + 1 < need) return;
-        finish_node_links<false, false>(nodes, bnodes, p, n, lr, none, none);
+        if (need == 2) sb = load_box_cg(nodes + sib);
+        const Box a = left ? box : sb, b = left ? sb : box;
+        box = write_node_boxes(nodes, bnodes, p, lr, a, b);
         flags[p] = 0;
         if (pn < 0) return;
+        c = p;
         p = pn;
         lr = lrn;
         pn = pnn;
@@ -605,12 +622,12 @@ int refit_dirty_impl(qk_tree* t, const int* ids, const void* items, int count, v
     int* skip = c.take<int>(count);
     stage_mark(kMarkStart, s);
     k_header_init<<<1, 32, 0, s>>>(h);
-    k_dirty_mark<Ops><<<blocks_for(count), kBlock, 0, s>>>(
+    k_dirty_mark<Ops><<<blocks_for(count, kDirtyBlock), kDirtyBlock, 0, s>>>(
         ids, static_cast<const float*>(items), count, n, t->slot_of, t->parent,
         static_cast<Node*>(t->nodes), static_cast<float*>(t->items),
         static_cast<float4*>(t->leaves), t->flags, skip, h);
     stage_mark(kMarkScatter, s);
-    k_dirty_merge<<<blocks_for(count), kBlock, 0, s>>>(ids, count, n, t->slot_of, t->parent,
+    k_dirty_merge<<<blocks_for(count, kDirtyBlock), kDirtyBlock, 0, s>>>(ids, count, n, t->slot_of, t->parent,
                                                        static_cast<Node*>(t->nodes),
                                                        static_cast<BNode*>(t->bnodes), t->flags,
                                                        skip);

@@ -149,6 +149,23 @@ __device__ __forceinline__ Box load_box_ca(const Node* nd) {
     return bx;
 }
 
+// Internal node p with links lr from its children's boxes: the union (returned), the canonical
+// node and the boxes of the traversal node.
+__device__ __forceinline__ Box write_node_boxes(Node* __restrict__ nodes, BNode* __restrict__ bnodes,
+                                                int p, int2 lr, const Box& a, const Box& b) {
+    Box u;
+    u.lo = f3(fmin_t(a.lo.x, b.lo.x), fmin_t(a.lo.y, b.lo.y), fmin_t(a.lo.z, b.lo.z));
+    u.hi = f3(fmax_t(a.hi.x, b.hi.x), fmax_t(a.hi.y, b.hi.y), fmax_t(a.hi.z, b.hi.z));
+    float4* np = reinterpret_cast<float4*>(nodes + p);
+    np[0] = make_float4(u.lo.x, u.lo.y, u.lo.z, u.hi.x);
+    np[1] = make_float4(u.hi.y, u.hi.z, __int_as_float(lr.x), __int_as_float(lr.y));
+    BNode& bn = bnodes[p];
+    bn.v0 = make_float4(a.lo.x, a.lo.y, a.lo.z, a.hi.x);
+    bn.v1 = make_float4(a.hi.y, a.hi.z, b.lo.x, b.lo.y);
+    bn.v2 = make_float4(b.lo.z, b.hi.x, b.hi.y, b.hi.z);
+    return u;
+}
+
 // Complete internal node p from its final children given its links lr = (left, right) and the
 // children's slot ranges (all static during the pass): box and traversal node, with the
 // children's small-subtree codes.  kLocal: both children were finished by threads of this
@@ -164,16 +181,7 @@ __device__ __forceinline__ void finish_node_links(Node* __restrict__ nodes,
             __int_as_float(small_code(l, n, rl)), __int_as_float(small_code(r, n, rr)));
     const Box a = kLocal ? load_box_ca(nodes + l) : load_box_cg(nodes + l);
     const Box b = kLocal ? load_box_ca(nodes + r) : load_box_cg(nodes + r);
-    Box u;
-    u.lo = f3(fmin_t(a.lo.x, b.lo.x), fmin_t(a.lo.y, b.lo.y), fmin_t(a.lo.z, b.lo.z));
-    u.hi = f3(fmax_t(a.hi.x, b.hi.x), fmax_t(a.hi.y, b.hi.y), fmax_t(a.hi.z, b.hi.z));
-    float4* np = reinterpret_cast<float4*>(nodes + p);
-    np[0] = make_float4(u.lo.x, u.lo.y, u.lo.z, u.hi.x);
-    np[1] = make_float4(u.hi.y, u.hi.z, __int_as_float(l), __int_as_float(r));
-    BNode& bn = bnodes[p];
-    bn.v0 = make_float4(a.lo.x, a.lo.y, a.lo.z, a.hi.x);
-    bn.v1 = make_float4(a.hi.y, a.hi.z, b.lo.x, b.lo.y);
-    bn.v2 = make_float4(b.lo.z, b.hi.x, b.hi.y, b.hi.z);
+    write_node_boxes(nodes, bnodes, p, lr, a, b);
 }
 
 // Refit: one leaf's climb toward the root of a tree whose topology is unchanged; flags[p]
