@@ -13,6 +13,8 @@
 // Morton ordering (RayOrder::Morton / QueryOrder::Morton) does not gather and scatter copies
 // of the inputs: the sorted permutation is handed to the traversal, thread i works on item
 // order[i] and writes its result in place.
+#include <algorithm>
+
 #include "qk_internal.cuh"
 #include "qk_traverse.cuh"
 
@@ -550,6 +552,9 @@ __global__ __launch_bounds__(kBlock) void k_ray_wide(const WideNode* __restrict_
 // queries in blocks of 256 would occupy only some of the 148 SMs, and these latency-bound
 // traversals run faster spread over all of them; large batches keep 256.
 inline int query_block(int count) { return count <= 148 * 512 ? 64 : kBlock; }
+// Rays: a few thousand diverge from the first node, and one warp per SM then leaves the L1 to
+// itself.
+inline int ray_block(int count) { return count <= 148 * 64 ? 32 : query_block(count); }
 // the same for the lane-group kernels, counted in threads
 inline int split_block(int count, int lanes) {
     return static_cast<long long>(count) * lanes <= 148 * 2048 ? 64 : kBlock;
@@ -953,6 +958,86 @@ __global__ __launch_bounds__(kBlock) void k_radius_split(
     flush_stats<kStats>(valid, valid ? tv.nodes : 0, valid ? tv.leaves : 0, valid && tv.overflow, stats);
 }
 
+// The single-pass radius with kPoolLanes lanes per query (few queries): every lane keeps the keys
+// of its subtree in a stash and chain of its own, entry q * kPoolLanes + lane of the pool.  Counts
+// of the lanes go to lane_counts, their sum to counts.
+constexpr int kPoolLanes = 4;
+template <class Ops, bool kStats>
+__global__ __launch_bounds__(kBlock) void k_radius_count_pool_split(
+    const BNode* __restrict__ bn, const float4* __restrict__ leaves, const float* __restrict__ pts,
+    const uint32_t* __restrict__ order, int count, float r2, int* __restrict__ counts,
+    int* __restrict__ lane_counts, RadiusPool pool, int max_iter,
+    unsigned long long* __restrict__ stats) {
+    constexpr int G = kPoolLanes;
+    if (static_cast<long long>(blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) / G >= count)
+        return;  // whole warps past the last query
+    bool valid;
+    int lane;
+    const int q = split_query<G>(count, order, valid, lane);
+    const float3 p = f3(pts[3 * q], pts[3 * q + 1], pts[3 * q + 2]);
+    const size_t v = static_cast<size_t>(q) * G + lane;
+    if (valid) pool.first[v] = -1;
+    PoolSink sink{pool.stash + v * kRadiusStash, pool.keys, pool.next, pool.taken, pool.chunks,
+                  pool.first + v, 0, -1};
+    Trav tv;
+    const int found = radius_split_visit<Ops, G>(bn, leaves, p, r2, lane, sink, max_iter, tv, valid);
+    const int total = group_sum<G>(found);
+    if (valid) {
+        lane_counts[v] = found;
+        if (lane == 0) counts[q] = total;
+    }
+    flush_stats<kStats>(valid, valid ? tv.nodes : 0, valid ? tv.leaves : 0, valid && tv.overflow, stats);
+}
+
+// whether the pool dropped some lane's keys of query q
+__device__ __forceinline__ bool pool_lost(const RadiusPool& pool, const int* __restrict__ lane_counts,
+                                          int q) {
+    bool lost = false;
+#pragma unroll
+    for (int l = 0; l < kPoolLanes; ++l) {
+        const size_t v = static_cast<size_t>(q) * kPoolLanes + l;
+        lost = lost || (lane_counts[v] > kRadiusStash && pool.first[v] == kPoolLost);
+    }
+    return lost;
+}
+
+// its copy pass: one warp per query moves the lanes' stashes and chains, lane after lane
+__global__ __launch_bounds__(kBlock) void k_radius_gather_split(
+    int count, const int* __restrict__ offsets, const int* __restrict__ lane_counts, RadiusPool pool,
+    unsigned long long* __restrict__ keys) {
+    const int q = static_cast<int>((static_cast<long long>(blockIdx.x) * kBlock + threadIdx.x) >> 5);
+    const int lane = threadIdx.x & 31;
+    if (q >= count || pool_lost(pool, lane_counts, q)) return;
+    int begin = offsets[q];
+#pragma unroll
+    for (int l = 0; l < kPoolLanes; ++l) {
+        const int v = q * kPoolLanes + l;
+        const int m = lane_counts[v];
+        copy_pooled_warp(pool, v, begin, m, keys, lane);
+        begin += m;
+    }
+}
+
+// its second traversal: queries that lost keys, each lane writing its own part again
+template <class Ops>
+__global__ __launch_bounds__(kBlock) void k_radius_fill_lost_split(
+    const BNode* __restrict__ bn, const float4* __restrict__ leaves, const float* __restrict__ pts,
+    int count, float r2, const int* __restrict__ offsets, const int* __restrict__ lane_counts,
+    RadiusPool pool, unsigned long long* __restrict__ keys, int max_iter) {
+    constexpr int G = kPoolLanes;
+    bool valid;
+    int lane;
+    const int q = split_query<G>(count, nullptr, valid, lane);
+    const bool lost = valid && pool_lost(pool, lane_counts, q);
+    if (!__any_sync(0xffffffffu, lost)) return;
+    const float3 p = f3(pts[3 * q], pts[3 * q + 1], pts[3 * q + 2]);
+    const int mine = lost ? lane_counts[static_cast<size_t>(q) * G + lane] : 0;
+    const int write = offsets[q] + warp_exclusive<G>(mine, lane);
+    const int end = lost ? min(write + mine, offsets[q + 1]) : write;
+    Trav tv;
+    radius_split_one<Ops, true, G>(bn, leaves, p, r2, lane, write, end, keys, max_iter, tv, lost);
+}
+
 // ---- segment sort of the radius keys ----
 constexpr int kWarpSortMax = 1024;   // largest segment sorted by one warp
 constexpr int kWarpSortBlock = 128;  // threads per block of the warp sort
@@ -1244,6 +1329,20 @@ inline int split_lanes(unsigned flags) {
     return (flags & QK_TUNE_SPLIT) ? 32 : (flags & QK_TUNE_SPLIT8) ? 8 : (flags & QK_TUNE_SPLIT4) ? 4 : 0;
 }
 
+// Few queries, no schedule asked for, binary nodes: groups of 4 lanes instead of one thread per
+// query (8 for 5 to 8 neighbours, to half as many queries: at 20,000 they win by 12 % on a terrain
+// and lose by 16 % on uniform points), whose latency otherwise leaves most of the GPU idle.  One thread -> groups, us, 8,000 and 32,000 queries: terrain of 131,072 triangles
+// closest 316 -> 182, 349 -> 244, kNN4 413 -> 218, 473 -> 307; 1 M uniform points closest 61 -> 51,
+// 95 -> 95, kNN4 113 -> 80, 152 -> 138, radius (48 found) 384 -> 304, 524 -> 446; 200,000
+// ellipsoids closest 295 -> 143, 321 -> 205.  The gain ends near 32,768 queries on the cheapest
+// tests (points, closest).  Calls that count nodes keep one thread per query (statistics), except
+// radius, whose two passes must agree.
+constexpr int kFewQueries = 32768;
+constexpr unsigned kScheduleFlags = kSplitFlags | QK_WIDE | QK_TUNE_LEAF4 | QK_TUNE_STASH | QK_TUNE_TAIL;
+inline unsigned few_flags(unsigned flags, int count) {
+    return (flags & kScheduleFlags) == 0 && count <= kFewQueries ? flags | QK_TUNE_SPLIT4 : flags;
+}
+
 template <class Ops, bool kStats>
 void launch_closest_split(int lanes, const BNode* bn, const float4* leaves, const float* pts,
                           const uint32_t* order, int count, uint2* out, int max_iter,
@@ -1288,6 +1387,7 @@ int closest_impl(const qk_tree* t, const float* pts, int count, uint2* out, unsi
     const int g = blocks_for(count, qb);
     const bool wide = (flags & QK_WIDE) != 0;
     const bool st = stats != nullptr;
+    if (!st) flags = few_flags(flags, count);
     if (tail.count) {
         // budgeted traversal (binary nodes, thread or warp per query), then the shared scan
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
@@ -1383,6 +1483,7 @@ int knn_impl(const qk_tree* t, const float* pts, int count, int k, int stride, u
              unsigned flags, unsigned long long* stats, const uint32_t* order, cudaStream_t s,
              const TailList& tail = TailList{}) {
     const bool wide = (flags & QK_WIDE) != 0;
+    if (!stats && k <= 8) flags = few_flags(flags, count * (k <= 4 ? 1 : 2));
     const int split = split_lanes(flags);  // 0: one thread per query
     const bool leaf4 = (flags & QK_TUNE_LEAF4) != 0;
     if (tail.count) {
@@ -1499,7 +1600,7 @@ int ray_query(const qk_tree* t, const void* rays, int count, uint64_t* out, int*
     auto* res = reinterpret_cast<unsigned long long*>(out);
     auto* stt = reinterpret_cast<unsigned long long*>(stats);
     const float4* leaves = static_cast<const float4*>(t->leaves);
-    const int rb = query_block(count);
+    const int rb = ray_block(count);
     const int g = blocks_for(count, rb);
     const int g256 = blocks_for(count);  // the short stack's shared arrays are sized for 256 threads
     if (flags & QK_WIDE) {
@@ -1620,7 +1721,28 @@ bool use_stash(unsigned flags) {
     return (flags & QK_TUNE_STASH) && !(flags & (kSplitFlags | QK_WIDE));
 }
 
-size_t radius_ws_bytes(int count, unsigned flags) {
+// lanes per query of the single-pass radius: groups for few queries (one thread -> groups, 8,000 and
+// 32,000 queries on 1 M uniform points, 48 found: 271 -> 223 us, 403 -> 343)
+inline int pool_lanes(unsigned flags, int count) {
+    return !(flags & QK_TUNE_LEAF4) && count <= kFewQueries ? kPoolLanes : 1;
+}
+
+// the pool of the single-pass radius and, with lane groups, the lanes' counts: a stash and a chain
+// per lane, the same number of chunks
+struct PoolBufs {
+    RadiusPool pool{};
+    int* lane_counts = nullptr;
+};
+PoolBufs carve_pool_lanes(Carve& c, int count, unsigned flags) {
+    PoolBufs b;
+    const int lanes = pool_lanes(flags, count);
+    b.pool = carve_pool(c, count * lanes, kPoolPerQuery / lanes);
+    if (lanes > 1) b.lane_counts = c.take<int>(static_cast<size_t>(count) * lanes);
+    return b;
+}
+
+static size_t radius_need(int count, unsigned flags) {
+    flags = few_flags(flags, count);
     Carve c;
     carve_order(c, count);
     c.take<int>(count);            // counts
@@ -1628,15 +1750,21 @@ size_t radius_ws_bytes(int count, unsigned flags) {
     c.take<int>(count);            // medium segment list
     c.take<int>(count);            // large segment list
     if (flags & kSplitFlags) c.take<int>(static_cast<size_t>(count) * 32);  // lane counts
-    if (use_stash(flags)) carve_pool(c, count);
+    if (use_stash(flags)) carve_pool_lanes(c, count, flags);
     return c.used;
+}
+
+// never less than a smaller batch needs, so a workspace sized for the largest serves them all
+size_t radius_ws_bytes(int count, unsigned flags) {
+    return std::max(radius_need(count, flags), radius_need(std::min(count, kFewQueries), flags));
 }
 
 template <class Ops>
 int radius_pool_launch(const qk_tree* t, const float* pts, int count, float r2, int* counts,
-                       const int* offsets, const RadiusPool& pool, unsigned long long* keys,
+                       const int* offsets, const PoolBufs& bufs, unsigned long long* keys,
                        unsigned flags, unsigned long long* stats, const uint32_t* order,
                        bool fill, cudaStream_t s) {
+    const RadiusPool& pool = bufs.pool;
     const BNode* bn = static_cast<const BNode*>(t->bnodes);
     const Node* nodes = static_cast<const Node*>(t->nodes);
     const float4* leaves = static_cast<const float4*>(t->leaves);
@@ -1644,7 +1772,20 @@ int radius_pool_launch(const qk_tree* t, const float* pts, int count, float r2, 
     const int g = blocks_for(count, qb);
     const int it = t->n * 2 + 64;
     const bool leaf4 = (flags & QK_TUNE_LEAF4) != 0;
-    if (fill) {
+    if (bufs.lane_counts) {
+        if (fill) {
+            k_radius_gather_split<<<blocks_for(static_cast<long long>(count) * 32), kBlock, 0, s>>>(
+                count, offsets, bufs.lane_counts, pool, keys);
+            k_radius_fill_lost_split<Ops><<<blocks_for(static_cast<long long>(count) * kPoolLanes), kBlock, 0, s>>>(
+                bn, leaves, pts, count, r2, offsets, bufs.lane_counts, pool, keys, it);
+        } else {
+            cudaMemsetAsync(pool.taken, 0, sizeof(int), s);
+            const int sb = split_block(count, kPoolLanes);
+            const int gs = blocks_for(static_cast<long long>(count) * kPoolLanes, sb);
+            if (stats) k_radius_count_pool_split<Ops, true><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, bufs.lane_counts, pool, it, stats);
+            else k_radius_count_pool_split<Ops, false><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, bufs.lane_counts, pool, it, stats);
+        }
+    } else if (fill) {
         k_radius_gather<<<blocks_for(static_cast<long long>(count) * 32), kBlock, 0, s>>>(
             pool, offsets, count, keys, -1);
         if (leaf4) k_radius_fill_lost<Ops, true><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, count, r2, offsets, pool, keys, it, leaf_nodes(t));
@@ -1664,7 +1805,7 @@ int radius_pool_launch(const qk_tree* t, const float* pts, int count, float r2, 
 }
 
 int radius_pool_dispatch(const qk_tree* t, const float* pts, int count, float r2, int* counts,
-                         const int* offsets, const RadiusPool& pool, unsigned long long* keys,
+                         const int* offsets, const PoolBufs& pool, unsigned long long* keys,
                          unsigned flags, unsigned long long* stats, const uint32_t* order,
                          bool fill, cudaStream_t s) {
     switch (t->kind) {
@@ -1682,6 +1823,7 @@ int radius_count(const qk_tree* t, const float* pts, int count, float r, int* of
         cudaMemsetAsync(offsets, 0, sizeof(int), s);
         return QK_OK;
     }
+    flags = few_flags(flags, count);
     Carve c{static_cast<char*>(ws)};
     OrderBufs o = carve_order(c, count);
     int* counts = c.take<int>(count);
@@ -1690,7 +1832,7 @@ int radius_count(const qk_tree* t, const float* pts, int count, float r, int* of
     c.take<int>(count);
     int* lane_counts = (flags & kSplitFlags) ? c.take<int>(static_cast<size_t>(count) * 32) : nullptr;
     const bool pooled = use_stash(flags);
-    const RadiusPool pool = pooled ? carve_pool(c, count) : RadiusPool{};
+    const PoolBufs pool = pooled ? carve_pool_lanes(c, count, flags) : PoolBufs{};
     int st = QK_OK;
     const uint32_t* order = make_order(pts, 3, 0, count, flags, o, s, &st);
     if (st != QK_OK) return st;
@@ -1714,6 +1856,7 @@ int radius_count(const qk_tree* t, const float* pts, int count, float r, int* of
 int radius_fill(const qk_tree* t, const float* pts, int count, float r, const int* offsets,
                 uint64_t* keys, unsigned flags, void* ws, cudaStream_t s) {
     if (count <= 0) return QK_OK;
+    flags = few_flags(flags, count);
     Carve c{static_cast<char*>(ws)};
     OrderBufs o = carve_order(c, count);
     c.take<int>(count);
@@ -1722,7 +1865,7 @@ int radius_fill(const qk_tree* t, const float* pts, int count, float r, const in
     int* large = c.take<int>(count);
     int* lane_counts = (flags & kSplitFlags) ? c.take<int>(static_cast<size_t>(count) * 32) : nullptr;
     const bool pooled = use_stash(flags);
-    const RadiusPool pool = pooled ? carve_pool(c, count) : RadiusPool{};
+    const PoolBufs pool = pooled ? carve_pool_lanes(c, count, flags) : PoolBufs{};
     auto* k64 = reinterpret_cast<unsigned long long*>(keys);
     int st = QK_OK;
     if (pooled) {

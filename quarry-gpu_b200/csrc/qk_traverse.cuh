@@ -1482,14 +1482,12 @@ __device__ __forceinline__ uint2 warp_table_entry(const WarpTable& tab) {
                                 : make_uint2(0u, 0xffffffffu);
 }
 
-// radius, split: returns this lane's count; the fill pass writes the lane's keys from
-// `write` on, never past `end` (the query's offset plus the counts of the lower lanes)
-template <class Ops, bool kFill, int G = 32>
-__device__ __forceinline__ int radius_split_one(const BNode* __restrict__ bn,
-                                                const float4* __restrict__ leaves, float3 p,
-                                                float r2, int lane, int write, int end,
-                                                unsigned long long* __restrict__ keys,
-                                                int max_iter, Trav& tv, bool valid = true) {
+// radius, split: hands this lane's keys to `sink` and returns their count
+template <class Ops, int G, class Sink>
+__device__ __forceinline__ int radius_split_visit(const BNode* __restrict__ bn,
+                                                  const float4* __restrict__ leaves, float3 p,
+                                                  float r2, int lane, Sink& sink, int max_iter,
+                                                  Trav& tv, bool valid) {
     int found = 0;
     auto keep = [&](float3 lo, float3 hi) { return dist2_box(p, lo, hi) <= r2; };
     auto on_leaf = [&](int slot) {
@@ -1497,7 +1495,7 @@ __device__ __forceinline__ int radius_split_one(const BNode* __restrict__ bn,
         int id;
         const float d2 = Ops::dist2(p, leaves, slot, id, r2);
         if (d2 <= r2) {
-            if (kFill && write < end) keys[write++] = radius_key(d2, id);
+            sink.put(radius_key(d2, id));
             ++found;
         }
     };
@@ -1547,6 +1545,18 @@ __device__ __forceinline__ int radius_split_one(const BNode* __restrict__ bn,
         }
     }
     return found;
+}
+
+// the same as two passes: the count pass drops the keys, the fill pass writes them from `write` on,
+// never past `end` (the query's offset plus the counts of the lower lanes)
+template <class Ops, bool kFill, int G = 32>
+__device__ __forceinline__ int radius_split_one(const BNode* __restrict__ bn,
+                                                const float4* __restrict__ leaves, float3 p,
+                                                float r2, int lane, int write, int end,
+                                                unsigned long long* __restrict__ keys,
+                                                int max_iter, Trav& tv, bool valid = true) {
+    SegmentSink sink{keys, write, kFill ? end : write};
+    return radius_split_visit<Ops, G>(bn, leaves, p, r2, lane, sink, max_iter, tv, valid);
 }
 
 // exclusive prefix over the lanes of `v` (of the group of G lanes; `lane` the lane in it)

@@ -142,3 +142,43 @@ def test_sah_bin_counts(cuda, bins):
     tris, _ = workloads.city(700, 11)
     t = capi.DeviceTree("tri", tris, builder="sah", sah_bins=bins)
     assert t.validate() == [0] * 8
+
+
+@pytest.mark.parametrize("kind", ["tri", "point", "gauss"])
+@pytest.mark.parametrize("count", [1, 2, 31, 65, 1000])
+def test_few_queries_take_lane_groups(cuda, kind, count):
+    """Batches small enough for lane groups, next to schedules that keep one thread per query."""
+    items = {"tri": lambda: workloads.terrain(20, 2), "point": lambda: _points(900, 5, 400),
+             "gauss": lambda: workloads.gaussians(500, 0.5, 10.0, 4)}[kind]()
+    c = items.reshape(len(items), -1)[:, :3]
+    q = workloads.uniform_points(count, c.min(0) - 5, c.max(0) + 5, 9, 13)
+    t, ref = capi.DeviceTree(kind, items), oracle.LBVH(kind, items)
+    r = 0.2 * float(np.linalg.norm(c.max(0) - c.min(0)))  # stashes and chains of every lane
+    woff, wkeys = ref.radius(q, r)
+    for f in (0, capi.QK_ORDER_MORTON, capi.QK_TUNE_LEAF4):
+        assert np.array_equal(t.closest(_dev(q), f).cpu().numpy().view(np.uint32), ref.closest(q)), f
+        for k in (3, 8):
+            assert np.array_equal(t.knn(_dev(q), k, f).cpu().numpy().view(np.uint32), ref.knn(q, k)), f
+        for g in (f, f | capi.QK_TUNE_STASH):
+            off, keys = t.radius(_dev(q), r, g)
+            assert np.array_equal(off.cpu().numpy().astype(np.int64), woff), g
+            assert np.array_equal(keys.cpu().numpy().view(np.uint64), wkeys), g
+
+
+def test_radius_pool_runs_out_with_lane_groups(cuda):
+    """Queries that find nearly every point: the pool holds 128 keys per query, so most are lost and
+    traversed again."""
+    pts = _points(3000, 6, 1 << 30)
+    q = workloads.uniform_points(40, [0.0] * 3, [100.0] * 3, 6, 13)
+    t, ref = capi.DeviceTree("point", pts), oracle.LBVH("point", pts)
+    off, keys = t.radius(_dev(q), 90.0, capi.QK_TUNE_STASH)
+    woff, wkeys = ref.radius(q, 90.0)
+    assert np.array_equal(off.cpu().numpy().astype(np.int64), woff)
+    assert np.array_equal(keys.cpu().numpy().view(np.uint64), wkeys)
+
+
+def test_radius_workspace_of_a_large_batch_serves_small_ones(cuda):
+    L = capi.lib()
+    for flags in (0, capi.QK_TUNE_STASH, capi.QK_TUNE_SPLIT4, capi.QK_WIDE):
+        sizes = [L.qk_radius_workspace_bytes(n, flags) for n in (1, 500, 32768, 32769, 40000, 200000)]
+        assert sizes == sorted(sizes)
