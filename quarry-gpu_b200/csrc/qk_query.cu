@@ -347,19 +347,29 @@ __global__ __launch_bounds__(kBlock) void k_coh_scatter(const uint32_t* __restri
 // ---------------------------------------------------------------------------------------
 // single-tree kernels: one thread per ray / query point, bodies in qk_traverse.cuh
 // ---------------------------------------------------------------------------------------
+// Ray of this thread when every 2^spread-th lane holds one.  A small batch in full warps occupies
+// few SMs, and a warp takes as many steps as its longest ray, each step's loads serving 32 nodes
+// one after the other; the same rays in a quarter of the lanes of four times the warps wait less.
+__device__ __forceinline__ bool ray_of_thread(int count, int spread, int& i) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    i = t >> spread;
+    return i < count && (t & ((1 << spread) - 1)) == 0;
+}
+
 template <bool kStats, int kMinBlocks, int kShort = 0, bool kLeaf4 = false>
 __global__ __launch_bounds__(kBlock, kMinBlocks) void k_ray_bin(const BNode* __restrict__ bn,
                                                    const float4* __restrict__ leaves,
                                                    const Node* __restrict__ nodes,
                                                    const float4* __restrict__ rays,
                                                    const uint32_t* __restrict__ order, int count,
+                                                   int spread,
                                                    unsigned long long* __restrict__ out,
                                                    int* __restrict__ ids,
                                                    int max_iter, unsigned long long* __restrict__ stats,
                                                    const Node* __restrict__ lnodes = nullptr) {
     cudaGridDependencySynchronize();  // the order, when the ordering kernels launched it early
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < count;
+    int i;
+    const bool active = ray_of_thread(count, spread, i);
     Trav tv;
     __shared__ float4 tails[kBlock];
     if (active) {
@@ -527,11 +537,12 @@ __global__ __launch_bounds__(kBlock) void k_ray_wide(const WideNode* __restrict_
                                                     const float4* __restrict__ leaves,
                                                     const float4* __restrict__ rays,
                                                     const uint32_t* __restrict__ order, int count,
+                                                    int spread,
                                                     unsigned long long* __restrict__ out,
                                                     int* __restrict__ ids,
                                                     int max_iter, unsigned long long* __restrict__ stats) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < count;
+    int i;
+    const bool active = ray_of_thread(count, spread, i);
     Trav tv;
     __shared__ float4 tails[kBlock];
     if (active) {
@@ -552,9 +563,16 @@ __global__ __launch_bounds__(kBlock) void k_ray_wide(const WideNode* __restrict_
 // queries in blocks of 256 would occupy only some of the 148 SMs, and these latency-bound
 // traversals run faster spread over all of them; large batches keep 256.
 inline int query_block(int count) { return count <= 148 * 512 ? 64 : kBlock; }
-// Rays: a few thousand diverge from the first node, and one warp per SM then leaves the L1 to
-// itself.
-inline int ray_block(int count) { return count <= 148 * 64 ? 32 : query_block(count); }
+// Rays: the most lanes per ray (ray_of_thread), up to 8, that keep the batch's threads within about
+// three quarters of a full GPU.  Every lane -> every 2nd, 4th, 8th, us: terrain of 8,192 triangles,
+// 2,048 rays 43, 36, 31, 26; 131,072 triangles, 12,000 rays 99, 85, 72, 67 and 24,000 rays 104, 89,
+// 77, 116; 48,000 rays 112, 97, 141, 176; city (SAH) 24,000 rays 53, 46, 43, 55.
+inline int ray_spread(int count) {
+    int s = 3;
+    while (s > 0 && (static_cast<long long>(count) << s) > 148 * 768) --s;
+    return s;
+}
+
 // the same for the lane-group kernels, counted in threads
 inline int split_block(int count, int lanes) {
     return static_cast<long long>(count) * lanes <= 148 * 2048 ? 64 : kBlock;
@@ -1600,17 +1618,19 @@ int ray_query(const qk_tree* t, const void* rays, int count, uint64_t* out, int*
     auto* res = reinterpret_cast<unsigned long long*>(out);
     auto* stt = reinterpret_cast<unsigned long long*>(stats);
     const float4* leaves = static_cast<const float4*>(t->leaves);
-    const int rb = ray_block(count);
-    const int g = blocks_for(count, rb);
-    const int g256 = blocks_for(count);  // the short stack's shared arrays are sized for 256 threads
+    const int sp = ray_spread(count);
+    const long long threads = static_cast<long long>(count) << sp;
+    const int rb = threads <= 148 * 512 ? 64 : kBlock;
+    const int g = blocks_for(threads, rb);
+    const int g256 = blocks_for(threads);  // the short stack's shared arrays are sized for 256 threads
     if (flags & QK_WIDE) {
         const WideNode* wn = static_cast<const WideNode*>(t->wide);
         if (t->wide_leaf == 4) {
-            if (stt) k_ray_wide<true, true><<<g, rb, 0, s>>>(wn, leaves, r4, order, count, res, ids, t->n * 2 + 64, stt);
-            else k_ray_wide<false, true><<<g, rb, 0, s>>>(wn, leaves, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            if (stt) k_ray_wide<true, true><<<g, rb, 0, s>>>(wn, leaves, r4, order, count, sp, res, ids, t->n * 2 + 64, stt);
+            else k_ray_wide<false, true><<<g, rb, 0, s>>>(wn, leaves, r4, order, count, sp, res, ids, t->n * 2 + 64, stt);
         } else {
-            if (stt) k_ray_wide<true><<<g, rb, 0, s>>>(wn, leaves, r4, order, count, res, ids, t->n * 2 + 64, stt);
-            else k_ray_wide<false><<<g, rb, 0, s>>>(wn, leaves, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            if (stt) k_ray_wide<true><<<g, rb, 0, s>>>(wn, leaves, r4, order, count, sp, res, ids, t->n * 2 + 64, stt);
+            else k_ray_wide<false><<<g, rb, 0, s>>>(wn, leaves, r4, order, count, sp, res, ids, t->n * 2 + 64, stt);
         }
     } else if (flags & QK_TUNE_DYNAMIC) {
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
@@ -1637,33 +1657,33 @@ int ray_query(const qk_tree* t, const void* rays, int count, uint64_t* out, int*
         if (!(flags & QK_TUNE_LEAF4) && reinterpret_cast<uintptr_t>(bn) % 32 != 0)
             flags |= QK_TUNE_SHORT_STACK;
         if ((flags & QK_TUNE_HIGH_OCC) && (flags & QK_TUNE_SHORT_STACK)) {
-            if (stt) k_ray_bin<true, 5, 8><<<g256, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
-            else k_ray_bin<false, 5, 8><<<g256, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            if (stt) k_ray_bin<true, 5, 8><<<g256, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt);
+            else k_ray_bin<false, 5, 8><<<g256, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt);
         } else if (flags & QK_TUNE_SHORT_STACK) {
-            if (stt) k_ray_bin<true, 1, 8><<<g256, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
-            else k_ray_bin<false, 1, 8><<<g256, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            if (stt) k_ray_bin<true, 1, 8><<<g256, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt);
+            else k_ray_bin<false, 1, 8><<<g256, kBlock, 0, s>>>(bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt);
         } else if ((flags & QK_TUNE_HIGH_OCC) && (flags & QK_TUNE_LEAF4)) {
-            if (stt) k_ray_bin<true, 5, 0, true><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
-            else k_ray_bin<false, 5, 0, true><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
+            if (stt) k_ray_bin<true, 5, 0, true><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
+            else k_ray_bin<false, 5, 0, true><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
         } else if (flags & QK_TUNE_LEAF4) {
-            if (stt) k_ray_bin<true, 1, 0, true><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
-            else k_ray_bin<false, 1, 0, true><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
+            if (stt) k_ray_bin<true, 1, 0, true><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
+            else k_ray_bin<false, 1, 0, true><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt, leaf_nodes(t));
         } else if (order) {
             // the previous kernel in the stream wrote the order: start while it drains
             const Node* no_leaf4 = nullptr;
             if (flags & QK_TUNE_HIGH_OCC) {
-                if (stt) launch_pdl(k_ray_bin<true, 5>, dim3(g), dim3(rb), s, bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, no_leaf4);
-                else launch_pdl(k_ray_bin<false, 5>, dim3(g), dim3(rb), s, bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, no_leaf4);
+                if (stt) launch_pdl(k_ray_bin<true, 5>, dim3(g), dim3(rb), s, bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt, no_leaf4);
+                else launch_pdl(k_ray_bin<false, 5>, dim3(g), dim3(rb), s, bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt, no_leaf4);
             } else {
-                if (stt) launch_pdl(k_ray_bin<true, 1>, dim3(g), dim3(rb), s, bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, no_leaf4);
-                else launch_pdl(k_ray_bin<false, 1>, dim3(g), dim3(rb), s, bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt, no_leaf4);
+                if (stt) launch_pdl(k_ray_bin<true, 1>, dim3(g), dim3(rb), s, bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt, no_leaf4);
+                else launch_pdl(k_ray_bin<false, 1>, dim3(g), dim3(rb), s, bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt, no_leaf4);
             }
         } else if (flags & QK_TUNE_HIGH_OCC) {
-            if (stt) k_ray_bin<true, 5><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
-            else k_ray_bin<false, 5><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            if (stt) k_ray_bin<true, 5><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt);
+            else k_ray_bin<false, 5><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt);
         } else {
-            if (stt) k_ray_bin<true, 1><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
-            else k_ray_bin<false, 1><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, res, ids, t->n * 2 + 64, stt);
+            if (stt) k_ray_bin<true, 1><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt);
+            else k_ray_bin<false, 1><<<g, rb, 0, s>>>(bn, leaves, nodes, r4, order, count, sp, res, ids, t->n * 2 + 64, stt);
         }
     }
     const cudaError_t e = cudaGetLastError();

@@ -182,3 +182,18 @@ def test_radius_workspace_of_a_large_batch_serves_small_ones(cuda):
     for flags in (0, capi.QK_TUNE_STASH, capi.QK_TUNE_SPLIT4, capi.QK_WIDE):
         sizes = [L.qk_radius_workspace_bytes(n, flags) for n in (1, 500, 32768, 32769, 40000, 200000)]
         assert sizes == sorted(sizes)
+
+
+@pytest.mark.parametrize("count", [1, 33, 14207, 14208, 14209, 28417, 56833, 113665])
+def test_spread_rays(cuda, count):
+    """Batches around the sizes where fewer lanes of a warp hold a ray."""
+    tris = workloads.terrain(24, 4)
+    lo, hi = workloads.bounds_of(tris)
+    rays = workloads.down_rays(count, float(lo[0]), float(hi[0]), float(lo[1]), float(hi[1]), 100.0, 4)
+    rays[1::3, 3:6] = [0.3, -0.2, -0.9]
+    t, ref = capi.DeviceTree("tri", tris), oracle.LBVH("tri", tris)
+    t.build_wide()
+    want = ref.raycast(rays)
+    for f in (0, capi.QK_WIDE, capi.QK_ORDER_COHERENT | capi.QK_TUNE_HIGH_OCC, capi.QK_TUNE_SHORT_STACK,
+              capi.QK_TUNE_LEAF4):
+        assert np.array_equal(t.raycast(_dev(rays), f).cpu().numpy().view(np.uint64), want), f
