@@ -347,10 +347,11 @@ __global__ __launch_bounds__(kBlock) void k_coh_scatter(const uint32_t* __restri
 // ---------------------------------------------------------------------------------------
 // single-tree kernels: one thread per ray / query point, bodies in qk_traverse.cuh
 // ---------------------------------------------------------------------------------------
-// Ray of this thread when every 2^spread-th lane holds one.  A small batch in full warps occupies
-// few SMs, and a warp takes as many steps as its longest ray, each step's loads serving 32 nodes
-// one after the other; the same rays in a quarter of the lanes of four times the warps wait less.
-__device__ __forceinline__ bool ray_of_thread(int count, int spread, int& i) {
+// Ray or query of this thread when every 2^spread-th lane holds one.  A small batch in full warps
+// occupies few SMs, and a warp takes as many steps as its longest traversal, each step's loads
+// serving 32 nodes one after the other; the same rays in a quarter of the lanes of four times the
+// warps wait less.
+__device__ __forceinline__ bool item_of_thread(int count, int spread, int& i) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     i = t >> spread;
     return i < count && (t & ((1 << spread) - 1)) == 0;
@@ -369,7 +370,7 @@ __global__ __launch_bounds__(kBlock, kMinBlocks) void k_ray_bin(const BNode* __r
                                                    const Node* __restrict__ lnodes = nullptr) {
     cudaGridDependencySynchronize();  // the order, when the ordering kernels launched it early
     int i;
-    const bool active = ray_of_thread(count, spread, i);
+    const bool active = item_of_thread(count, spread, i);
     Trav tv;
     __shared__ float4 tails[kBlock];
     if (active) {
@@ -542,7 +543,7 @@ __global__ __launch_bounds__(kBlock) void k_ray_wide(const WideNode* __restrict_
                                                     int* __restrict__ ids,
                                                     int max_iter, unsigned long long* __restrict__ stats) {
     int i;
-    const bool active = ray_of_thread(count, spread, i);
+    const bool active = item_of_thread(count, spread, i);
     Trav tv;
     __shared__ float4 tails[kBlock];
     if (active) {
@@ -563,11 +564,11 @@ __global__ __launch_bounds__(kBlock) void k_ray_wide(const WideNode* __restrict_
 // queries in blocks of 256 would occupy only some of the 148 SMs, and these latency-bound
 // traversals run faster spread over all of them; large batches keep 256.
 inline int query_block(int count) { return count <= 148 * 512 ? 64 : kBlock; }
-// Rays: the most lanes per ray (ray_of_thread), up to 8, that keep the batch's threads within about
+// The most lanes per ray or query (item_of_thread), up to 8, that keep the batch's threads within about
 // three quarters of a full GPU.  Every lane -> every 2nd, 4th, 8th, us: terrain of 8,192 triangles,
 // 2,048 rays 43, 36, 31, 26; 131,072 triangles, 12,000 rays 99, 85, 72, 67 and 24,000 rays 104, 89,
 // 77, 116; 48,000 rays 112, 97, 141, 176; city (SAH) 24,000 rays 53, 46, 43, 55.
-inline int ray_spread(int count) {
+inline int lane_spread(int count) {
     int s = 3;
     while (s > 0 && (static_cast<long long>(count) << s) > 148 * 768) --s;
     return s;
@@ -609,12 +610,12 @@ __global__ __launch_bounds__(kBlock) void k_closest_bin(const BNode* __restrict_
                                                        const float4* __restrict__ leaves,
                                                        const float* __restrict__ pts,
                                                        const uint32_t* __restrict__ order,
-                                                       int count, uint2* __restrict__ out,
+                                                       int count, int spread, uint2* __restrict__ out,
                                                        int max_iter, unsigned long long* __restrict__ stats,
                                                        const Node* __restrict__ lnodes = nullptr,
                                                        TailList tail = TailList{}) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < count;
+    int i;
+    const bool active = item_of_thread(count, spread, i);
     Trav tv;
     if (active) {
         const int q = order ? static_cast<int>(order[i]) : i;
@@ -632,10 +633,10 @@ __global__ __launch_bounds__(kBlock) void k_closest_wide(const WideNode* __restr
                                                         const float4* __restrict__ leaves,
                                                         const float* __restrict__ pts,
                                                         const uint32_t* __restrict__ order,
-                                                        int count, uint2* __restrict__ out,
+                                                        int count, int spread, uint2* __restrict__ out,
                                                         int max_iter, unsigned long long* __restrict__ stats) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < count;
+    int i;
+    const bool active = item_of_thread(count, spread, i);
     Trav tv;
     if (active) {
         const int q = order ? static_cast<int>(order[i]) : i;
@@ -650,13 +651,13 @@ template <class Ops, int K, bool kStats, bool kLeaf4 = false>
 __global__ __launch_bounds__(kBlock) void k_knn_bin(const BNode* __restrict__ bn,
                                                    const float4* __restrict__ leaves,
                                                    const float* __restrict__ pts,
-                                                   const uint32_t* __restrict__ order, int count,
+                                                   const uint32_t* __restrict__ order, int count, int spread,
                                                    int k, int stride, uint2* __restrict__ out,
                                                    int max_iter, unsigned long long* __restrict__ stats,
                                                    const Node* __restrict__ lnodes = nullptr,
                                                    TailList tail = TailList{}) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < count;
+    int i;
+    const bool active = item_of_thread(count, spread, i);
     Trav tv;
     if (active) {
         const int q = order ? static_cast<int>(order[i]) : i;
@@ -675,11 +676,11 @@ template <class Ops, int K, bool kStats, bool kRange = false>
 __global__ __launch_bounds__(kBlock) void k_knn_wide(const WideNode* __restrict__ wn,
                                                     const float4* __restrict__ leaves,
                                                     const float* __restrict__ pts,
-                                                    const uint32_t* __restrict__ order, int count,
+                                                    const uint32_t* __restrict__ order, int count, int spread,
                                                     int k, int stride, uint2* __restrict__ out,
                                                     int max_iter, unsigned long long* __restrict__ stats) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < count;
+    int i;
+    const bool active = item_of_thread(count, spread, i);
     Trav tv;
     if (active) {
         const int q = order ? static_cast<int>(order[i]) : i;
@@ -696,12 +697,12 @@ __global__ __launch_bounds__(kBlock) void k_knn_wide(const WideNode* __restrict_
 template <class Ops, bool kFill, bool kStats, bool kLeaf4 = false>
 __global__ __launch_bounds__(kBlock) void k_radius_bin(
     const BNode* __restrict__ bn, const float4* __restrict__ leaves, const Node* __restrict__ nodes,
-    const float* __restrict__ pts, const uint32_t* __restrict__ order, int count, float r2,
+    const float* __restrict__ pts, const uint32_t* __restrict__ order, int count, int spread, float r2,
     int* __restrict__ counts, const int* __restrict__ offsets,
     unsigned long long* __restrict__ keys, int max_iter, unsigned long long* __restrict__ stats,
     const Node* __restrict__ lnodes = nullptr) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < count;
+    int i;
+    const bool active = item_of_thread(count, spread, i);
     Trav tv;
     if (active) {
         const int q = order ? static_cast<int>(order[i]) : i;
@@ -724,11 +725,11 @@ __global__ __launch_bounds__(kBlock) void k_radius_bin(
 template <class Ops, bool kStats, bool kLeaf4 = false>
 __global__ __launch_bounds__(kBlock) void k_radius_count_pool(
     const BNode* __restrict__ bn, const float4* __restrict__ leaves, const Node* __restrict__ nodes,
-    const float* __restrict__ pts, const uint32_t* __restrict__ order, int count, float r2,
+    const float* __restrict__ pts, const uint32_t* __restrict__ order, int count, int spread, float r2,
     int* __restrict__ counts, RadiusPool pool, int max_iter,
     unsigned long long* __restrict__ stats, const Node* __restrict__ lnodes = nullptr) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < count;
+    int i;
+    const bool active = item_of_thread(count, spread, i);
     Trav tv;
     if (active) {
         const int q = order ? static_cast<int>(order[i]) : i;
@@ -764,12 +765,12 @@ __global__ __launch_bounds__(kBlock) void k_radius_fill_lost(
 template <class Ops, bool kFill, bool kStats, bool kRange = false>
 __global__ __launch_bounds__(kBlock) void k_radius_wide(
     const WideNode* __restrict__ wn, const float4* __restrict__ leaves,
-    const float* __restrict__ pts, const uint32_t* __restrict__ order, int count, float r2,
+    const float* __restrict__ pts, const uint32_t* __restrict__ order, int count, int spread, float r2,
     int* __restrict__ counts, const int* __restrict__ offsets,
     unsigned long long* __restrict__ keys, int max_iter, unsigned long long* __restrict__ stats,
     const Node* __restrict__ lnodes = nullptr) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = i < count;
+    int i;
+    const bool active = item_of_thread(count, spread, i);
     Trav tv;
     if (active) {
         const int q = order ? static_cast<int>(order[i]) : i;
@@ -1401,8 +1402,9 @@ int closest_impl(const qk_tree* t, const float* pts, int count, uint2* out, unsi
                  unsigned long long* stats, const uint32_t* order, cudaStream_t s,
                  const TailList& tail = TailList{}) {
     const float4* leaves = static_cast<const float4*>(t->leaves);
-    const int qb = query_block(count);
-    const int g = blocks_for(count, qb);
+    const int sp = lane_spread(count);
+    const int qb = query_block(count << sp);
+    const int g = blocks_for(static_cast<long long>(count) << sp, qb);
     const bool wide = (flags & QK_WIDE) != 0;
     const bool st = stats != nullptr;
     if (!st) flags = few_flags(flags, count);
@@ -1414,7 +1416,7 @@ int closest_impl(const qk_tree* t, const float* pts, int count, uint2* out, unsi
             launch_closest_split<Ops, false>(split_lanes(flags), bn, leaves, pts, order, count, out,
                                              kTailBudgetLane, nullptr, tail, s);
         else
-            k_closest_bin<Ops, false><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, out,
+            k_closest_bin<Ops, false><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, sp, out,
                                                            kTailBudgetThread, nullptr, nullptr, tail);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_status(e, "closest (tail)");
@@ -1423,11 +1425,11 @@ int closest_impl(const qk_tree* t, const float* pts, int count, uint2* out, unsi
     if (wide) {
         const WideNode* wn = static_cast<const WideNode*>(t->wide);
         if (t->wide_leaf == 4) {
-            if (st) k_closest_wide<Ops, true, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, out, t->n * 2 + 64, stats);
-            else k_closest_wide<Ops, false, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, out, t->n * 2 + 64, stats);
+            if (st) k_closest_wide<Ops, true, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, sp, out, t->n * 2 + 64, stats);
+            else k_closest_wide<Ops, false, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, sp, out, t->n * 2 + 64, stats);
         } else {
-            if (st) k_closest_wide<Ops, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, out, t->n * 2 + 64, stats);
-            else k_closest_wide<Ops, false><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, out, t->n * 2 + 64, stats);
+            if (st) k_closest_wide<Ops, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, sp, out, t->n * 2 + 64, stats);
+            else k_closest_wide<Ops, false><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, sp, out, t->n * 2 + 64, stats);
         }
     } else if (flags & kSplitFlags) {
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
@@ -1435,12 +1437,12 @@ int closest_impl(const qk_tree* t, const float* pts, int count, uint2* out, unsi
         else launch_closest_split<Ops, false>(split_lanes(flags), bn, leaves, pts, order, count, out, t->n * 2 + 64, stats, TailList{}, s);
     } else if (flags & QK_TUNE_LEAF4) {
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
-        if (st) k_closest_bin<Ops, true, true><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, out, t->n * 2 + 64, stats, leaf_nodes(t));
-        else k_closest_bin<Ops, false, true><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, out, t->n * 2 + 64, stats, leaf_nodes(t));
+        if (st) k_closest_bin<Ops, true, true><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, sp, out, t->n * 2 + 64, stats, leaf_nodes(t));
+        else k_closest_bin<Ops, false, true><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, sp, out, t->n * 2 + 64, stats, leaf_nodes(t));
     } else {
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
-        if (st) k_closest_bin<Ops, true><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, out, t->n * 2 + 64, stats);
-        else k_closest_bin<Ops, false><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, out, t->n * 2 + 64, stats);
+        if (st) k_closest_bin<Ops, true><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, sp, out, t->n * 2 + 64, stats);
+        else k_closest_bin<Ops, false><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, sp, out, t->n * 2 + 64, stats);
     }
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? QK_OK : cuda_status(e, "closest");
@@ -1451,8 +1453,9 @@ void launch_knn(const qk_tree* t, const float* pts, int count, int k, int stride
                 bool wide, int split, bool leaf4, unsigned long long* stats,
                 const uint32_t* order, cudaStream_t s) {
     const float4* leaves = static_cast<const float4*>(t->leaves);
-    const int qb = query_block(count);
-    const int g = blocks_for(count, qb);
+    const int sp = lane_spread(count);
+    const int qb = query_block(count << sp);
+    const int g = blocks_for(static_cast<long long>(count) << sp, qb);
     if (split && !wide) {
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
         const int lanes = knn_lanes(split, k);
@@ -1461,20 +1464,20 @@ void launch_knn(const qk_tree* t, const float* pts, int count, int k, int stride
     } else if (wide) {
         const WideNode* wn = static_cast<const WideNode*>(t->wide);
         if (t->wide_leaf == 4) {
-            if (stats) k_knn_wide<Ops, K, true, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, k, stride, out, t->n * 2 + 64, stats);
-            else k_knn_wide<Ops, K, false, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, k, stride, out, t->n * 2 + 64, stats);
+            if (stats) k_knn_wide<Ops, K, true, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, sp, k, stride, out, t->n * 2 + 64, stats);
+            else k_knn_wide<Ops, K, false, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, sp, k, stride, out, t->n * 2 + 64, stats);
         } else {
-            if (stats) k_knn_wide<Ops, K, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, k, stride, out, t->n * 2 + 64, stats);
-            else k_knn_wide<Ops, K, false><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, k, stride, out, t->n * 2 + 64, stats);
+            if (stats) k_knn_wide<Ops, K, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, sp, k, stride, out, t->n * 2 + 64, stats);
+            else k_knn_wide<Ops, K, false><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, sp, k, stride, out, t->n * 2 + 64, stats);
         }
     } else if (leaf4) {
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
-        if (stats) k_knn_bin<Ops, K, true, true><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, k, stride, out, t->n * 2 + 64, stats, leaf_nodes(t));
-        else k_knn_bin<Ops, K, false, true><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, k, stride, out, t->n * 2 + 64, stats, leaf_nodes(t));
+        if (stats) k_knn_bin<Ops, K, true, true><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, sp, k, stride, out, t->n * 2 + 64, stats, leaf_nodes(t));
+        else k_knn_bin<Ops, K, false, true><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, sp, k, stride, out, t->n * 2 + 64, stats, leaf_nodes(t));
     } else {
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
-        if (stats) k_knn_bin<Ops, K, true><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, k, stride, out, t->n * 2 + 64, stats);
-        else k_knn_bin<Ops, K, false><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, k, stride, out, t->n * 2 + 64, stats);
+        if (stats) k_knn_bin<Ops, K, true><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, sp, k, stride, out, t->n * 2 + 64, stats);
+        else k_knn_bin<Ops, K, false><<<g, qb, 0, s>>>(bn, leaves, pts, order, count, sp, k, stride, out, t->n * 2 + 64, stats);
     }
 }
 
@@ -1490,7 +1493,7 @@ int knn_tail(const qk_tree* t, const float* pts, int count, int k, int stride, u
                                      stride, out, kTailBudgetLane, nullptr, tail, s);
     else
         k_knn_bin<Ops, K, false><<<blocks_for(count, query_block(count)), query_block(count), 0, s>>>(
-            bn, leaves, pts, order, count, k, stride, out, kTailBudgetThread, nullptr, nullptr, tail);
+            bn, leaves, pts, order, count, 0, k, stride, out, kTailBudgetThread, nullptr, nullptr, tail);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_status(e, "knn (tail)");
     return tail_resolve<K>(t, pts, k, stride, out, tail, stats, s);
@@ -1523,8 +1526,9 @@ int radius_launch(const qk_tree* t, const float* pts, int count, float r2, int* 
                   int* lane_counts, const int* offsets, unsigned long long* keys, unsigned flags,
                   unsigned long long* stats, const uint32_t* order, cudaStream_t s) {
     const float4* leaves = static_cast<const float4*>(t->leaves);
-    const int qb = query_block(count);
-    const int g = blocks_for(count, qb);
+    const int sp = lane_spread(count);
+    const int qb = query_block(count << sp);
+    const int g = blocks_for(static_cast<long long>(count) << sp, qb);
     if ((flags & kSplitFlags) && !(flags & QK_WIDE)) {
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
         const int lanes = split_lanes(flags);
@@ -1543,22 +1547,22 @@ int radius_launch(const qk_tree* t, const float* pts, int count, float r2, int* 
     } else if (flags & QK_WIDE) {
         const WideNode* wn = static_cast<const WideNode*>(t->wide);
         if (t->wide_leaf == 4) {
-            if (stats) k_radius_wide<Ops, kFill, true, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, r2, counts, offsets, keys, t->n * 2 + 64, stats);
-            else k_radius_wide<Ops, kFill, false, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, r2, counts, offsets, keys, t->n * 2 + 64, stats);
+            if (stats) k_radius_wide<Ops, kFill, true, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, sp, r2, counts, offsets, keys, t->n * 2 + 64, stats);
+            else k_radius_wide<Ops, kFill, false, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, sp, r2, counts, offsets, keys, t->n * 2 + 64, stats);
         } else {
-            if (stats) k_radius_wide<Ops, kFill, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, r2, counts, offsets, keys, t->n * 2 + 64, stats);
-            else k_radius_wide<Ops, kFill, false><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, r2, counts, offsets, keys, t->n * 2 + 64, stats);
+            if (stats) k_radius_wide<Ops, kFill, true><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, sp, r2, counts, offsets, keys, t->n * 2 + 64, stats);
+            else k_radius_wide<Ops, kFill, false><<<g, qb, 0, s>>>(wn, leaves, pts, order, count, sp, r2, counts, offsets, keys, t->n * 2 + 64, stats);
         }
     } else if (flags & QK_TUNE_LEAF4) {
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
         const Node* nodes = static_cast<const Node*>(t->nodes);
-        if (stats) k_radius_bin<Ops, kFill, true, true><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, r2, counts, offsets, keys, t->n * 2 + 64, stats, leaf_nodes(t));
-        else k_radius_bin<Ops, kFill, false, true><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, r2, counts, offsets, keys, t->n * 2 + 64, stats, leaf_nodes(t));
+        if (stats) k_radius_bin<Ops, kFill, true, true><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, sp, r2, counts, offsets, keys, t->n * 2 + 64, stats, leaf_nodes(t));
+        else k_radius_bin<Ops, kFill, false, true><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, sp, r2, counts, offsets, keys, t->n * 2 + 64, stats, leaf_nodes(t));
     } else {
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
         const Node* nodes = static_cast<const Node*>(t->nodes);
-        if (stats) k_radius_bin<Ops, kFill, true><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, r2, counts, offsets, keys, t->n * 2 + 64, stats);
-        else k_radius_bin<Ops, kFill, false><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, r2, counts, offsets, keys, t->n * 2 + 64, stats);
+        if (stats) k_radius_bin<Ops, kFill, true><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, sp, r2, counts, offsets, keys, t->n * 2 + 64, stats);
+        else k_radius_bin<Ops, kFill, false><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, sp, r2, counts, offsets, keys, t->n * 2 + 64, stats);
     }
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? QK_OK : cuda_status(e, "radius traversal");
@@ -1618,7 +1622,7 @@ int ray_query(const qk_tree* t, const void* rays, int count, uint64_t* out, int*
     auto* res = reinterpret_cast<unsigned long long*>(out);
     auto* stt = reinterpret_cast<unsigned long long*>(stats);
     const float4* leaves = static_cast<const float4*>(t->leaves);
-    const int sp = ray_spread(count);
+    const int sp = lane_spread(count);
     const long long threads = static_cast<long long>(count) << sp;
     const int rb = threads <= 148 * 512 ? 64 : kBlock;
     const int g = blocks_for(threads, rb);
@@ -1788,8 +1792,9 @@ int radius_pool_launch(const qk_tree* t, const float* pts, int count, float r2, 
     const BNode* bn = static_cast<const BNode*>(t->bnodes);
     const Node* nodes = static_cast<const Node*>(t->nodes);
     const float4* leaves = static_cast<const float4*>(t->leaves);
-    const int qb = query_block(count);
-    const int g = blocks_for(count, qb);
+    const int sp = lane_spread(count);
+    const int qb = query_block(count << sp);
+    const int g = blocks_for(static_cast<long long>(count) << sp, qb);
     const int it = t->n * 2 + 64;
     const bool leaf4 = (flags & QK_TUNE_LEAF4) != 0;
     if (bufs.lane_counts) {
@@ -1813,11 +1818,11 @@ int radius_pool_launch(const qk_tree* t, const float* pts, int count, float r2, 
     } else {
         cudaMemsetAsync(pool.taken, 0, sizeof(int), s);
         if (leaf4) {
-            if (stats) k_radius_count_pool<Ops, true, true><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, r2, counts, pool, it, stats, leaf_nodes(t));
-            else k_radius_count_pool<Ops, false, true><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, r2, counts, pool, it, stats, leaf_nodes(t));
+            if (stats) k_radius_count_pool<Ops, true, true><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, sp, r2, counts, pool, it, stats, leaf_nodes(t));
+            else k_radius_count_pool<Ops, false, true><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, sp, r2, counts, pool, it, stats, leaf_nodes(t));
         } else {
-            if (stats) k_radius_count_pool<Ops, true><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, r2, counts, pool, it, stats);
-            else k_radius_count_pool<Ops, false><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, r2, counts, pool, it, stats);
+            if (stats) k_radius_count_pool<Ops, true><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, sp, r2, counts, pool, it, stats);
+            else k_radius_count_pool<Ops, false><<<g, qb, 0, s>>>(bn, leaves, nodes, pts, order, count, sp, r2, counts, pool, it, stats);
         }
     }
     const cudaError_t e = cudaGetLastError();

@@ -197,3 +197,20 @@ def test_spread_rays(cuda, count):
     for f in (0, capi.QK_WIDE, capi.QK_ORDER_COHERENT | capi.QK_TUNE_HIGH_OCC, capi.QK_TUNE_SHORT_STACK,
               capi.QK_TUNE_LEAF4):
         assert np.array_equal(t.raycast(_dev(rays), f).cpu().numpy().view(np.uint64), want), f
+
+
+@pytest.mark.parametrize("count", [14208, 14209, 28417, 40001, 56833])
+def test_spread_queries(cuda, count):
+    """Thread-per-query kernels around the sizes where fewer lanes of a warp hold a query."""
+    pts = _points(1500, 3, 700)
+    q = workloads.uniform_points(count, [-5.0] * 3, [105.0] * 3, 3, 13)
+    t, ref = capi.DeviceTree("point", pts), oracle.LBVH("point", pts)
+    t.build_wide()
+    woff, wkeys = ref.radius(q, 9.0)
+    closest, knn = ref.closest(q), ref.knn(q, 9)
+    for f in (0, capi.QK_WIDE, capi.QK_TUNE_LEAF4, capi.QK_TUNE_STASH):
+        assert np.array_equal(t.closest(_dev(q), f).cpu().numpy().view(np.uint32), closest), f
+        assert np.array_equal(t.knn(_dev(q), 9, f).cpu().numpy().view(np.uint32), knn), f
+        off, keys = t.radius(_dev(q), 9.0, f)
+        assert np.array_equal(off.cpu().numpy().astype(np.int64), woff), f
+        assert np.array_equal(keys.cpu().numpy().view(np.uint64), wkeys), f
