@@ -94,15 +94,32 @@ template <class Ops>
 __global__ __launch_bounds__(kBlock) void k_morton(const float* __restrict__ items, int n,
                                                    const Header* __restrict__ h,
                                                    uint32_t* __restrict__ codes,
-                                                   int* __restrict__ flags) {
-    const int i = blockIdx.x * kBlock + threadIdx.x;
-    if (i >= n) return;
-    if (i < n - 1) flags[i] = 0;  // the tree pass's arrival words
+                                                   int* __restrict__ flags,
+                                                   uint32_t* __restrict__ totals) {
+    __shared__ uint32_t digits[kSortPasses * kSortRadix];
+    if (totals) {
+        for (int j = threadIdx.x; j < kSortPasses * kSortRadix; j += kBlock) digits[j] = 0;
+        __syncthreads();
+    }
     const float lx = unord_f(h->lo[0]), ly = unord_f(h->lo[1]), lz = unord_f(h->lo[2]);
     const float hx = unord_f(h->hi[0]), hy = unord_f(h->hi[1]), hz = unord_f(h->hi[2]);
-    const float3 c = Ops::centroid(items + static_cast<size_t>(i) * Ops::kFloats);
-    codes[i] = spread10(quant(c.x, lx, hx - lx)) | (spread10(quant(c.y, ly, hy - ly)) << 1) |
-               (spread10(quant(c.z, lz, hz - lz)) << 2);
+    for (int i = blockIdx.x * kBlock + threadIdx.x; i < n; i += kBlock * gridDim.x) {
+        if (i < n - 1) flags[i] = 0;  // the tree pass's arrival words
+        const float3 c = Ops::centroid(items + static_cast<size_t>(i) * Ops::kFloats);
+        const uint32_t code = spread10(quant(c.x, lx, hx - lx)) |
+                              (spread10(quant(c.y, ly, hy - ly)) << 1) |
+                              (spread10(quant(c.z, lz, hz - lz)) << 2);
+        codes[i] = code;
+        if (totals) {
+#pragma unroll
+            for (int p = 0; p < kSortPasses; ++p)
+                atomicAdd(&digits[p * kSortRadix + ((code >> (8 * p)) & 0xffu)], 1u);
+        }
+    }
+    if (!totals) return;
+    __syncthreads();
+    for (int j = threadIdx.x; j < kSortPasses * kSortRadix; j += kBlock)
+        if (digits[j]) atomicAdd(&totals[j], digits[j]);
 }
 
 // masks of every block boundary (lbvh_boundary in qk_lbvh.cuh): warp b takes the boundary left
@@ -555,10 +572,13 @@ int build_lbvh(qk_tree* t, const void* items_v, void* ws, cudaStream_t s) {
     k_header_init<<<1, 32, 0, s>>>(h);
     const int grid = min(blocks_for(n), 148 * 8);
     k_centroid_bounds<Ops><<<grid, kBlock, 0, s>>>(items, n, h);
-    k_morton<Ops><<<blocks_for(n), kBlock, 0, s>>>(items, n, h, codes, t->flags);
+    // the codes' digits are counted as they are made (287 -> 282 us for 1,048,576 points against a
+    // pass of the sort's own)
+    uint32_t* totals = sort_begin(sort_ws, n, s);
+    k_morton<Ops><<<min(blocks_for(n), 148 * 6), kBlock, 0, s>>>(items, n, h, codes, t->flags, totals);
     stage_mark(kMarkMorton, s);
     SortedPairs order;
-    cudaError_t e = sort_pairs(codes, idx, codes_s, idx_s, n, 30, sort_ws, s, &order, true);
+    cudaError_t e = sort_pairs(codes, idx, codes_s, idx_s, n, 30, sort_ws, s, &order, true, true);
     if (e != cudaSuccess) return cuda_status(e, "build sort");
     stage_mark(kMarkSort, s);
     LbvhView v;

@@ -136,9 +136,15 @@ struct SortedPairs {
     const uint32_t* keys;
     const uint32_t* vals;
 };
+// For a caller that makes its keys in a kernel of its own: clears the sort's counters in `ws` and
+// returns where that kernel adds every pass's digit counts (kSortPasses x kSortRadix words; key
+// digit p is bits 8p..8p+7), to be followed by sort_pairs(..., counted = true) with the same n and
+// ws.  nullptr: nothing to count (one tile of keys).
+constexpr int kSortRadix = 256, kSortPasses = 4;
+uint32_t* sort_begin(void* ws, int n, cudaStream_t s);
 cudaError_t sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout,
                        int n, int bits, void* ws, cudaStream_t s, SortedPairs* sorted = nullptr,
-                       bool iota = false);
+                       bool iota = false, bool counted = false);
 size_t scan_ws_bytes(int n);
 // exclusive scan of n ints; writes the total to out[n] when write_total is set
 cudaError_t scan_exclusive(const int* in, int* out, int n, bool write_total, void* ws,

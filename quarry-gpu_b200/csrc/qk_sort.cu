@@ -24,7 +24,7 @@ namespace qk {
 
 namespace {
 
-constexpr int kRadix = 256;
+constexpr int kRadix = kSortRadix;
 constexpr int kWarps = kBlock / 32;
 constexpr int kItems = kSortTile / kBlock;  // 16 keys per thread
 static_assert(kItems * kBlock == kSortTile, "tile size");
@@ -118,7 +118,7 @@ __device__ __forceinline__ uint32_t rs_rank_tile(RsTile& sh, const uint32_t (&ke
 
 // What the passes share, cleared before a sort: the next tile of each pass and each pass's
 // digit totals.
-constexpr int kMaxPasses = 4;
+constexpr int kMaxPasses = kSortPasses;
 struct RsCounts {
     int ticket[kMaxPasses];
     int pad[60];
@@ -358,6 +358,16 @@ size_t sort_ws_bytes(int n) {
     return c.used;
 }
 
+uint32_t* sort_begin(void* ws, int n, cudaStream_t s) {
+    if (n <= kSortTile) return nullptr;
+    Carve c{static_cast<char*>(ws)};
+    RsCounts* counts = c.take<RsCounts>(1);
+    const char* state = c.take<char>(rs_state_bytes(n));
+    // the counters and the first pass's states are one run of bytes
+    cudaMemsetAsync(counts, 0, static_cast<size_t>(state - reinterpret_cast<char*>(counts)) + rs_state_bytes(n), s);
+    return &counts->total[0][0];
+}
+
 template <class S>
 static void rs_launch(const uint32_t* sk, const uint32_t* sv, uint32_t* dk, uint32_t* dv, int n,
                       int pass, RsCounts* c, char* state, char* next, bool iota, cudaStream_t s) {
@@ -374,7 +384,8 @@ static void rs_launch(const uint32_t* sk, const uint32_t* sv, uint32_t* dk, uint
 // One pass over 1,048,576 pairs (20 us under ncu) is bound by its latency, not by bytes (16 MB):
 // 256 tiles on 148 SMs, 16 ranking rounds each, then the earlier tiles' counts.
 cudaError_t sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout,
-                       int n, int bits, void* ws, cudaStream_t s, SortedPairs* sorted, bool iota) {
+                       int n, int bits, void* ws, cudaStream_t s, SortedPairs* sorted, bool iota,
+                       bool counted) {
     if (n <= 0) return cudaSuccess;
     const int passes = bits <= 0 ? 1 : (bits + 7) / 8;
     if (sorted) *sorted = {kout, vout};
@@ -387,9 +398,10 @@ cudaError_t sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
     char* state[2];
     state[0] = c.take<char>(rs_state_bytes(n));
     state[1] = c.take<char>(rs_state_bytes(n));
-    // the counters and the first pass's states are one run of bytes
-    cudaMemsetAsync(counts, 0, static_cast<size_t>(state[0] - reinterpret_cast<char*>(counts)) + rs_state_bytes(n), s);
-    k_rs_hist<<<min(blocks_for(n, 4 * kBlock), 148 * 4), kBlock, 0, s>>>(kin, n, passes, counts);
+    if (!counted) {
+        sort_begin(ws, n, s);
+        k_rs_hist<<<min(blocks_for(n, 4 * kBlock), 148 * 4), kBlock, 0, s>>>(kin, n, passes, counts);
+    }
     const uint32_t* sk = kin;
     const uint32_t* sv = vin;
     for (int p = 0; p < passes; ++p) {
