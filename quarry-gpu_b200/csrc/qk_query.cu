@@ -564,12 +564,13 @@ __global__ __launch_bounds__(kBlock) void k_ray_wide(const WideNode* __restrict_
 // queries in blocks of 256 would occupy only some of the 148 SMs, and these latency-bound
 // traversals run faster spread over all of them; large batches keep 256.
 inline int query_block(int count) { return count <= 148 * 512 ? 64 : kBlock; }
-// The most lanes per ray or query (item_of_thread), up to 8, that keep the batch's threads within about
-// three quarters of a full GPU.  Every lane -> every 2nd, 4th, 8th, us: terrain of 8,192 triangles,
-// 2,048 rays 43, 36, 31, 26; 131,072 triangles, 12,000 rays 99, 85, 72, 67 and 24,000 rays 104, 89,
-// 77, 116; 48,000 rays 112, 97, 141, 176; city (SAH) 24,000 rays 53, 46, 43, 55.
+// The most lanes per ray or query (item_of_thread), up to a whole warp, that keep the batch's
+// threads within about three quarters of a full GPU.  Every lane -> every 2nd, 4th, 8th, 16th, one
+// ray per warp, us: terrain of 8,192 triangles, 2,048 rays 43, 36, 31, 26, 24, 21, 6,000 rays 43,
+// 37, 30, 27, 25, 35; 131,072 triangles, 12,000 rays 99, 85, 72, 67 and 24,000 rays 104, 89, 77,
+// 116; 48,000 rays 112, 97, 141, 176; city (SAH) 24,000 rays 53, 46, 43, 55.
 inline int lane_spread(int count) {
-    int s = 3;
+    int s = 5;
     while (s > 0 && (static_cast<long long>(count) << s) > 148 * 768) --s;
     return s;
 }

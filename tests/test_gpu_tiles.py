@@ -184,7 +184,7 @@ def test_radius_workspace_of_a_large_batch_serves_small_ones(cuda):
         assert sizes == sorted(sizes)
 
 
-@pytest.mark.parametrize("count", [1, 33, 14207, 14208, 14209, 28417, 56833, 113665])
+@pytest.mark.parametrize("count", [1, 33, 3552, 3553, 7105, 14208, 14209, 28417, 56833, 113665])
 def test_spread_rays(cuda, count):
     """Batches around the sizes where fewer lanes of a warp hold a ray."""
     tris = workloads.terrain(24, 4)
