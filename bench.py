@@ -1694,20 +1694,21 @@ def batch_parity(cfg, got, threads: int):
 # ---------------------------------------------------------------------------------------
 KERNEL_CASES = {
     "build_lbvh": "LBVH build of the 1,048,576-point volume cloud (k_centroid_bounds, k_morton, "
-                  "k_rs_*, k_emit, k_bottom_up_ranged, k_depth)",
+                  "k_rs_*, k_lbvh_*)",
     "build_sah": "binned SAH build (32 bins) of the 1,310,720-triangle city (k_level_*, "
                  "k_warp_tasks, k_sah_leaves, k_bottom_up_ranged)",
     "refit": "full and 1% dirty refit of the volume cloud's LBVH (k_refit_leaves, k_bottom_up, "
              "k_dirty_mark, k_dirty_merge)",
-    "closest_tri": "20,000 closest-point queries on the terrain's LBVH, 131,072 triangles, one "
-                   "thread per query (k_closest_bin) and 4 lanes per query (k_closest_split)",
+    "closest_tri": "20,000 closest-point queries on the terrain's LBVH, 131,072 triangles, without "
+                   "a schedule flag and with 4 lanes per query (k_closest_split both)",
     "closest_gauss": "262,144 closest-ellipsoid queries on 1,048,576 Gaussians (k_closest_bin)",
     "knn_points": "kNN k=8, 20,000 queries on each 1,048,576-point cloud (k_knn_split: a warp "
                   "per query on the sphere shell's SAH tree in coherent order, then 8 lanes per "
                   "query on the uniform cloud; k_knn_bin: one thread per query on the uniform "
                   "cloud)",
     "radius_points": "radius 1.0, 20,000 queries on the uniform cloud, single pass "
-                     "(k_radius_count_pool, k_radius_gather, k_radius_fill_lost, k_seg_sort_*)",
+                     "(k_radius_count_pool_split, k_radius_gather_split, "
+                     "k_radius_fill_lost_split, k_seg_sort_*)",
     "grad": "adjoints: 262,144 Gaussian distances (k_dist_grad, k_segment_sum) and 1,000,000 "
             "terrain ray t (k_ray_grad)",
     "rays_terrain": "1,000,000 down rays on the terrain's LBVH, coherent order, 5 blocks/SM "
