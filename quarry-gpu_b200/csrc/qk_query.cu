@@ -1359,7 +1359,7 @@ inline int split_lanes(unsigned flags) {
 // radius, whose two passes must agree.
 constexpr int kFewQueries = 32768;
 constexpr unsigned kScheduleFlags = kSplitFlags | QK_WIDE | QK_TUNE_LEAF4 | QK_TUNE_STASH | QK_TUNE_TAIL;
-inline unsigned few_flags(unsigned flags, int count) {
+inline unsigned few_flags(unsigned flags, long long count) {
     return (flags & kScheduleFlags) == 0 && count <= kFewQueries ? flags | QK_TUNE_SPLIT4 : flags;
 }
 
@@ -1505,7 +1505,7 @@ int knn_impl(const qk_tree* t, const float* pts, int count, int k, int stride, u
              unsigned flags, unsigned long long* stats, const uint32_t* order, cudaStream_t s,
              const TailList& tail = TailList{}) {
     const bool wide = (flags & QK_WIDE) != 0;
-    if (!stats && k <= 8) flags = few_flags(flags, count * (k <= 4 ? 1 : 2));
+    if (!stats && k <= 8) flags = few_flags(flags, (k <= 4 ? 1ll : 2ll) * count);
     const int split = split_lanes(flags);  // 0: one thread per query
     const bool leaf4 = (flags & QK_TUNE_LEAF4) != 0;
     if (tail.count) {
