@@ -48,8 +48,9 @@ constexpr int emit_stage_floats() {
 // 40-byte items, 48-byte payloads) the sorted items, leaf nodes and leaf payloads go out
 // through the warp's shared staging (16-byte aligned, emit_stage_floats<Ops>() floats) so that
 // each store instruction covers consecutive whole lines instead of one strided piece per lane
-// (city LBVH build 0.587 -> 0.572 ms); points store per lane.
-template <class Ops>
+// (city LBVH build 0.587 -> 0.572 ms); points store per lane.  kIds false: prim_ids and slot_of
+// hold these slots' ids already.
+template <class Ops, bool kIds = true>
 __device__ __forceinline__ void store_leaves_warp(const float (&it)[Ops::kFloats], int src, int n,
                                                   Node* __restrict__ nodes,
                                                   float* __restrict__ sorted,
@@ -60,7 +61,7 @@ __device__ __forceinline__ void store_leaves_warp(const float (&it)[Ops::kFloats
     const int lane = threadIdx.x & 31;
     const int k = k0 + lane;
     const bool ok = lane < m;
-    if (ok) {
+    if (kIds && ok) {
         prim_ids[k] = src;
         slot_of[src] = k;
     }
@@ -170,15 +171,13 @@ __device__ __forceinline__ Box write_node_boxes(Node* __restrict__ nodes, BNode*
 // children's slot ranges (all static during the pass): box and traversal node, with the
 // children's small-subtree codes.  kLocal: both children were finished by threads of this
 // block, whose writes a plain load sees after the block fence; otherwise they are read from L2.
-// kCodes false (refits): the small-subtree codes, which depend on the topology only, are kept.
-template <bool kLocal, bool kCodes = true>
+template <bool kLocal>
 __device__ __forceinline__ void finish_node_links(Node* __restrict__ nodes,
                                                   BNode* __restrict__ bnodes, int p, int n,
                                                   int2 lr, int2 rl, int2 rr) {
     const int l = lr.x, r = lr.y;
-    if (kCodes)
-        *reinterpret_cast<float2*>(&bnodes[p].v3.z) = make_float2(
-            __int_as_float(small_code(l, n, rl)), __int_as_float(small_code(r, n, rr)));
+    *reinterpret_cast<float2*>(&bnodes[p].v3.z) = make_float2(
+        __int_as_float(small_code(l, n, rl)), __int_as_float(small_code(r, n, rr)));
     const Box a = kLocal ? load_box_ca(nodes + l) : load_box_cg(nodes + l);
     const Box b = kLocal ? load_box_ca(nodes + r) : load_box_cg(nodes + r);
     write_node_boxes(nodes, bnodes, p, lr, a, b);
@@ -187,27 +186,33 @@ __device__ __forceinline__ void finish_node_links(Node* __restrict__ nodes,
 // Refit: one leaf's climb toward the root of a tree whose topology is unchanged; flags[p]
 // counts arrivals at internal node p, the second arrival finishes p's box and traversal node
 // (its small-subtree codes kept), resets the counter and continues.  The next level's parent
-// and links (static) are loaded while this level's arrival and boxes wait.
+// and links (static) are loaded while this level's arrival and boxes wait, and the thread
+// carries its child's box, so an arrival leaves only the sibling's to load.
 __device__ __forceinline__ void climb_refit(Node* __restrict__ nodes, BNode* __restrict__ bnodes,
                                             const int* __restrict__ parent,
                                             int* __restrict__ flags, int n, int k) {
     auto links = [&](int v) { return *reinterpret_cast<const int2*>(&nodes[v].left); };
-    int p = parent[n - 1 + k];
+    int c = n - 1 + k;
+    int p = parent[c];
     if (p < 0) return;
     int2 lr = links(p);
     int pn = parent[p];
-    const int2 none = make_int2(0, 0);
+    Box box = load_box_cg(nodes + c);
     for (int guard = 0; guard < 4096; ++guard) {
-        int2 lrn = none;
+        int2 lrn = make_int2(0, 0);
         int pnn = -1;
         if (pn >= 0) {
             lrn = links(pn);
             pnn = parent[pn];
         }
         if (arrive_add(&flags[p], 1) == 0) return;
-        finish_node_links<false, false>(nodes, bnodes, p, n, lr, none, none);
+        const bool left = lr.x == c;
+        const Box sb = load_box_cg(nodes + (left ? lr.y : lr.x));
+        const Box a = left ? box : sb, b = left ? sb : box;
+        box = write_node_boxes(nodes, bnodes, p, lr, a, b);
         flags[p] = 0;
         if (pn < 0) return;
+        c = p;
         p = pn;
         lr = lrn;
         pn = pnn;
