@@ -941,15 +941,37 @@ int tail_resolve(const qk_tree* t, const float* pts, int k, int stride, uint2* o
     return e == cudaSuccess ? QK_OK : cuda_status(e, "heavy-query tail");
 }
 
-// radius, split: the count pass stores every lane's count (lane_counts[q * 32 + lane]) and
-// the query's total; the fill pass writes each lane's keys at the query's offset plus the
-// counts of the lower lanes.
+// Where the fill pass of a split radius puts its keys: the lanes of a group share the query's
+// segment through a cursor in shared memory, so the pass needs nothing of the count pass but the
+// offsets (a caller may use another workspace, or run other queries in this one, in between).
+// The order inside a segment does not matter: it is sorted afterwards.
+struct GroupSink {
+    unsigned long long* keys;
+    int* cursor;  // keys of the segment handed out
+    int begin, end;
+    // the key before the last put's, stored once the cursor's answer has had time to arrive
+    unsigned long long held = 0;
+    int at = 0x7fffffff;
+    __device__ __forceinline__ void put(unsigned long long k) {
+        flush();
+        held = k;
+        at = begin + atomicAdd(cursor, 1);
+    }
+    __device__ __forceinline__ void flush() {
+        if (at < end) keys[at] = held;
+    }
+};
+struct NoSink {
+    __device__ __forceinline__ void put(unsigned long long) {}
+};
+
+// radius, split: the count pass stores the query's total, the fill pass its keys
 template <class Ops, bool kFill, bool kStats, int G>
 __global__ __launch_bounds__(kBlock) void k_radius_split(
     const BNode* __restrict__ bn, const float4* __restrict__ leaves, const float* __restrict__ pts,
     const uint32_t* __restrict__ order, int count, float r2, int* __restrict__ counts,
-    int* __restrict__ lane_counts, const int* __restrict__ offsets,
-    unsigned long long* __restrict__ keys, int max_iter, unsigned long long* __restrict__ stats) {
+    const int* __restrict__ offsets, unsigned long long* __restrict__ keys, int max_iter,
+    unsigned long long* __restrict__ stats) {
     if (static_cast<long long>(blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) / G >= count)
         return;  // whole warps past the last query
     bool valid;
@@ -957,24 +979,21 @@ __global__ __launch_bounds__(kBlock) void k_radius_split(
     const int q = split_query<G>(count, order, valid, lane);
     const float3 p = f3(pts[3 * q], pts[3 * q + 1], pts[3 * q + 2]);
     Trav tv;
-    int write = 0, end = 0;
-    if (kFill) {
-        // lane counts of the query: G per query at q * G
-        const int mine = valid ? lane_counts[static_cast<size_t>(q) * G + lane] : 0;
-        const int below = warp_exclusive<G>(mine, lane);  // every lane takes part
-        write = valid ? offsets[q] + below : 0;
-        end = valid ? min(write + mine, offsets[q + 1]) : 0;
-    }
-    const int found = radius_split_one<Ops, kFill, G>(bn, leaves, p, r2, lane, write, end, keys,
-                                                      max_iter, tv, valid);
-    if (!kFill) {
+    if constexpr (kFill) {
+        __shared__ int cursors[kBlock / G];
+        int* cursor = cursors + threadIdx.x / G;
+        if (lane == 0) *cursor = 0;
+        __syncwarp();
+        GroupSink sink{keys, cursor, offsets[q], offsets[q + 1]};
+        radius_split_visit<Ops, G>(bn, leaves, p, r2, lane, sink, max_iter, tv, valid);
+        sink.flush();
+    } else {
+        NoSink sink;
+        const int found = radius_split_visit<Ops, G>(bn, leaves, p, r2, lane, sink, max_iter, tv, valid);
         const int total = group_sum<G>(found);
-        if (valid) {
-            lane_counts[static_cast<size_t>(q) * G + lane] = found;
-            if (lane == 0) counts[q] = total;
-        }
+        if (valid && lane == 0) counts[q] = total;
     }
-    // a group past the last query traced query 0: it counts nothing
+    // a group past the last query traced nothing: it counts nothing
     flush_stats<kStats>(valid, valid ? tv.nodes : 0, valid ? tv.leaves : 0, valid && tv.overflow, stats);
 }
 
@@ -1524,7 +1543,7 @@ int knn_impl(const qk_tree* t, const float* pts, int count, int k, int stride, u
 
 template <class Ops, bool kFill>
 int radius_launch(const qk_tree* t, const float* pts, int count, float r2, int* counts,
-                  int* lane_counts, const int* offsets, unsigned long long* keys, unsigned flags,
+                  const int* offsets, unsigned long long* keys, unsigned flags,
                   unsigned long long* stats, const uint32_t* order, cudaStream_t s) {
     const float4* leaves = static_cast<const float4*>(t->leaves);
     const int sp = lane_spread(count);
@@ -1536,14 +1555,14 @@ int radius_launch(const qk_tree* t, const float* pts, int count, float r2, int* 
         const int sb = split_block(count, lanes);
         const int gs = blocks_for(static_cast<long long>(count) * lanes, sb);
         if (lanes == 4) {
-            if (stats) k_radius_split<Ops, kFill, true, 4><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
-            else k_radius_split<Ops, kFill, false, 4><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
+            if (stats) k_radius_split<Ops, kFill, true, 4><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, offsets, keys, t->n * 2 + 64, stats);
+            else k_radius_split<Ops, kFill, false, 4><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, offsets, keys, t->n * 2 + 64, stats);
         } else if (lanes == 8) {
-            if (stats) k_radius_split<Ops, kFill, true, 8><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
-            else k_radius_split<Ops, kFill, false, 8><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
+            if (stats) k_radius_split<Ops, kFill, true, 8><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, offsets, keys, t->n * 2 + 64, stats);
+            else k_radius_split<Ops, kFill, false, 8><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, offsets, keys, t->n * 2 + 64, stats);
         } else {
-            if (stats) k_radius_split<Ops, kFill, true, 32><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
-            else k_radius_split<Ops, kFill, false, 32><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, lane_counts, offsets, keys, t->n * 2 + 64, stats);
+            if (stats) k_radius_split<Ops, kFill, true, 32><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, offsets, keys, t->n * 2 + 64, stats);
+            else k_radius_split<Ops, kFill, false, 32><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, offsets, keys, t->n * 2 + 64, stats);
         }
     } else if (flags & QK_WIDE) {
         const WideNode* wn = static_cast<const WideNode*>(t->wide);
@@ -1571,12 +1590,12 @@ int radius_launch(const qk_tree* t, const float* pts, int count, float r2, int* 
 
 template <bool kFill>
 int radius_dispatch(const qk_tree* t, const float* pts, int count, float r2, int* counts,
-                    int* lane_counts, const int* offsets, unsigned long long* keys, unsigned flags,
+                    const int* offsets, unsigned long long* keys, unsigned flags,
                     unsigned long long* stats, const uint32_t* order, cudaStream_t s) {
     switch (t->kind) {
-        case kTri: return radius_launch<TriOps, kFill>(t, pts, count, r2, counts, lane_counts, offsets, keys, flags, stats, order, s);
-        case kPoint: return radius_launch<PointOps, kFill>(t, pts, count, r2, counts, lane_counts, offsets, keys, flags, stats, order, s);
-        case kGauss: return radius_launch<GaussOps, kFill>(t, pts, count, r2, counts, lane_counts, offsets, keys, flags, stats, order, s);
+        case kTri: return radius_launch<TriOps, kFill>(t, pts, count, r2, counts, offsets, keys, flags, stats, order, s);
+        case kPoint: return radius_launch<PointOps, kFill>(t, pts, count, r2, counts, offsets, keys, flags, stats, order, s);
+        case kGauss: return radius_launch<GaussOps, kFill>(t, pts, count, r2, counts, offsets, keys, flags, stats, order, s);
         default: return fail(QK_ERR_INVALID, "unknown primitive kind %d", t->kind);
     }
 }
@@ -1767,14 +1786,12 @@ PoolBufs carve_pool_lanes(Carve& c, int count, unsigned flags) {
 }
 
 static size_t radius_need(int count, unsigned flags) {
-    flags = few_flags(flags, count);
     Carve c;
     carve_order(c, count);
     c.take<int>(count);            // counts
     c.take<char>(scan_ws_bytes(count));
     c.take<int>(count);            // medium segment list
     c.take<int>(count);            // large segment list
-    if (flags & kSplitFlags) c.take<int>(static_cast<size_t>(count) * 32);  // lane counts
     if (use_stash(flags)) carve_pool_lanes(c, count, flags);
     return c.used;
 }
@@ -1856,7 +1873,6 @@ int radius_count(const qk_tree* t, const float* pts, int count, float r, int* of
     void* scan_ws = c.take<char>(scan_ws_bytes(count));
     c.take<int>(count);
     c.take<int>(count);
-    int* lane_counts = (flags & kSplitFlags) ? c.take<int>(static_cast<size_t>(count) * 32) : nullptr;
     const bool pooled = use_stash(flags);
     const PoolBufs pool = pooled ? carve_pool_lanes(c, count, flags) : PoolBufs{};
     int st = QK_OK;
@@ -1866,7 +1882,7 @@ int radius_count(const qk_tree* t, const float* pts, int count, float r, int* of
         st = radius_pool_dispatch(t, pts, count, r * r, counts, nullptr, pool, nullptr, flags,
                                   reinterpret_cast<unsigned long long*>(stats), order, false, s);
     else
-        st = radius_dispatch<false>(t, pts, count, r * r, counts, lane_counts, nullptr, nullptr, flags,
+        st = radius_dispatch<false>(t, pts, count, r * r, counts, nullptr, nullptr, flags,
                                     reinterpret_cast<unsigned long long*>(stats), order, s);
     if (st != QK_OK) return st;
     cudaError_t e = scan_exclusive(counts, offsets, count, true, scan_ws, s);
@@ -1889,7 +1905,6 @@ int radius_fill(const qk_tree* t, const float* pts, int count, float r, const in
     c.take<char>(scan_ws_bytes(count));
     int* medium = c.take<int>(count);
     int* large = c.take<int>(count);
-    int* lane_counts = (flags & kSplitFlags) ? c.take<int>(static_cast<size_t>(count) * 32) : nullptr;
     const bool pooled = use_stash(flags);
     const PoolBufs pool = pooled ? carve_pool_lanes(c, count, flags) : PoolBufs{};
     auto* k64 = reinterpret_cast<unsigned long long*>(keys);
@@ -1904,8 +1919,8 @@ int radius_fill(const qk_tree* t, const float* pts, int count, float r, const in
     }
     const uint32_t* order = make_order(pts, 3, 0, count, flags, o, s, &st);
     if (st != QK_OK) return st;
-    st = radius_dispatch<true>(t, pts, count, r * r, nullptr, lane_counts, offsets, k64, flags,
-                               nullptr, order, s);
+    st = radius_dispatch<true>(t, pts, count, r * r, nullptr, offsets, k64, flags, nullptr, order,
+                               s);
     if (st != QK_OK) return st;
     // reset the segment lists (make_order only resets them on its Morton path)
     return radius_sort_segments(offsets, count, keys, medium, large, o.h, -1, s);

@@ -214,3 +214,39 @@ def test_spread_queries(cuda, count):
         off, keys = t.radius(_dev(q), 9.0, f)
         assert np.array_equal(off.cpu().numpy().astype(np.int64), woff), f
         assert np.array_equal(keys.cpu().numpy().view(np.uint64), wkeys), f
+
+
+@pytest.mark.parametrize("flags", [0, capi.QK_ORDER_MORTON, capi.QK_TUNE_SPLIT4, capi.QK_TUNE_SPLIT8,
+                                   capi.QK_TUNE_SPLIT, capi.QK_WIDE, capi.QK_TUNE_LEAF4])
+@pytest.mark.parametrize("count", [1, 33, 400])
+def test_radius_fill_needs_only_the_offsets(cuda, flags, count):
+    """Two queries counted before either is filled, in one workspace, and a fill in a workspace of
+    its own: without the single-pass flag the fill pass takes nothing but the offsets."""
+    import ctypes
+
+    L = capi.lib()
+    pts = _points(2000, 4, 900)
+    t, ref = capi.DeviceTree("point", pts), oracle.LBVH("point", pts)
+    t.build_wide()
+    nb = int(L.qk_radius_workspace_bytes(count, flags))
+    shared = cuda.zeros(nb, dtype=cuda.uint8, device="cuda")
+    jobs = []
+    for seed, r in ((1, 12.0), (2, 7.0)):
+        q = workloads.uniform_points(count, [-5.0] * 3, [105.0] * 3, seed, 13)
+        off = cuda.empty(count + 1, dtype=cuda.int32, device="cuda")
+        total = ctypes.c_int64(0)
+        head = (ctypes.byref(t.t), _dev(q), count, r, off)
+        args = tuple(a.data_ptr() if hasattr(a, "data_ptr") else a for a in head)
+        capi.check(L.qk_radius_count(*args, ctypes.byref(total), flags, None, shared.data_ptr(), nb,
+                                     None), "qk_radius_count")
+        jobs.append((q, r, off, total.value, args, head))
+    for q, r, off, total, args, _ in jobs:
+        woff, wkeys = ref.radius(q, r)
+        assert np.array_equal(off.cpu().numpy().astype(np.int64), woff)
+        assert total == len(wkeys)
+        for ws in (shared, cuda.zeros(nb, dtype=cuda.uint8, device="cuda")):
+            keys = cuda.zeros(max(total, 1), dtype=cuda.int64, device="cuda")
+            capi.check(L.qk_radius_fill(*args, keys.data_ptr(), flags, ws.data_ptr(), nb, None),
+                       "qk_radius_fill")
+            cuda.cuda.synchronize()
+            assert np.array_equal(keys.cpu().numpy().view(np.uint64)[:total], wkeys), (flags, r)
