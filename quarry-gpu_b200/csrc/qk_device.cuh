@@ -424,10 +424,13 @@ __device__ __forceinline__ Box gauss_bounds(float3 mean, float4 q, float3 s) {
 // `limit`: a caller that drops distances above it gets +inf for them as soon as they are known
 // to end there, with the same bits otherwise.  Every later t of the iteration is >= lo, and
 // e_i(t) = y_i t / (t + s_i^2) only grows with t, so the final distance is at least the one at
-// a t that became lo.  Both are computed with an error below 7 ulp of |y_i| in each e_i, under
-// 30 x 2^-24 |y|^2 in their difference; the margin 1e-5 |y|^2 is five times that.  Most leaf
-// tests of a closest query are such misses, and Newton from the left is near its root after two
-// or three steps of four divisions each instead of 14.
+// a t that became lo.  While every 1 / (t + s_i^2) is finite, both are computed with an error
+// below 7 ulp of |y_i| in each e_i, under 30 x 2^-24 |y|^2 in their difference; the margin
+// 1e-5 |y|^2 is five times that.  An axis under 5.4e-20 makes its reciprocal infinite at t = 0
+// and with it e_i: such a step proves nothing and the iteration goes on (84 M random ellipsoids
+// with axes from 1e-44 to 1e19, limits at and around their distances, on the CPU: no distance
+// within the limit was cut off).  Most leaf tests of a closest query are misses, and Newton from
+// the left is near its root after two or three steps of four divisions each instead of 14.
 __device__ __forceinline__ float gauss_d2(float3 p, float3 mean, float4 q, float3 s,
                                           float limit = kInf) {
     float3 u, v, w;
@@ -459,7 +462,8 @@ __device__ __forceinline__ float gauss_d2(float3 p, float3 mean, float4 q, float
             const float e0 = y0 - gy0 * ir0 * a;
             const float e1 = y1 - gy1 * ir1 * b;
             const float e2 = y2 - gy2 * ir2 * c;
-            if (fmaf(e2, e2, fmaf(e1, e1, e0 * e0)) > over) return kInf;
+            const float so_far = fmaf(e2, e2, fmaf(e1, e1, e0 * e0));
+            if (so_far > over && so_far < kInf) return kInf;
         } else {
             hi = t;
         }

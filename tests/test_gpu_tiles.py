@@ -120,6 +120,32 @@ def test_ellipsoid_tests_end_early_with_the_same_bits(cuda, smin, smax):
         assert np.array_equal(keys.cpu().numpy().view(np.uint64), wkeys), f
 
 
+@pytest.mark.parametrize("thin", [1e-12, 6e-20, 5e-20, 1e-20, 1e-22, 1e-40])
+@pytest.mark.parametrize("axes", [1, 2])
+def test_ellipsoids_with_a_very_short_axis(cuda, thin, axes):
+    """Axes whose squares are subnormal or zero, queries nearer to a centre than the longest axis
+    (the iteration then starts at t = 0, where 1 / axis^2 overflows) and farther away: the oracle's
+    results, which its brute force confirms do not depend on the visit order."""
+    g = workloads.gaussians(300, 5.0, 20.0, 8)
+    for i in range(len(g)):
+        for a in range(axes if i % 3 else 0):  # a third keeps its axes
+            g[i, 7 + (i + a) % 3] = thin
+    q = np.concatenate([workloads.uniform_points(500, [-20.0] * 3, [120.0] * 3, 8, 13),
+                        g[:200, :3] + workloads.uniform_points(200, [-3.0] * 3, [3.0] * 3, 9, 13)])
+    t, ref = capi.DeviceTree("gauss", g), oracle.LBVH("gauss", g)
+    t.build_wide()
+    closest, knn = ref.closest(q), ref.knn(q, 6)
+    assert np.array_equal(closest, oracle.closest_brute("gauss", g, q))
+    assert np.array_equal(knn, oracle.knn_brute("gauss", g, q, 6))
+    woff, wkeys = ref.radius(q, 9.0)
+    for f in (0, capi.QK_WIDE, capi.QK_TUNE_SPLIT, capi.QK_TUNE_LEAF4):
+        assert np.array_equal(t.closest(_dev(q), f).cpu().numpy().view(np.uint32), closest), f
+        assert np.array_equal(t.knn(_dev(q), 6, f).cpu().numpy().view(np.uint32), knn), f
+        off, keys = t.radius(_dev(q), 9.0, f)
+        assert np.array_equal(off.cpu().numpy().astype(np.int64), woff), f
+        assert np.array_equal(keys.cpu().numpy().view(np.uint64), wkeys), f
+
+
 @pytest.mark.parametrize("builder", ["sah", "sah4"])
 @pytest.mark.parametrize("n", [2, 3, 5, 31, 32, 33, 64, 255, 256, 257, 600, 2048, 2049, 4500, 30011])
 @pytest.mark.parametrize("distinct", [1, 9, 1 << 30])
