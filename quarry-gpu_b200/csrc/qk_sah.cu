@@ -310,11 +310,16 @@ __device__ __forceinline__ void warp_sweep_axis(const unsigned* B, int bins, int
     float lcost = kInf;
     int lsplit = 0x7fffffff, lleft = 0;
     // plane after bin 2l (valid when 2l <= bins - 2)
+    // a cost that is NaN (an infinite extent beside a flat one) is no candidate: lanes holding one
+    // would end the reduction with planes of their own
     if (2 * lane <= bins - 2 && l0c != 0 && l0c != count) {
-        lcost = half_area(l0lo, l0hi) * static_cast<float>(l0c) +
-                half_area(r1lo, r1hi) * static_cast<float>(count - l0c);
-        lsplit = 2 * lane + 1;
-        lleft = l0c;
+        const float c1 = half_area(l0lo, l0hi) * static_cast<float>(l0c) +
+                         half_area(r1lo, r1hi) * static_cast<float>(count - l0c);
+        if (c1 < lcost) {
+            lcost = c1;
+            lsplit = 2 * lane + 1;
+            lleft = l0c;
+        }
     }
     if (2 * lane + 1 <= bins - 2 && l1c != 0 && l1c != count) {
         const float c2 = half_area(l1lo, l1hi) * static_cast<float>(l1c) +
@@ -794,7 +799,8 @@ __device__ void warp_build(int* perm, const float4* sc, const float4* slo, const
     const float4 cc = sc[li], blo = slo[li], bhi = shi[li];
     int ord[3];
     for (int a = 0; a < 3; ++a) {
-        const float key = mine ? (a == 0 ? cc.x : (a == 1 ? cc.y : cc.z)) : kInf;
+        float key = mine ? (a == 0 ? cc.x : (a == 1 ? cc.y : cc.z)) : kInf;
+        if (key != key) key = kInf;  // a NaN has a rank too: the ranks are a permutation
         int rank = 0;
         for (int j = 0; j < c; ++j) {  // c is warp-uniform: only the piece's lanes are ranked
             const float kj = __shfl_sync(0xffffffffu, key, j);

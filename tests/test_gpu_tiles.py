@@ -276,3 +276,30 @@ def test_radius_fill_needs_only_the_offsets(cuda, flags, count):
                        "qk_radius_fill")
             cuda.cuda.synchronize()
             assert np.array_equal(keys.cpu().numpy().view(np.uint64)[:total], wkeys), (flags, r)
+
+
+@pytest.mark.parametrize("builder", ["sah", "sah4"])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf, 1e25, 3e38])
+@pytest.mark.parametrize("n", [40, 256, 257, 700, 9000])
+def test_sah_of_coordinates_that_are_not_finite(cuda, builder, bad, n):
+    """NaN has no rank and an infinite extent no area: every primitive still gets one slot, every
+    node one parent, and the build repeats."""
+    pts = workloads.point_cloud("volume", n, 3).copy()
+    pts[::5, 0] = bad
+    pts[1::11, 2] = -bad
+    pts[:2] = bad
+    tris = workloads.terrain(int(np.sqrt(n / 2)) + 2, 4).copy()
+    tris[::3, 3] = bad
+    tris[1::7] = bad
+    for kind, items in (("point", pts), ("tri", tris)):
+        t = capi.DeviceTree(kind, items, builder=builder)
+        m = len(items)
+        assert np.array_equal(np.sort(t.host("prim_ids", np.int32)), np.arange(m))
+        parent = t.host("parent", np.int32)
+        nodes = t.nodes_bytes().view(np.int32).reshape(-1, 8)[: m - 1, 6:]
+        assert np.array_equal(np.sort(nodes.reshape(-1)), np.arange(1, 2 * m - 1))
+        assert np.array_equal(parent[nodes[:, 0]], np.arange(m - 1))
+        assert np.array_equal(parent[nodes[:, 1]], np.arange(m - 1))
+        first = t.nodes_bytes().tobytes()
+        t.build()
+        assert t.nodes_bytes().tobytes() == first
