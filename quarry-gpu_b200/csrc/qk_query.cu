@@ -14,6 +14,7 @@
 // of the inputs: the sorted permutation is handed to the traversal, thread i works on item
 // order[i] and writes its result in place.
 #include <algorithm>
+#include <type_traits>
 
 #include "qk_internal.cuh"
 #include "qk_traverse.cuh"
@@ -1370,16 +1371,22 @@ inline int split_lanes(unsigned flags) {
 
 // Few queries, no schedule asked for, binary nodes: groups of 4 lanes instead of one thread per
 // query (8 for 5 to 8 neighbours, to half as many queries: at 20,000 they win by 12 % on a terrain
-// and lose by 16 % on uniform points), whose latency otherwise leaves most of the GPU idle.  One thread -> groups, us, 8,000 and 32,000 queries: terrain of 131,072 triangles
-// closest 316 -> 182, 349 -> 244, kNN4 413 -> 218, 473 -> 307; 1 M uniform points closest 61 -> 51,
-// 95 -> 95, kNN4 113 -> 80, 152 -> 138, radius (48 found) 384 -> 304, 524 -> 446; 200,000
-// ellipsoids closest 295 -> 143, 321 -> 205.  The gain ends near 32,768 queries on the cheapest
-// tests (points, closest).  Calls that count nodes keep one thread per query (statistics), except
-// radius, whose two passes must agree.
+// and lose by 16 % on uniform points), whose latency otherwise leaves most of the GPU idle.  One
+// thread -> groups, us, 8,000 and 32,000 queries: terrain of 131,072 triangles closest 316 -> 182,
+// 349 -> 244, kNN4 413 -> 218, 473 -> 307; 1 M uniform points closest 61 -> 51, 95 -> 95, kNN4
+// 113 -> 80, 152 -> 138, radius (48 found) 384 -> 304, 524 -> 446.  The gain ends near 32,768
+// queries on the cheapest tests (points, closest).  Closest and kNN calls that count nodes keep one
+// thread per query.  So do those over ellipsoids, whose 14 steps may end nearer than the boxes
+// around them: which of two such primitives is met first then decides (up to 1 query in 1,000 far
+// outside a scene answers differently on groups), and radius alone does not depend on it.
 constexpr int kFewQueries = 32768;
 constexpr unsigned kScheduleFlags = kSplitFlags | QK_WIDE | QK_TUNE_LEAF4 | QK_TUNE_STASH | QK_TUNE_TAIL;
 inline unsigned few_flags(unsigned flags, long long count) {
     return (flags & kScheduleFlags) == 0 && count <= kFewQueries ? flags | QK_TUNE_SPLIT4 : flags;
+}
+template <class Ops>
+inline unsigned few_nearest_flags(unsigned flags, long long count, bool stats) {
+    return stats || std::is_same<Ops, GaussOps>::value ? flags : few_flags(flags, count);
 }
 
 template <class Ops, bool kStats>
@@ -1427,7 +1434,7 @@ int closest_impl(const qk_tree* t, const float* pts, int count, uint2* out, unsi
     const int g = blocks_for(static_cast<long long>(count) << sp, qb);
     const bool wide = (flags & QK_WIDE) != 0;
     const bool st = stats != nullptr;
-    if (!st) flags = few_flags(flags, count);
+    flags = few_nearest_flags<Ops>(flags, count, st);
     if (tail.count) {
         // budgeted traversal (binary nodes, thread or warp per query), then the shared scan
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
@@ -1524,7 +1531,7 @@ int knn_impl(const qk_tree* t, const float* pts, int count, int k, int stride, u
              unsigned flags, unsigned long long* stats, const uint32_t* order, cudaStream_t s,
              const TailList& tail = TailList{}) {
     const bool wide = (flags & QK_WIDE) != 0;
-    if (!stats && k <= 8) flags = few_flags(flags, (k <= 4 ? 1ll : 2ll) * count);
+    if (k <= 8) flags = few_nearest_flags<Ops>(flags, (k <= 4 ? 1ll : 2ll) * count, stats != nullptr);
     const int split = split_lanes(flags);  // 0: one thread per query
     const bool leaf4 = (flags & QK_TUNE_LEAF4) != 0;
     if (tail.count) {

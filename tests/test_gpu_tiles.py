@@ -303,3 +303,19 @@ def test_sah_of_coordinates_that_are_not_finite(cuda, builder, bad, n):
         first = t.nodes_bytes().tobytes()
         t.build()
         assert t.nodes_bytes().tobytes() == first
+
+
+@pytest.mark.parametrize("builder", ["lbvh", "sah"])
+@pytest.mark.parametrize("smin,smax", [(0.05, 3.0), (0.01, 30.0)])
+def test_few_queries_on_ellipsoids_answer_as_many_do(cuda, builder, smin, smax):
+    """Far from the scene a computed distance can be nearer than the boxes around its ellipsoid, so
+    results depend on the visit order: a small batch without a schedule flag keeps the order of
+    one thread per query."""
+    g = workloads.gaussians(700, smin, smax, 5)
+    t = capi.DeviceTree("gauss", g, builder=builder)
+    rng = np.random.default_rng(7)
+    for far in (1e3, 1e6, 1e8):
+        q = _dev(rng.uniform(-far, far, (16_000, 3)).astype(np.float32))
+        many = cuda.cat([q, q, q])  # 48,000
+        for op in (lambda p: t.closest(p), lambda p: t.knn(p, 3), lambda p: t.knn(p, 8)):
+            assert cuda.equal(op(q), op(many)[: len(q)]), far
