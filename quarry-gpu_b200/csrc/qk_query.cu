@@ -802,7 +802,7 @@ __device__ __forceinline__ int split_query(int count, const uint32_t* order, boo
     return valid ? (order ? static_cast<int>(order[w]) : w) : 0;
 }
 
-template <class Ops, bool kStats, int G>
+template <class Ops, bool kStats, int G, bool kFirst = false>
 __global__ __launch_bounds__(kBlock) void k_closest_split(const BNode* __restrict__ bn,
                                                          const float4* __restrict__ leaves,
                                                          const float* __restrict__ pts,
@@ -818,7 +818,7 @@ __global__ __launch_bounds__(kBlock) void k_closest_split(const BNode* __restric
     const int q = split_query<G>(count, order, valid, lane);
     const float3 p = f3(pts[3 * q], pts[3 * q + 1], pts[3 * q + 2]);
     Trav tv;
-    const uint2 r = closest_split_one<Ops, G>(bn, leaves, p, lane, max_iter, tv, valid);
+    const uint2 r = closest_split_one<Ops, G, kFirst>(bn, leaves, p, lane, max_iter, tv, valid);
     if (valid && lane == 0) out[q] = r;
     const bool ovf = group_any<G>(tv.overflow);
     if (tail.count && valid && ovf && lane == 0) tail_append(tail, q);
@@ -1434,7 +1434,17 @@ int closest_impl(const qk_tree* t, const float* pts, int count, uint2* out, unsi
     const int g = blocks_for(static_cast<long long>(count) << sp, qb);
     const bool wide = (flags & QK_WIDE) != 0;
     const bool st = stats != nullptr;
-    flags = few_nearest_flags<Ops>(flags, count, st);
+    if constexpr (!std::is_same<Ops, GaussOps>::value) {
+        if (few_nearest_flags<Ops>(flags, count, st) != flags) {
+            // no schedule asked for: the answers of one thread per query, NaN included
+            const int sb = split_block(count, 4);
+            k_closest_split<Ops, false, 4, true><<<blocks_for(4ll * count, sb), sb, 0, s>>>(
+                static_cast<const BNode*>(t->bnodes), leaves, pts, order, count, out, t->n * 2 + 64,
+                nullptr);
+            const cudaError_t e = cudaGetLastError();
+            return e == cudaSuccess ? QK_OK : cuda_status(e, "closest");
+        }
+    }
     if (tail.count) {
         // budgeted traversal (binary nodes, thread or warp per query), then the shared scan
         const BNode* bn = static_cast<const BNode*>(t->bnodes);

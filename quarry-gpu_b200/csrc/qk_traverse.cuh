@@ -1178,19 +1178,19 @@ __device__ __forceinline__ void warp_min_lex(float& d, int& id) {
 
 // Forced descent of lane `lane` from the root: returns the subtree root the lane owns (an
 // internal node) or -1; a leaf met on the way is handed to `on_leaf` by its owning lane.
-// `keep(box)` decides whether a child box can still hold a result.
-template <int kLevels = kSplitLevels, class Leaf, class Keep>
+// `keep(box)` decides whether a child box can still hold a result; `on_child(node, right)` sees
+// every node the lane passes and the side it takes there.
+template <int kLevels = kSplitLevels, class Leaf, class Keep, class Child>
 __device__ __forceinline__ int split_descend(const BNode* __restrict__ bn, int lane, Leaf on_leaf,
-                                             Keep keep) {
+                                             Keep keep, Child on_child) {
     int node = 0;
     for (int d = 0; d < kLevels; ++d) {
-        float3 llo, lhi, rlo, rhi;
-        int lref, rref;
-        load_bnode(bn, node, llo, lhi, rlo, rhi, lref, rref);
+        const NodePair nd = load_pair(bn, node);
         const bool right = ((lane >> d) & 1) != 0;
-        const int ref = right ? rref : lref;
-        const float3 lo = right ? rlo : llo;
-        const float3 hi = right ? rhi : lhi;
+        const int ref = right ? nd.rref : nd.lref;
+        const float3 lo = boxq_lo(right ? nd.r : nd.l);
+        const float3 hi = boxq_hi(right ? nd.r : nd.l);
+        on_child(nd, right);
         if (ref < 0) {
             if ((lane >> (d + 1)) == 0 && keep(lo, hi)) on_leaf(~ref);
             return -1;
@@ -1200,26 +1200,57 @@ __device__ __forceinline__ int split_descend(const BNode* __restrict__ bn, int l
     }
     return node;
 }
+template <int kLevels = kSplitLevels, class Leaf, class Keep>
+__device__ __forceinline__ int split_descend(const BNode* __restrict__ bn, int lane, Leaf on_leaf,
+                                             Keep keep) {
+    return split_descend<kLevels>(bn, lane, on_leaf, keep, [](const NodePair&, bool) {});
+}
 
-template <class Ops, int G = 32>
+// kFirst: one thread per query takes the first leaf it meets whatever its distance, so a NaN there
+// (a query that is not finite, or a triangle with a = b) is its answer; a NaN met later is never
+// closer.  The lane whose subtree holds that leaf then keeps to the one-thread path down to it,
+// unpruned, and a NaN there is the group's answer too.
+template <class Ops, int G = 32, bool kFirst = false>
 __device__ __forceinline__ uint2 closest_split_one(const BNode* __restrict__ bn,
                                                    const float4* __restrict__ leaves, float3 p,
                                                    int lane, int max_iter, Trav& tv,
                                                    bool valid = true) {
     float best = kInf;
     int best_id = 0x7fffffff;
+    bool first = kFirst;   // this lane is on the one-thread path and that has met no leaf
+    float first_d = 0.0f;  // NaN: the answer is first_id
+    int first_id = 0;
     auto on_leaf = [&](int slot) {
         ++tv.leaves;
         int id;
-        const float d2 = Ops::dist2(p, leaves, slot, id, best);
+        const float d2 = Ops::dist2(p, leaves, slot, id, kFirst && first ? kInf : best);
+        if (kFirst && first) {
+            first_d = d2;
+            first_id = id;
+            first = false;
+        }
         if (closer(d2, id, best, best_id)) {
             best = d2;
             best_id = id;
         }
     };
-    int node = valid ? split_descend<log2_lanes(G)>(bn, lane, on_leaf,
-                                                    [](float3, float3) { return true; })
-                     : -1;
+    // a lane leaves the one-thread path when its child is not the one that takes: a leaf before an
+    // internal child, the nearer (left of equals) of two alike
+    auto on_child = [&](const NodePair& nd, bool right) {
+        float dl, dr;
+        dist2_boxq2(vec3q(p), nd.l, nd.r, dl, dr);
+        const bool ll = nd.lref < 0, rl = nd.rref < 0;
+        const bool take_right = ll == rl ? !(dl <= dr) : rl;
+        if (take_right != right) first = false;
+    };
+    int node = -1;
+    if (valid) {
+        if constexpr (kFirst)
+            node = split_descend<log2_lanes(G)>(bn, lane, on_leaf, [](float3, float3) { return true; },
+                                                on_child);
+        else
+            node = split_descend<log2_lanes(G)>(bn, lane, on_leaf, [](float3, float3) { return true; });
+    }
     warp_min_lex<G>(best, best_id);
     const Vec3Q qp = vec3q(p);
     LocalStack<kStack> st;
@@ -1236,8 +1267,8 @@ __device__ __forceinline__ uint2 closest_split_one(const BNode* __restrict__ bn,
                 const int lref = nd.lref, rref = nd.rref;
                 float dl, dr;
                 dist2_boxq2(qp, nd.l, nd.r, dl, dr);
-                bool okl = dl <= best;
-                bool okr = dr <= best;
+                bool okl = dl <= best || (kFirst && first);
+                bool okr = dr <= best || (kFirst && first);
                 const bool lfirst = dl <= dr;
                 const int lslot = okl && lref < 0 ? ~lref : -1, rslot = okr && rref < 0 ? ~rref : -1;
                 int leaf = lfirst ? lslot : rslot, other = lfirst ? rslot : lslot;
@@ -1283,6 +1314,13 @@ __device__ __forceinline__ uint2 closest_split_one(const BNode* __restrict__ bn,
             }
         }
         warp_min_lex<G>(best, best_id);
+    }
+    if constexpr (kFirst) {
+        const unsigned nan = group_bits<G>(__ballot_sync(0xffffffffu, first_d != first_d));
+        const int src = nan ? __ffs(nan) - 1 : 0;
+        const float nd = __shfl_sync(0xffffffffu, first_d, src, G);
+        const int ni = __shfl_sync(0xffffffffu, first_id, src, G);
+        if (nan) return make_uint2(__float_as_uint(nd), static_cast<unsigned>(ni));
     }
     return best_id != 0x7fffffff ? make_uint2(__float_as_uint(best), static_cast<unsigned>(best_id))
                                  : make_uint2(0u, 0xffffffffu);

@@ -319,3 +319,30 @@ def test_few_queries_on_ellipsoids_answer_as_many_do(cuda, builder, smin, smax):
         many = cuda.cat([q, q, q])  # 48,000
         for op in (lambda p: t.closest(p), lambda p: t.knn(p, 3), lambda p: t.knn(p, 8)):
             assert cuda.equal(op(q), op(many)[: len(q)]), far
+
+
+@pytest.mark.parametrize("kind", ["tri", "point"])
+@pytest.mark.parametrize("builder", ["lbvh", "sah"])
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 9, 700])
+def test_few_closest_queries_answer_nan_as_many_do(cuda, kind, builder, n):
+    """Queries that are not finite or overflow, and triangles whose first two corners coincide (on
+    one side of them the distance is NaN): a batch small enough for lane groups answers each
+    query as one thread per query does, which takes the first leaf it meets even when that is NaN."""
+    rng = np.random.default_rng(n)
+    if kind == "tri":
+        items = rng.uniform(0, 10, (n, 9)).astype(np.float32)
+        items[::2, 3:6] = items[::2, 0:3]
+    else:
+        items = rng.uniform(0, 10, (n, 3)).astype(np.float32)
+    q = rng.uniform(-15, 25, (700, 3)).astype(np.float32)
+    for i, bad in enumerate((np.nan, np.inf, -np.inf, 1e10, 1e19, 3e38)):
+        q[i:60:6, i % 3] = bad
+    q[60:64] = np.nan
+    t = capi.DeviceTree(kind, items, builder=builder)
+    many = t.closest(_dev(np.tile(q, (50, 1))))[:len(q)]  # 35,000: one thread per query
+    assert cuda.isnan(many[:, 0].contiguous().view(cuda.float32)).any()
+    stats = cuda.zeros(4, dtype=cuda.int64, device="cuda")
+    assert cuda.equal(t.closest(_dev(q), stats=stats), many)  # counting keeps one thread per query
+    for f in (0, capi.QK_ORDER_MORTON, capi.QK_ORDER_COHERENT):
+        assert cuda.equal(t.closest(_dev(q), f), many), f
+    assert cuda.equal(t.closest(_dev(q[37:38])), many[37:38])
