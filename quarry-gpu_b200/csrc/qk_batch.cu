@@ -927,9 +927,15 @@ int launch_bq(const Q& q, const qk_batch_plan* p, const qk_batch_tune& tune, cud
     a.stats = p->d_stats;
     const size_t smem = static_cast<size_t>(tune.short_stack) * tune.block * 8;
     const int grid = p->sms * tune.blocks_per_sm;
+    // the largest short stacks reach the 48 KB a launch may use by default, and the ray kernels'
+    // static arrays come on top
+    cudaError_t e = cudaSuccess;
+    if (smem > 40 * 1024)
+        e = cudaFuncSetAttribute(k_bq<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024);
+    if (e != cudaSuccess) return cuda_status(e, "batched query shared memory");
     cudaMemsetAsync(p->d_counter, 0, sizeof(int), s);
     k_bq<Q><<<grid, tune.block, smem, s>>>(q, a);
-    const cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     return e == cudaSuccess ? QK_OK : cuda_status(e, "batched query");
 }
 

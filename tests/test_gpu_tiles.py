@@ -346,3 +346,30 @@ def test_few_closest_queries_answer_nan_as_many_do(cuda, kind, builder, n):
     for f in (0, capi.QK_ORDER_MORTON, capi.QK_ORDER_COHERENT):
         assert cuda.equal(t.closest(_dev(q), f), many), f
     assert cuda.equal(t.closest(_dev(q[37:38])), many[37:38])
+
+
+@pytest.mark.parametrize("block,short", [(64, 32), (128, 32), (256, 16), (256, 22), (256, 23), (256, 24)])
+def test_batched_queries_with_the_largest_short_stacks(cuda, block, short):
+    """Every short stack up to 48 KB per block is taken, beside the kernels' own shared arrays."""
+    scenes = [workloads.terrain(k, k) for k in (3, 40, 17)]
+    b = capi.Batch("tri", scenes, wide=True)
+    b.build()
+    b.sync()
+    lo, hi = workloads.bounds_of(scenes[1])
+    rays = workloads.down_rays(900, float(lo[0]), float(hi[0]), float(lo[1]), float(hi[1]), 100.0, 4)
+    pts = workloads.uniform_points(900, lo, hi, 3, 13)
+    counts = np.array([300] * 3, np.int32)
+    refs = [oracle.LBVH("tri", s) for s in scenes]
+    tune = {"block": block, "blocks_per_sm": 2, "short_stack": short, "chunks_per_fetch": 1}
+    want = np.concatenate([r.raycast(rays[300 * i:300 * (i + 1)]) for i, r in enumerate(refs)])
+    near = np.concatenate([r.closest(pts[300 * i:300 * (i + 1)]) for i, r in enumerate(refs)])
+    for flags in (0, capi.QK_WIDE):
+        out = cuda.zeros(900, dtype=cuda.int64, device="cuda")
+        plan = b.plan(capi.QK_OP_RAY, counts, flags=flags)
+        plan.query(_dev(rays), out, tune=tune)
+        assert plan.status()[1] == 0
+        assert np.array_equal(out.cpu().numpy().view(np.uint64), want), flags
+        out = cuda.zeros((900, 2), dtype=cuda.int32, device="cuda")
+        plan = b.plan(capi.QK_OP_CLOSEST, counts, flags=flags)
+        plan.query(_dev(pts), out, tune=tune)
+        assert np.array_equal(out.cpu().numpy().view(np.uint32), near), flags
