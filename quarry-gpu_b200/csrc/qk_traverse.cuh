@@ -301,6 +301,9 @@ struct RayTail {
     unsigned at;  // shared-memory address of this thread's {d.xyz, tmax}
     __device__ __forceinline__ RayTail(float4* slot, const RayPre& r)
         : at(static_cast<unsigned>(__cvta_generic_to_shared(slot))) {
+        // get() does not tell the compiler that it reads the slot: the store stays behind the
+        // reads for the ray before and ahead of those for this one
+        asm volatile("" ::: "memory");
         *slot = make_float4(r.d.x, r.d.y, r.d.z, r.tmax);
         asm volatile("" ::: "memory");
     }
