@@ -1002,12 +1002,11 @@ __global__ __launch_bounds__(kBlock) void k_radius_split(
 // of its subtree in a stash and chain of its own, entry q * kPoolLanes + lane of the pool.  Counts
 // of the lanes go to lane_counts, their sum to counts.
 constexpr int kPoolLanes = 4;
-template <class Ops, bool kStats>
+template <class Ops>
 __global__ __launch_bounds__(kBlock) void k_radius_count_pool_split(
     const BNode* __restrict__ bn, const float4* __restrict__ leaves, const float* __restrict__ pts,
     const uint32_t* __restrict__ order, int count, float r2, int* __restrict__ counts,
-    int* __restrict__ lane_counts, RadiusPool pool, int max_iter,
-    unsigned long long* __restrict__ stats) {
+    int* __restrict__ lane_counts, RadiusPool pool, int max_iter) {
     constexpr int G = kPoolLanes;
     if (static_cast<long long>(blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) / G >= count)
         return;  // whole warps past the last query
@@ -1026,7 +1025,6 @@ __global__ __launch_bounds__(kBlock) void k_radius_count_pool_split(
         lane_counts[v] = found;
         if (lane == 0) counts[q] = total;
     }
-    flush_stats<kStats>(valid, valid ? tv.nodes : 0, valid ? tv.leaves : 0, valid && tv.overflow, stats);
 }
 
 // whether the pool dropped some lane's keys of query q
@@ -1375,8 +1373,8 @@ inline int split_lanes(unsigned flags) {
 // thread -> groups, us, 8,000 and 32,000 queries: terrain of 131,072 triangles closest 316 -> 182,
 // 349 -> 244, kNN4 413 -> 218, 473 -> 307; 1 M uniform points closest 61 -> 51, 95 -> 95, kNN4
 // 113 -> 80, 152 -> 138, radius (48 found) 384 -> 304, 524 -> 446.  The gain ends near 32,768
-// queries on the cheapest tests (points, closest).  Closest and kNN calls that count nodes keep one
-// thread per query.  So do those over ellipsoids, whose 14 steps may end nearer than the boxes
+// queries on the cheapest tests (points, closest).  Calls that count nodes keep one thread per
+// query.  So do closest and kNN over ellipsoids, whose 14 steps may end nearer than the boxes
 // around them: which of two such primitives is met first then decides (up to 1 query in 1,000 far
 // outside a scene answers differently on groups), and radius alone does not depend on it.
 constexpr int kFewQueries = 32768;
@@ -1842,8 +1840,7 @@ int radius_pool_launch(const qk_tree* t, const float* pts, int count, float r2, 
             cudaMemsetAsync(pool.taken, 0, sizeof(int), s);
             const int sb = split_block(count, kPoolLanes);
             const int gs = blocks_for(static_cast<long long>(count) * kPoolLanes, sb);
-            if (stats) k_radius_count_pool_split<Ops, true><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, bufs.lane_counts, pool, it, stats);
-            else k_radius_count_pool_split<Ops, false><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, bufs.lane_counts, pool, it, stats);
+            k_radius_count_pool_split<Ops><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, bufs.lane_counts, pool, it);
         }
     } else if (fill) {
         k_radius_gather<<<blocks_for(static_cast<long long>(count) * 32), kBlock, 0, s>>>(
@@ -1883,7 +1880,8 @@ int radius_count(const qk_tree* t, const float* pts, int count, float r, int* of
         cudaMemsetAsync(offsets, 0, sizeof(int), s);
         return QK_OK;
     }
-    flags = few_flags(flags, count);
+    // statistics are those of one thread per query
+    if (!stats) flags = few_flags(flags, count);
     Carve c{static_cast<char*>(ws)};
     OrderBufs o = carve_order(c, count);
     int* counts = c.take<int>(count);
@@ -1895,12 +1893,18 @@ int radius_count(const qk_tree* t, const float* pts, int count, float r, int* of
     int st = QK_OK;
     const uint32_t* order = make_order(pts, 3, 0, count, flags, o, s, &st);
     if (st != QK_OK) return st;
+    auto* stt = reinterpret_cast<unsigned long long*>(stats);
+    if (pooled && pool.lane_counts && stt) {
+        // the pool's lane groups count nothing: a pass of one thread per query does
+        st = radius_dispatch<false>(t, pts, count, r * r, counts, nullptr, nullptr,
+                                    flags & ~QK_TUNE_STASH, stt, order, s);
+        if (st != QK_OK) return st;
+    }
     if (pooled)
-        st = radius_pool_dispatch(t, pts, count, r * r, counts, nullptr, pool, nullptr, flags,
-                                  reinterpret_cast<unsigned long long*>(stats), order, false, s);
+        st = radius_pool_dispatch(t, pts, count, r * r, counts, nullptr, pool, nullptr, flags, stt,
+                                  order, false, s);
     else
-        st = radius_dispatch<false>(t, pts, count, r * r, counts, nullptr, nullptr, flags,
-                                    reinterpret_cast<unsigned long long*>(stats), order, s);
+        st = radius_dispatch<false>(t, pts, count, r * r, counts, nullptr, nullptr, flags, stt, order, s);
     if (st != QK_OK) return st;
     cudaError_t e = scan_exclusive(counts, offsets, count, true, scan_ws, s);
     if (e != cudaSuccess) return cuda_status(e, "radius scan");

@@ -373,3 +373,46 @@ def test_batched_queries_with_the_largest_short_stacks(cuda, block, short):
         plan = b.plan(capi.QK_OP_CLOSEST, counts, flags=flags)
         plan.query(_dev(pts), out, tune=tune)
         assert np.array_equal(out.cpu().numpy().view(np.uint32), near), flags
+
+
+@pytest.mark.parametrize("kind", ["tri", "point", "gauss"])
+@pytest.mark.parametrize("order", [0, capi.QK_ORDER_MORTON])
+def test_statistics_are_those_of_one_thread_per_query(cuda, kind, order):
+    """Node and leaf counts of a batch small enough for lane groups, against 50 copies of it, which
+    is not; the radius results after a counted pass are those of an uncounted one."""
+    import ctypes
+
+    L = capi.lib()
+    items = {"tri": lambda: workloads.terrain(20, 2), "point": lambda: _points(900, 5, 400),
+             "gauss": lambda: workloads.gaussians(500, 0.5, 10.0, 4)}[kind]()
+    c = items.reshape(len(items), -1)[:, :3]
+    q = workloads.uniform_points(700, c.min(0) - 5, c.max(0) + 5, 9, 13)
+    r = 0.15 * float(np.linalg.norm(c.max(0) - c.min(0)))
+    t, ref = capi.DeviceTree(kind, items), oracle.LBVH(kind, items)
+
+    def radius(p, flags, stats):
+        n = len(p)
+        d, off, total = _dev(p), cuda.empty(n + 1, dtype=cuda.int32, device="cuda"), ctypes.c_int64(0)
+        nb = int(L.qk_radius_workspace_bytes(n, flags))
+        ws = cuda.empty(nb, dtype=cuda.uint8, device="cuda")
+        a = (ctypes.byref(t.t), d.data_ptr(), n, r, off.data_ptr())
+        capi.check(L.qk_radius_count(*a, ctypes.byref(total), flags, stats.data_ptr(), ws.data_ptr(),
+                                     nb, None), "qk_radius_count")
+        keys = cuda.zeros(max(total.value, 1), dtype=cuda.int64, device="cuda")
+        capi.check(L.qk_radius_fill(*a, keys.data_ptr(), flags, ws.data_ptr(), nb, None),
+                   "qk_radius_fill")
+        cuda.cuda.synchronize()
+        return off.cpu().numpy(), keys.cpu().numpy().view(np.uint64)
+
+    many = np.tile(q, (50, 1))
+    ops = [lambda p, s: t.closest(_dev(p), order, stats=s), lambda p, s: t.knn(_dev(p), 4, order, stats=s),
+           lambda p, s: radius(p, order, s), lambda p, s: radius(p, order | capi.QK_TUNE_STASH, s)]
+    woff, wkeys = ref.radius(q, r)
+    for i, op in enumerate(ops):
+        few, all50 = (cuda.zeros(4, dtype=cuda.int64, device="cuda") for _ in range(2))
+        got = op(q, few)
+        op(many, all50)
+        assert few[0] > 0 and all50.tolist() == [50 * x for x in few.tolist()], i
+        if i >= 2:
+            assert np.array_equal(got[0].astype(np.int64), woff)
+            assert np.array_equal(got[1], wkeys)
