@@ -161,8 +161,9 @@ __device__ __forceinline__ BoxQ load_wide_entry(const WideNode* __restrict__ w, 
 }
 
 // The four slots of a 4-wide node with their keys (entry t or squared distance), in registers:
-// a miss or an empty slot holds (+inf, kEmptySlot).  sort() orders them by key with a network
-// of five exchanges; dynamic indexing would put the arrays in local memory.
+// a miss or an empty slot holds (+inf, kEmptySlot).  sort() orders them by key, equal keys in slot
+// order (a query inside several boxes has equal keys, and the first leaf met decides a NaN answer):
+// exchanges of neighbours only, six of them; dynamic indexing would put the arrays in local memory.
 struct WideHits {
     float k0, k1, k2, k3;
     int c0, c1, c2, c3;
@@ -187,8 +188,9 @@ struct WideHits {
     __device__ __forceinline__ void sort() {
         exchange<kRange>(k0, c0, n0, k1, c1, n1);
         exchange<kRange>(k2, c2, n2, k3, c3, n3);
-        exchange<kRange>(k0, c0, n0, k2, c2, n2);
-        exchange<kRange>(k1, c1, n1, k3, c3, n3);
+        exchange<kRange>(k1, c1, n1, k2, c2, n2);
+        exchange<kRange>(k0, c0, n0, k1, c1, n1);
+        exchange<kRange>(k2, c2, n2, k3, c3, n3);
         exchange<kRange>(k1, c1, n1, k2, c2, n2);
     }
     // bit j: slot j holds a leaf

@@ -416,3 +416,58 @@ def test_statistics_are_those_of_one_thread_per_query(cuda, kind, order):
         if i >= 2:
             assert np.array_equal(got[0].astype(np.int64), woff)
             assert np.array_equal(got[1], wkeys)
+
+
+def _closest_wide(wide, wide_ids, items, p):
+    """Closest triangle by the 4-wide nodes (child >= 0 a node, < 0 the leaf of slot ~child): near
+    children first, equal distances in slot order, the first leaf taken whatever its distance."""
+    box = wide.view(np.float32).reshape(-1, 4, 8)
+    child = wide.view(np.int32).reshape(-1, 4, 8)[:, :, 6]
+    best, best_id, stack, leaves = np.float32(np.inf), -1, [(np.float32(0), 0)], 0
+    while stack:
+        key, node = stack.pop()
+        if best_id >= 0 and not key <= best:
+            continue
+        hits = []
+        for s in range(4):
+            if child[node, s] == EMPTY:
+                continue
+            with np.errstate(invalid="ignore", over="ignore"):
+                gap = np.fmax(np.fmax(box[node, s, 0:3] - p, p - box[node, s, 3:6]), np.float32(0))
+                d = gap * gap
+                d = (d[0] + d[1]) + d[2]
+            if best_id < 0 or d <= best:
+                hits.append((d, int(child[node, s])))
+        hits.sort(key=lambda h: h[0])  # stable
+        for d, c in hits:
+            if c < 0 and (best_id < 0 or d <= best):
+                leaves += 1
+                i = int(wide_ids[~c])
+                x = np.float32(oracle.prim_dist2("tri", p, items[i]))
+                if best_id < 0 or x < best or (x == best and i < best_id):
+                    best, best_id = x, i
+        stack += [(d, c) for d, c in reversed(hits) if c >= 0 and (best_id < 0 or d <= best)]
+    return best, best_id, leaves
+
+
+EMPTY = -0x80000000
+
+
+@pytest.mark.parametrize("builder", ["lbvh", "sah"])
+def test_wide_children_at_equal_distance_in_slot_order(cuda, builder):
+    """Overlapping triangles (queries inside many boxes: equal distances), half of them NaN on one
+    side: the answers and the number of leaf tests of a traversal that keeps slot order."""
+    rng = np.random.default_rng(5)
+    items = rng.uniform(0, 10, (300, 9)).astype(np.float32)
+    items[::2, 3:6] = items[::2, 0:3]
+    q = rng.uniform(-2, 12, (150, 3)).astype(np.float32)
+    t = capi.DeviceTree("tri", items, builder=builder)
+    t.build_wide()
+    wide = t.host("wide", np.uint8)[: t.t.wide_count * 128]
+    ids = t.host("prim_ids", np.int32)
+    want = [_closest_wide(wide, ids, items, p) for p in q]
+    stats = cuda.zeros(4, dtype=cuda.int64, device="cuda")
+    got = t.closest(_dev(q), capi.QK_WIDE, stats=stats).cpu().numpy()
+    assert got[:, 1].tolist() == [w[1] for w in want]
+    assert np.array_equal(got[:, 0].copy().view(np.float32), np.array([w[0] for w in want]), equal_nan=True)
+    assert int(stats[1]) == sum(w[2] for w in want)
