@@ -580,6 +580,12 @@ inline int lane_spread(int count) {
 inline int split_block(int count, int lanes) {
     return static_cast<long long>(count) * lanes <= 148 * 2048 ? 64 : kBlock;
 }
+// two-pass radius: a shell's few long queries gain from larger blocks (1 M points on a noisy shell,
+// 20,000 queries, blocks of 64, 128, 256: 4 lanes 2,101, 2,089, 1,979 us; 8 lanes 1,876, 1,834,
+// 1,917; uniform points 4 lanes 419, 425, 424, 8 lanes 381, 388, 387)
+inline int split_radius_block(int count, int lanes) {
+    return lanes == 4 || static_cast<long long>(count) * lanes > 148 * 2048 ? kBlock : 128;
+}
 
 // ---------------------------------------------------------------------------------------
 // heavy-query tail (QK_TUNE_TAIL, point clouds).  A point near the centre of a spherical shell
@@ -1567,7 +1573,7 @@ int radius_launch(const qk_tree* t, const float* pts, int count, float r2, int* 
     if ((flags & kSplitFlags) && !(flags & QK_WIDE)) {
         const BNode* bn = static_cast<const BNode*>(t->bnodes);
         const int lanes = split_lanes(flags);
-        const int sb = split_block(count, lanes);
+        const int sb = split_radius_block(count, lanes);
         const int gs = blocks_for(static_cast<long long>(count) * lanes, sb);
         if (lanes == 4) {
             if (stats) k_radius_split<Ops, kFill, true, 4><<<gs, sb, 0, s>>>(bn, leaves, pts, order, count, r2, counts, offsets, keys, t->n * 2 + 64, stats);

@@ -1525,7 +1525,10 @@ __device__ __forceinline__ uint2 warp_table_entry(const WarpTable& tab) {
                                 : make_uint2(0u, 0xffffffffu);
 }
 
-// radius, split: hands this lane's keys to `sink` and returns their count
+// radius, split: hands this lane's keys to `sink` and returns their count.  Groups of 4 and 8 lanes
+// take scalar box distances and both leaf tests in line, as radius_bin_visit's kFew (1 M points on a
+// noisy shell, 8,000 queries on 4 lanes: 1,879 us packed with one copy of the test, 1,758 this way);
+// whole warps the packed form (20,000 queries: 1,724 against 1,830).
 template <class Ops, int G, class Sink>
 __device__ __forceinline__ int radius_split_visit(const BNode* __restrict__ bn,
                                                   const float4* __restrict__ leaves, float3 p,
@@ -1555,7 +1558,7 @@ __device__ __forceinline__ int radius_split_visit(const BNode* __restrict__ bn,
         const NodePair nd = load_pair(bn, node);
         const int lref = nd.lref, rref = nd.rref;
         float dl, dr;
-        dist2_boxq2(qp, nd.l, nd.r, dl, dr);
+        dist2_boxq2<(G == 32)>(qp, nd.l, nd.r, dl, dr);
         bool okl = dl <= r2;
         bool okr = dr <= r2;
         int leaf = okl && lref < 0 ? ~lref : -1;
@@ -1564,11 +1567,16 @@ __device__ __forceinline__ int radius_split_visit(const BNode* __restrict__ bn,
             leaf = other;
             other = -1;
         }
+        if constexpr (G < 32) {
+            if (leaf >= 0) on_leaf(leaf);
+            if (other >= 0) on_leaf(other);
+        } else {
 #pragma unroll 1
-        while (leaf >= 0) {
-            on_leaf(leaf);
-            leaf = other;
-            other = -1;
+            while (leaf >= 0) {
+                on_leaf(leaf);
+                leaf = other;
+                other = -1;
+            }
         }
         okl = okl && lref >= 0;
         okr = okr && rref >= 0;
