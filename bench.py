@@ -533,13 +533,17 @@ def rays_arm(args, world, rank, local, workload):
     def query(flags, out_t=None):
         return tree.knn(q_d, 8, flags, out=out_t) if city else tree.closest(q_d, flags, out=out_t)
 
-    q_base = (trees["lbvh"].knn(q_d, 8, 0) if city else trees["lbvh"].closest(q_d, 0)).clone()
+    thread = capi.QK_TUNE_THREAD
+    q_base = (trees["lbvh"].knn(q_d, 8, thread) if city else trees["lbvh"].closest(q_d, thread)).clone()
     q_out = torch.empty_like(q_base)
     q_ms_by = {}
     for kname, kf in (("layout_of_rays", best_flags & (capi.QK_WIDE | capi.QK_ORDER_MORTON |
                                                        capi.QK_ORDER_COHERENT)),
                       ("input", 0), ("morton", capi.QK_ORDER_MORTON),
                       ("coherent", capi.QK_ORDER_COHERENT),
+                      ("thread", capi.QK_TUNE_THREAD),
+                      ("thread_morton", capi.QK_TUNE_THREAD | capi.QK_ORDER_MORTON),
+                      ("thread_coherent", capi.QK_TUNE_THREAD | capi.QK_ORDER_COHERENT),
                       ("split", capi.QK_TUNE_SPLIT),
                       ("split_morton", capi.QK_TUNE_SPLIT | capi.QK_ORDER_MORTON),
                       ("split_coherent", capi.QK_TUNE_SPLIT | capi.QK_ORDER_COHERENT),
@@ -966,11 +970,13 @@ def points_arm(args, world, rank, local):
     # Every (cloud, operation) takes its fastest (tree, schedule): the sphere shell's queries
     # have a heavy tail that the warp-per-query kernels spread out, the uniform cloud's do not.
     # All candidates must return the bits of the LBVH thread-per-query run.
-    variants = {"bin": 0, "bin_morton": capi.QK_ORDER_MORTON, "wide": capi.QK_WIDE,
+    thread = capi.QK_TUNE_THREAD
+    variants = {"auto": 0, "auto_morton": capi.QK_ORDER_MORTON, "auto_coh": capi.QK_ORDER_COHERENT,
+                "bin": thread, "bin_morton": thread | capi.QK_ORDER_MORTON, "wide": capi.QK_WIDE,
                 "wide_morton": capi.QK_WIDE | capi.QK_ORDER_MORTON,
                 "split": capi.QK_TUNE_SPLIT, "split_morton": capi.QK_TUNE_SPLIT | capi.QK_ORDER_MORTON,
                 "leaf4": capi.QK_TUNE_LEAF4, "leaf4_morton": capi.QK_TUNE_LEAF4 | capi.QK_ORDER_MORTON,
-                "bin_coh": capi.QK_ORDER_COHERENT, "split_coh": capi.QK_TUNE_SPLIT | capi.QK_ORDER_COHERENT,
+                "bin_coh": thread | capi.QK_ORDER_COHERENT, "split_coh": capi.QK_TUNE_SPLIT | capi.QK_ORDER_COHERENT,
                 "split8": capi.QK_TUNE_SPLIT8, "split8_coh": capi.QK_TUNE_SPLIT8 | capi.QK_ORDER_COHERENT,
                 "split4": capi.QK_TUNE_SPLIT4, "split4_coh": capi.QK_TUNE_SPLIT4 | capi.QK_ORDER_COHERENT,
                 "leaf4_coh": capi.QK_TUNE_LEAF4 | capi.QK_ORDER_COHERENT}
@@ -986,7 +992,7 @@ def points_arm(args, world, rank, local):
     vms, plan = {}, {}
     for kind, c in clouds.items():
         for op in ops:
-            run(kind, op, c["trees"]["lbvh"], 0)
+            run(kind, op, c["trees"]["lbvh"], thread)
             base = snapshot((kind, op))
             cands = ({**variants, **radius_variants} if op == "radius" else
                      {**variants, **tail_variants})
@@ -1038,7 +1044,8 @@ def points_arm(args, world, rank, local):
 
     def kernel_of(op, vname):
         f = variants[vname]
-        split = f & (capi.QK_TUNE_SPLIT | capi.QK_TUNE_SPLIT8 | capi.QK_TUNE_SPLIT4)
+        split = (f & (capi.QK_TUNE_SPLIT | capi.QK_TUNE_SPLIT8 | capi.QK_TUNE_SPLIT4)
+                 or vname.startswith("auto"))
         return ("k_%s_wide" if f & capi.QK_WIDE else "k_%s_split" if split else "k_%s_bin") % op
 
     roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": pk["hbm_gbs"],
@@ -1699,8 +1706,8 @@ KERNEL_CASES = {
                  "k_warp_tasks, k_sah_leaves, k_bottom_up_ranged)",
     "refit": "full and 1% dirty refit of the volume cloud's LBVH (k_refit_leaves, k_bottom_up, "
              "k_dirty_mark, k_dirty_merge)",
-    "closest_tri": "20,000 closest-point queries on the terrain's LBVH, 131,072 triangles, without "
-                   "a schedule flag and with 4 lanes per query (k_closest_split both)",
+    "closest_tri": "20,000 closest-point queries on the terrain's LBVH, 131,072 triangles, one "
+                   "thread per query (k_closest_bin) and 4 lanes per query (k_closest_split)",
     "closest_gauss": "262,144 closest-ellipsoid queries on 1,048,576 Gaussians (k_closest_bin)",
     "knn_points": "kNN k=8, 20,000 queries on each 1,048,576-point cloud (k_knn_split: a warp "
                   "per query on the sphere shell's SAH tree in coherent order, then 8 lanes per "
@@ -1755,7 +1762,7 @@ def kernel_case(args):
         t2 = capi.DeviceTree("tri", cfg.tris)
         qd = dev(cfg.queries, np.float32)
         for _ in range(2):
-            t2.closest(qd, 0)
+            t2.closest(qd, capi.QK_TUNE_THREAD)
             t2.closest(qd, capi.QK_TUNE_SPLIT4)
     elif name == "closest_gauss":
         g = capi.DeviceTree("gauss", w.gaussians(1_048_576, 0.05, 1.0, 1))

@@ -62,15 +62,19 @@ extern "C" {
                                     a Morton key of at most 15 bits over origin and direction
                                     (rays) or position (queries); same results as input order;
                                     batches under 64 keep input order */
-/* tuning flags (same results, different schedules; chosen by the autotuner) */
+/* tuning flags (same results, different schedules; chosen by the autotuner).  Without one of
+   QK_WIDE, QK_TUNE_THREAD, SPLIT*, LEAF4, STASH and TAIL, batches of up to 32,768 closest, kNN
+   (k <= 4; to 16,384 for k <= 8) and radius queries run with 4 (8) lanes per query, since one
+   thread each would leave most of the GPU idle; closest and kNN over ellipsoids do not. */
 #define QK_TUNE_DYNAMIC 256u     /* persistent warps fetching new rays as lanes finish */
 #define QK_TUNE_HIGH_OCC 512u    /* register cap for 5 resident blocks of 256 per SM */
 #define QK_TUNE_SHORT_STACK 2048u /* binary rays: top 8 stack entries per thread in shared memory */
 #define QK_TUNE_LEAF4 4096u      /* binary nodes: child subtrees of 2..4 primitives are tested
                                     as leaves (skips their inner boxes) */
-#define QK_TUNE_STASH 8192u     /* single-pass radius (binary nodes, one thread per query;
-                                    batched plans on 4-wide nodes too; ignored with
-                                    QK_TUNE_SPLIT): the count pass keeps every key it finds -- a
+#define QK_TUNE_STASH 8192u     /* single-pass radius (binary nodes, one thread per query, or 4
+                                    lanes each for up to 32,768 queries without QK_TUNE_LEAF4
+                                    and QK_TUNE_THREAD; batched plans on 4-wide nodes too; ignored
+                                    with QK_TUNE_SPLIT): the count pass keeps every key it finds -- a
                                     query's first 16 in its stash, the rest in chained 32-key
                                     chunks of a pool of 128 keys per query in the workspace --
                                     and the fill pass copies them, traversing again only the
@@ -83,6 +87,8 @@ extern "C" {
                                     GPU); kNN takes at least the next group size >= k (k > 8:
                                     a warp) */
 #define QK_TUNE_SPLIT4 65536u    /* the same with 4 lanes per query (kNN: at least k lanes) */
+#define QK_TUNE_THREAD 131072u   /* closest / kNN / radius on binary nodes: one thread per query
+                                    whatever the batch's size */
 #define QK_TUNE_TAIL 16384u      /* closest / kNN on point clouds, binary nodes (thread or warp
                                     per query): a query still traversing after a step budget is
                                     answered by a brute-force scan over all points that every
@@ -273,7 +279,9 @@ int qk_raycast_mapped(const qk_tree* tree, const void* host_rays, int count, uin
 
 /* Closest primitive per query point (closestPointGPU / closestVertexGPU /
  * closestGaussianGPU, src/gpu/gpu_bvh.h:283-330).  points: count x 3 floats; out: count
- * query results. */
+ * query results.  stats (here, in qk_knn and in qk_radius_count; nullable, device, 4 uint64,
+ * accumulated): node tests, primitive tests, stack overflows, heavy queries of QK_TUNE_TAIL;
+ * without a schedule flag they are those of one thread per query, whatever the batch's size. */
 int qk_closest(const qk_tree* tree, const float* points, int count, void* out, unsigned flags,
                uint64_t* stats, void* workspace, size_t workspace_bytes, void* stream);
 

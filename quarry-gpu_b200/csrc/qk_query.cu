@@ -1384,7 +1384,8 @@ inline int split_lanes(unsigned flags) {
 // around them: which of two such primitives is met first then decides (up to 1 query in 1,000 far
 // outside a scene answers differently on groups), and radius alone does not depend on it.
 constexpr int kFewQueries = 32768;
-constexpr unsigned kScheduleFlags = kSplitFlags | QK_WIDE | QK_TUNE_LEAF4 | QK_TUNE_STASH | QK_TUNE_TAIL;
+constexpr unsigned kScheduleFlags = kSplitFlags | QK_WIDE | QK_TUNE_LEAF4 | QK_TUNE_STASH |
+                                    QK_TUNE_TAIL | QK_TUNE_THREAD;
 inline unsigned few_flags(unsigned flags, long long count) {
     return (flags & kScheduleFlags) == 0 && count <= kFewQueries ? flags | QK_TUNE_SPLIT4 : flags;
 }
@@ -1789,7 +1790,7 @@ bool use_stash(unsigned flags) {
 // lanes per query of the single-pass radius: groups for few queries (one thread -> groups, 8,000 and
 // 32,000 queries on 1 M uniform points, 48 found: 271 -> 223 us, 403 -> 343)
 inline int pool_lanes(unsigned flags, int count) {
-    return !(flags & QK_TUNE_LEAF4) && count <= kFewQueries ? kPoolLanes : 1;
+    return !(flags & (QK_TUNE_LEAF4 | QK_TUNE_THREAD)) && count <= kFewQueries ? kPoolLanes : 1;
 }
 
 // the pool of the single-pass radius and, with lane groups, the lanes' counts: a stash and a chain

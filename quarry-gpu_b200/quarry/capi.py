@@ -28,6 +28,7 @@ QK_TUNE_STASH = 8192
 QK_TUNE_TAIL = 16384
 QK_TUNE_SPLIT8 = 32768
 QK_TUNE_SPLIT4 = 65536
+QK_TUNE_THREAD = 131072
 QK_SCHEDULE_BATCHED, QK_SCHEDULE_LOOP = 0, 1
 QK_OP_RAY, QK_OP_CLOSEST, QK_OP_KNN, QK_OP_RADIUS = 0, 1, 2, 3
 KINDS = {"tri": QK_TRI, "point": QK_POINT, "gauss": QK_GAUSS}

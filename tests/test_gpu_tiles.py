@@ -471,3 +471,31 @@ def test_wide_children_at_equal_distance_in_slot_order(cuda, builder):
     assert got[:, 1].tolist() == [w[1] for w in want]
     assert np.array_equal(got[:, 0].copy().view(np.float32), np.array([w[0] for w in want]), equal_nan=True)
     assert int(stats[1]) == sum(w[2] for w in want)
+
+
+@pytest.mark.parametrize("kind", ["tri", "point", "gauss"])
+def test_one_thread_per_query_on_request(cuda, kind):
+    """QK_TUNE_THREAD: the oracle's results, the counts of a counted call, and the single-pass
+    radius in the layout of one chain per query."""
+    items = {"tri": lambda: workloads.terrain(20, 2), "point": lambda: _points(900, 5, 400),
+             "gauss": lambda: workloads.gaussians(500, 0.5, 10.0, 4)}[kind]()
+    c = items.reshape(len(items), -1)[:, :3]
+    q = workloads.uniform_points(500, c.min(0) - 5, c.max(0) + 5, 9, 13)
+    t, ref = capi.DeviceTree(kind, items), oracle.LBVH(kind, items)
+    r = 0.2 * float(np.linalg.norm(c.max(0) - c.min(0)))
+    woff, wkeys = ref.radius(q, r)
+    th = capi.QK_TUNE_THREAD
+    for f in (th, th | capi.QK_ORDER_MORTON, th | capi.QK_ORDER_COHERENT):
+        assert np.array_equal(t.closest(_dev(q), f).cpu().numpy().view(np.uint32), ref.closest(q)), f
+        for k in (3, 8, 16):
+            assert np.array_equal(t.knn(_dev(q), k, f).cpu().numpy().view(np.uint32), ref.knn(q, k)), f
+        for g in (f, f | capi.QK_TUNE_STASH):
+            off, keys = t.radius(_dev(q), r, g)
+            assert np.array_equal(off.cpu().numpy().astype(np.int64), woff), g
+            assert np.array_equal(keys.cpu().numpy().view(np.uint64), wkeys), g
+    size = capi.lib().qk_radius_workspace_bytes
+    assert size(500, capi.QK_TUNE_STASH | th) < size(500, capi.QK_TUNE_STASH)
+    a, b = (cuda.zeros(4, dtype=cuda.int64, device="cuda") for _ in range(2))
+    t.closest(_dev(q), th, stats=a)
+    t.closest(_dev(q), 0, stats=b)
+    assert cuda.equal(a, b)
