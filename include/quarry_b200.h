@@ -382,6 +382,14 @@ size_t qk_sort_workspace_bytes(int n);
 int qk_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
                   uint32_t* vals_out, int n, int bits, void* workspace, size_t workspace_bytes,
                   void* stream);
+/* The same sort along two paths that few calls take, so that they can be tested: max_polls is the
+ * number of empty reads after which a tile stops waiting for the tiles before it and counts their
+ * keys itself (negative: every tile, at once); wide_states takes the 64-bit tile states of
+ * n >= 2^30 at any n. */
+size_t qk_sort_workspace_bytes_paths(int n, int wide_states);
+int qk_sort_pairs_paths(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
+                        uint32_t* vals_out, int n, int bits, int max_polls, int wide_states,
+                        void* workspace, size_t workspace_bytes, void* stream);
 
 /*
  * ---- Batched scenes (new; quarry has no batched API) ----

@@ -530,16 +530,32 @@ int qk_validate(const qk_tree* tree, const void* items, int32_t* errors, void* w
 
 size_t qk_sort_workspace_bytes(int n) { return n > 0 ? sort_ws_bytes(n) : 0; }
 
+size_t qk_sort_workspace_bytes_paths(int n, int wide_states) {
+    SortPaths paths;
+    paths.wide_states = wide_states != 0;
+    return n > 0 ? sort_ws_bytes(n, paths) : 0;
+}
+
 int qk_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
                   uint32_t* vals_out, int n, int bits, void* workspace, size_t workspace_bytes,
                   void* stream) {
+    return qk_sort_pairs_paths(keys_in, vals_in, keys_out, vals_out, n, bits, SortPaths{}.max_polls,
+                               0, workspace, workspace_bytes, stream);
+}
+
+int qk_sort_pairs_paths(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
+                        uint32_t* vals_out, int n, int bits, int max_polls, int wide_states,
+                        void* workspace, size_t workspace_bytes, void* stream) {
     if (n < 0 || bits < 1 || bits > 32) return fail(QK_ERR_INVALID, "bad n or bits");
     if (n == 0) return QK_OK;
     if (!keys_in || !vals_in || !keys_out || !vals_out) return fail(QK_ERR_INVALID, "NULL buffer");
-    int st = check_ws(workspace, workspace_bytes, sort_ws_bytes(n));
+    SortPaths paths;
+    paths.max_polls = max_polls;
+    paths.wide_states = wide_states != 0;
+    int st = check_ws(workspace, workspace_bytes, sort_ws_bytes(n, paths));
     if (st) return st;
     const cudaError_t e = sort_pairs(keys_in, vals_in, keys_out, vals_out, n, bits, workspace,
-                                     as_stream(stream));
+                                     as_stream(stream), nullptr, false, false, paths);
     return e == cudaSuccess ? QK_OK : cuda_status(e, "sort");
 }
 

@@ -130,7 +130,14 @@ struct Header {
 };
 
 // ---- sort / scan (qk_sort.cu) ----
-size_t sort_ws_bytes(int n);
+// Two paths of the sort that few calls take, which a test asks for: max_polls is the number of
+// empty reads after which a tile counts the earlier keys itself (< 0: every tile does, at once), and
+// wide_states the 64-bit tile states of n >= 2^30.
+struct SortPaths {
+    int max_polls = 1 << 12;
+    bool wide_states = false;
+};
+size_t sort_ws_bytes(int n, const SortPaths& paths = SortPaths{});
 // where a sort left its result
 struct SortedPairs {
     const uint32_t* keys;
@@ -141,10 +148,11 @@ struct SortedPairs {
 // digit p is bits 8p..8p+7), to be followed by sort_pairs(..., counted = true) with the same n and
 // ws.  nullptr: nothing to count (one tile of keys).
 constexpr int kSortRadix = 256, kSortPasses = 4;
-uint32_t* sort_begin(void* ws, int n, cudaStream_t s);
+uint32_t* sort_begin(void* ws, int n, cudaStream_t s, const SortPaths& paths = SortPaths{});
 cudaError_t sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout,
                        int n, int bits, void* ws, cudaStream_t s, SortedPairs* sorted = nullptr,
-                       bool iota = false, bool counted = false);
+                       bool iota = false, bool counted = false,
+                       const SortPaths& paths = SortPaths{});
 size_t scan_ws_bytes(int n);
 // exclusive scan of n ints; writes the total to out[n] when write_total is set
 cudaError_t scan_exclusive(const int* in, int* out, int n, bool write_total, void* ws,

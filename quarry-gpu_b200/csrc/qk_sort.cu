@@ -12,7 +12,8 @@
 //               a tile that has published its own sum), publishes its sums, lays the tile out
 //               in digit order in shared memory and writes every digit's run with consecutive
 //               threads.  Equal digits keep their input order, so the sort is stable.
-// Up to one tile of keys is sorted by one block in one launch (k_rs_small).
+// Up to one tile of keys is sorted by one block in one launch (k_rs_small).  The chained sums are
+// the decoupled look-back of Merrill and Garland (2016), with an end to every wait.
 //
 // A 30-bit sort of 1,048,576 pairs took 24 launches before (a histogram, three scan kernels and
 // a scatter per digit) and takes 5: 143 -> 91 us of kernel time, the cloud's LBVH 361 -> 308 us.
@@ -147,7 +148,6 @@ __global__ __launch_bounds__(kBlock) void k_rs_hist(const uint32_t* __restrict__
 constexpr uint32_t kTileCount = 1;  // the tile's own keys
 constexpr uint32_t kTileSum = 2;    // with those of every tile before it
 constexpr int kLookback = 8;        // tiles read per step
-constexpr int kMaxPolls = 1 << 12;  // empty reads before a block counts the earlier keys itself
 
 template <class S>
 __device__ __forceinline__ S rs_load(const S* p) {
@@ -160,16 +160,17 @@ __device__ __forceinline__ void rs_store(S* p, S v) {
 
 // One digit's pass.  state: tiles x 256 entries of this pass, zero on entry; next_state (null:
 // none) the next pass's, cleared tile by tile here.  Tiles are taken in order from a counter,
-// so every tile a block waits for has started; a wait that still sees nothing after kMaxPolls
+// so every tile a block waits for has started; a wait that still sees nothing after max_polls
 // reads ends by counting the keys before the tile directly, so no block depends on another to
-// finish.  iota: the values are the keys' positions and vin is not read.
+// finish (max_polls < 0: at once).  iota: the values are the keys' positions and vin is not read.
 template <class S>
 __global__ __launch_bounds__(kBlock) void k_rs_pass(const uint32_t* __restrict__ kin,
                                                     const uint32_t* __restrict__ vin,
                                                     uint32_t* __restrict__ kout,
                                                     uint32_t* __restrict__ vout, int n, int pass,
                                                     RsCounts* __restrict__ c, S* state,
-                                                    S* __restrict__ next_state, int iota) {
+                                                    S* __restrict__ next_state, int iota,
+                                                    int max_polls) {
     __shared__ RsTile sh;
     __shared__ uint32_t gbase[kRadix];
     __shared__ int tile_s;
@@ -177,7 +178,7 @@ __global__ __launch_bounds__(kBlock) void k_rs_pass(const uint32_t* __restrict__
     const int d = threadIdx.x, lane = d & 31, warp = d >> 5;
     if (d == 0) {
         tile_s = atomicAdd(&c->ticket[pass], 1);
-        late = 0;
+        late = max_polls < 0;
     }
     __syncthreads();
     const int tile = tile_s, shift = 8 * pass;
@@ -200,7 +201,7 @@ __global__ __launch_bounds__(kBlock) void k_rs_pass(const uint32_t* __restrict__
     int all;
     const uint32_t start = static_cast<uint32_t>(block_excl_scan(static_cast<int>(total), &all));
     uint32_t before = 0;
-    int t = tile - 1, polls = 0;
+    int t = max_polls < 0 ? -1 : tile - 1, polls = 0;
     while (t >= 0) {
         S v[kLookback];
 #pragma unroll
@@ -219,7 +220,7 @@ __global__ __launch_bounds__(kBlock) void k_rs_pass(const uint32_t* __restrict__
         }
         if (done) break;
         t -= used;
-        if (used == 0 && ++polls > kMaxPolls) {
+        if (used == 0 && ++polls > max_polls) {
             late = 1;
             break;
         }
@@ -345,34 +346,37 @@ cudaError_t scan_exclusive(const int* in, int* out, int n, bool write_total, voi
 }
 
 // tile states: two passes' worth, each pass clearing the next one's
-inline size_t rs_state_bytes(int n) {
-    return (n < (1 << 30) ? sizeof(uint32_t) : sizeof(uint64_t)) * kRadix *
+inline size_t rs_state_bytes(int n, bool wide) {
+    return (n < (1 << 30) && !wide ? sizeof(uint32_t) : sizeof(uint64_t)) * kRadix *
            static_cast<size_t>(blocks_for(n, kSortTile));
 }
 
-size_t sort_ws_bytes(int n) {
+size_t sort_ws_bytes(int n, const SortPaths& paths) {
     Carve c;
     c.take<RsCounts>(1);
-    c.take<char>(rs_state_bytes(n));
-    c.take<char>(rs_state_bytes(n));
+    c.take<char>(rs_state_bytes(n, paths.wide_states));
+    c.take<char>(rs_state_bytes(n, paths.wide_states));
     return c.used;
 }
 
-uint32_t* sort_begin(void* ws, int n, cudaStream_t s) {
+uint32_t* sort_begin(void* ws, int n, cudaStream_t s, const SortPaths& paths) {
     if (n <= kSortTile) return nullptr;
     Carve c{static_cast<char*>(ws)};
     RsCounts* counts = c.take<RsCounts>(1);
-    const char* state = c.take<char>(rs_state_bytes(n));
+    const size_t bytes = rs_state_bytes(n, paths.wide_states);
+    const char* state = c.take<char>(bytes);
     // the counters and the first pass's states are one run of bytes
-    cudaMemsetAsync(counts, 0, static_cast<size_t>(state - reinterpret_cast<char*>(counts)) + rs_state_bytes(n), s);
+    cudaMemsetAsync(counts, 0, static_cast<size_t>(state - reinterpret_cast<char*>(counts)) + bytes, s);
     return &counts->total[0][0];
 }
 
 template <class S>
 static void rs_launch(const uint32_t* sk, const uint32_t* sv, uint32_t* dk, uint32_t* dv, int n,
-                      int pass, RsCounts* c, char* state, char* next, bool iota, cudaStream_t s) {
+                      int pass, RsCounts* c, char* state, char* next, bool iota, int max_polls,
+                      cudaStream_t s) {
     k_rs_pass<S><<<blocks_for(n, kSortTile), kBlock, 0, s>>>(
-        sk, sv, dk, dv, n, pass, c, reinterpret_cast<S*>(state), reinterpret_cast<S*>(next), iota);
+        sk, sv, dk, dv, n, pass, c, reinterpret_cast<S*>(state), reinterpret_cast<S*>(next), iota,
+        max_polls);
 }
 
 // Sorts (kin, vin) by the low `bits` bits.  Passes alternate between the output pair and the
@@ -385,7 +389,7 @@ static void rs_launch(const uint32_t* sk, const uint32_t* sv, uint32_t* dk, uint
 // 256 tiles on 148 SMs, 16 ranking rounds each, then the earlier tiles' counts.
 cudaError_t sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout,
                        int n, int bits, void* ws, cudaStream_t s, SortedPairs* sorted, bool iota,
-                       bool counted) {
+                       bool counted, const SortPaths& paths) {
     if (n <= 0) return cudaSuccess;
     const int passes = bits <= 0 ? 1 : (bits + 7) / 8;
     if (sorted) *sorted = {kout, vout};
@@ -396,10 +400,10 @@ cudaError_t sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
     Carve c{static_cast<char*>(ws)};
     RsCounts* counts = c.take<RsCounts>(1);
     char* state[2];
-    state[0] = c.take<char>(rs_state_bytes(n));
-    state[1] = c.take<char>(rs_state_bytes(n));
+    state[0] = c.take<char>(rs_state_bytes(n, paths.wide_states));
+    state[1] = c.take<char>(rs_state_bytes(n, paths.wide_states));
     if (!counted) {
-        sort_begin(ws, n, s);
+        sort_begin(ws, n, s, paths);
         k_rs_hist<<<min(blocks_for(n, 4 * kBlock), 148 * 4), kBlock, 0, s>>>(kin, n, passes, counts);
     }
     const uint32_t* sk = kin;
@@ -408,8 +412,8 @@ cudaError_t sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
         uint32_t* dk = (p % 2 == 0) ? kout : const_cast<uint32_t*>(kin);
         uint32_t* dv = (p % 2 == 0) ? vout : const_cast<uint32_t*>(vin);
         char* next = p + 1 < passes ? state[(p + 1) % 2] : nullptr;
-        if (n < (1 << 30)) rs_launch<uint32_t>(sk, sv, dk, dv, n, p, counts, state[p % 2], next, iota && p == 0, s);
-        else rs_launch<uint64_t>(sk, sv, dk, dv, n, p, counts, state[p % 2], next, iota && p == 0, s);
+        const auto launch = n < (1 << 30) && !paths.wide_states ? rs_launch<uint32_t> : rs_launch<uint64_t>;
+        launch(sk, sv, dk, dv, n, p, counts, state[p % 2], next, iota && p == 0, paths.max_polls, s);
         sk = dk;
         sv = dv;
     }

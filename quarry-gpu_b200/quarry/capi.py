@@ -125,6 +125,8 @@ EXPORTS = {
     "qk_raycast_host": (_I, [ctypes.POINTER(QkTree), _P, _I, _P, _P, _P, _I, _U, _P, _SZ, _P, _P,
                              _P, _P]),
     "qk_sort_pairs": (_I, [_P, _P, _P, _P, _I, _I, _P, _SZ, _P]),
+    "qk_sort_workspace_bytes_paths": (_SZ, [_I, _I]),
+    "qk_sort_pairs_paths": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _P, _SZ, _P]),
     "qk_batch_arena_bytes": (_SZ, [_I, _P, _I, _U]),
     "qk_batch_create": (_I, [_PP, _I, _P, _I, _P, _P, _SZ, _U, _P]),
     "qk_batch_build": (_I, [_P, _U, _P]),

@@ -499,3 +499,28 @@ def test_one_thread_per_query_on_request(cuda, kind):
     t.closest(_dev(q), th, stats=a)
     t.closest(_dev(q), 0, stats=b)
     assert cuda.equal(a, b)
+
+
+@pytest.mark.parametrize("n", [4097, 8192, 12289, 70001])
+@pytest.mark.parametrize("bits", [8, 16, 24, 32])
+@pytest.mark.parametrize("spread", [1, 3, 1 << 32])
+@pytest.mark.parametrize("max_polls,wide_states", [(-1, 0), (0, 0), (-1, 1), (4096, 1)])
+def test_sort_paths_few_calls_take(cuda, n, bits, spread, max_polls, wide_states):
+    """Tiles that count the earlier keys themselves (every one, or those whose first read is empty)
+    and 64-bit tile states, after an even and an odd number of passes."""
+    L = capi.lib()
+    rng = np.random.default_rng(n + bits)
+    keys = (rng.integers(0, spread, n, dtype=np.uint64) & ((1 << bits) - 1)).astype(np.uint32)
+    vals = rng.integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32)
+    kin, vin = (_dev(a.view(np.int32), np.int32) for a in (keys, vals))
+    kout, vout = cuda.empty_like(kin), cuda.empty_like(vin)
+    nb = int(L.qk_sort_workspace_bytes_paths(n, wide_states))
+    assert nb >= int(L.qk_sort_workspace_bytes(n))
+    ws = cuda.empty(nb, dtype=cuda.uint8, device="cuda")
+    capi.check(L.qk_sort_pairs_paths(kin.data_ptr(), vin.data_ptr(), kout.data_ptr(), vout.data_ptr(), n,
+                                     bits, max_polls, wide_states, ws.data_ptr(), nb, None),
+               "qk_sort_pairs_paths")
+    cuda.cuda.synchronize()
+    o = np.argsort(keys, kind="stable")
+    assert np.array_equal(kout.cpu().numpy().view(np.uint32), keys[o])
+    assert np.array_equal(vout.cpu().numpy().view(np.uint32), vals[o])
