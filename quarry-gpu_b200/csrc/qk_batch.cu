@@ -261,10 +261,9 @@ __global__ __launch_bounds__(128) void k_bt_top(const BScene* __restrict__ tab,
                                                 const uint32_t* __restrict__ codes_f,
                                                 const uint32_t* __restrict__ ids_f,
                                                 LbvhPending pending) {
-    const int count = min(*pending.count, pending.capacity);
+    const int count = *pending.count;
     for (int i = blockIdx.x * 128 + threadIdx.x; i < count; i += 128 * gridDim.x) {
         const uint2 e = pending.list[i];
-        if (e.x == 0xffffffffu) continue;
         const int2 ch = chunks[e.x / kChunkSpans];
         const int base = ch.y + static_cast<int>(e.x % kChunkSpans) * kLbvhSpan;
         lbvh_climb_out(bt_view(tab[ch.x], codes_f, ids_f), base + static_cast<int>(e.y & 255u),
@@ -810,7 +809,6 @@ int batch_build_impl(qk_batch* b, cudaStream_t s) {
     LbvhPending pending;
     pending.list = reinterpret_cast<uint2*>(idx_s);
     pending.count = &b->d_hdr->list_count[1];
-    pending.capacity = N / 2;
     k_bt_tree<Ops><<<C * kChunkSpans, kLbvhSpan, 0, s>>>(b->d_tab, b->d_chunks, codes, codes_s, carry,
                                                          b->d_hdr, pending);
     k_bt_top<<<blocks_for(16ll * C * kChunkSpans, 128), 128, 0, s>>>(b->d_tab, b->d_chunks, codes,

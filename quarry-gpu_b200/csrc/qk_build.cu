@@ -150,10 +150,9 @@ __global__ __launch_bounds__(kLbvhSpan, 6) void k_lbvh_tree(LbvhView v,
 
 // the listed climbs, one thread each
 __global__ __launch_bounds__(128) void k_lbvh_top(LbvhView v, LbvhPending pending) {
-    const int count = min(*pending.count, pending.capacity);
+    const int count = *pending.count;
     for (int i = blockIdx.x * 128 + threadIdx.x; i < count; i += 128 * gridDim.x) {
         const uint2 e = pending.list[i];
-        if (e.x == 0xffffffffu) continue;
         const int base = static_cast<int>(e.x) * kLbvhSpan;
         lbvh_climb_out(v, base + static_cast<int>(e.y & 255u), base + static_cast<int>(e.y >> 8));
     }
@@ -603,7 +602,6 @@ int build_lbvh(qk_tree* t, const void* items_v, void* ws, cudaStream_t s) {
     LbvhPending pending;
     pending.list = reinterpret_cast<uint2*>(order.vals == idx ? idx_s : idx);
     pending.count = &h->counter;
-    pending.capacity = n / 2;
     k_lbvh_tree<Ops><<<blocks, kLbvhSpan, 0, s>>>(v, carry, h, pending);
     stage_mark(kMarkTopo, s);  // leaves, links and the boxes inside blocks
     if (blocks > 1) k_lbvh_top<<<blocks_for(16ll * blocks, 128), 128, 0, s>>>(v, pending);

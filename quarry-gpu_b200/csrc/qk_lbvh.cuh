@@ -56,11 +56,14 @@ struct LbvhView {
 };
 
 // Climbs left for the second launch: {block of the first launch, first | last slot << 8 inside
-// it}.  A block that finds the list full climbs on itself.
+// it}.  Half an entry per leaf holds them all.  A climb leaves its block toward a node that spans
+// the block's left or right end; the nodes across one end have distinct prefix lengths, of which
+// there are 62 (2..63), and each has at most one child inside the block.  So a block hands over at
+// most 124 climbs (128 entries for 256 leaves), a tree's first block at most 62 and its last, with
+// m leaves, at most min(m, 62), which the first's spare entries cover; a tree of one block none.
 struct LbvhPending {
     uint2* list;
-    int* count;  // zero before the first launch; may pass `capacity`
-    int capacity;
+    int* count;  // zero before the first launch
 };
 
 // block-boundary masks of prefix lengths (see above): to the left of a block's first slot, to
@@ -383,21 +386,9 @@ __device__ __forceinline__ void lbvh_block(const LbvhView& v, int base, const Lb
     if (all == 0) return;
     if (t == 0) sh.bound[0] = atomicAdd(pending.count, static_cast<int>(all));
     __syncthreads();
-    const int first = sh.bound[0];
-    if (first <= pending.capacity - static_cast<int>(all)) {
-        if (on)
-            pending.list[first + static_cast<int>(at)] =
-                make_uint2(static_cast<unsigned>(block), static_cast<unsigned>(l | (r << 8)));
-        return;
-    }
-    // a full list: leave this block's reserved entries empty, and climb once every node the
-    // block hands over is in device memory
-    for (int i = first + t; i < min(first + static_cast<int>(all), pending.capacity); i += kLbvhSpan)
-        pending.list[i] = make_uint2(0xffffffffu, 0u);
-    __threadfence();
-    __syncthreads();
-    if (!on) return;
-    lbvh_climb_out(v, base + l, base + r);
+    if (on)
+        pending.list[sh.bound[0] + static_cast<int>(at)] =
+            make_uint2(static_cast<unsigned>(block), static_cast<unsigned>(l | (r << 8)));
 }
 
 }  // namespace qk
