@@ -569,7 +569,10 @@ inline int query_block(int count) { return count <= 148 * 512 ? 64 : kBlock; }
 // threads within about three quarters of a full GPU.  Every lane -> every 2nd, 4th, 8th, 16th, one
 // ray per warp, us: terrain of 8,192 triangles, 2,048 rays 43, 36, 31, 26, 24, 21, 6,000 rays 43,
 // 37, 30, 27, 25, 35; 131,072 triangles, 12,000 rays 99, 85, 72, 67 and 24,000 rays 104, 89, 77,
-// 116; 48,000 rays 112, 97, 141, 176; city (SAH) 24,000 rays 53, 46, 43, 55.
+// 116; 48,000 rays 112, 97, 141, 176; city (SAH) 24,000 rays 53, 46, 43, 55.  Rays read from and
+// results written to mapped host memory gain too, although a warp's records are then short runs over
+// the link: 2,048, 12,000, 48,000 and 100,000 rays on 8,192 triangles 78 -> 37, 70 -> 45, 95 -> 82,
+// 138 -> 130.
 inline int lane_spread(int count) {
     int s = 5;
     while (s > 0 && (static_cast<long long>(count) << s) > 148 * 768) --s;
@@ -1375,14 +1378,22 @@ inline int split_lanes(unsigned flags) {
 
 // Few queries, no schedule asked for, binary nodes: groups of 4 lanes instead of one thread per
 // query (8 for 5 to 8 neighbours, to half as many queries: at 20,000 they win by 12 % on a terrain
-// and lose by 16 % on uniform points), whose latency otherwise leaves most of the GPU idle.  One
-// thread -> groups, us, 8,000 and 32,000 queries: terrain of 131,072 triangles closest 316 -> 182,
-// 349 -> 244, kNN4 413 -> 218, 473 -> 307; 1 M uniform points closest 61 -> 51, 95 -> 95, kNN4
-// 113 -> 80, 152 -> 138, radius (48 found) 384 -> 304, 524 -> 446.  The gain ends near 32,768
-// queries on the cheapest tests (points, closest).  Calls that count nodes keep one thread per
-// query.  So do closest and kNN over ellipsoids, whose 14 steps may end nearer than the boxes
-// around them: which of two such primitives is met first then decides (up to 1 query in 1,000 far
-// outside a scene answers differently on groups), and radius alone does not depend on it.
+// and lose by 16 % on uniform points).  One thread (its lanes spread, lane_spread) / groups, us, at
+// 1,000, 8,000 and 32,000 queries:
+//   closest  terrain, 131,072 triangles 157 / 241, 183 / 208, 270 / 241; city, 200,000 triangles
+//            75 / 114, 85 / 116, 130 / 138; 1 M uniform points 48 / 70, 68 / 79, 101 / 97; 1 M points
+//            on a noisy shell 493 / 585, 951 / 724, 929 / 777
+//   kNN4     167 / 292, 228 / 254, 373 / 298; 88 / 145, 106 / 159, 165 / 189; 64 / 115, 101 / 120,
+//            149 / 145; 688 / 785, 1,341 / 944, 1,588 / 1,056
+//   radius   at 2,000, 8,000 and 32,000: uniform points 238 / 355, 322 / 367, 493 / 463; shell 1,250 /
+//            1,740, 1,678 / 1,799, 2,184 / 2,116
+// So groups win where queries are long and uneven or fill the GPU, and lose on small even batches;
+// the line was drawn against one thread per query in full warps (terrain closest 316 -> 182 at
+// 8,000), and one at about 4,000 (closest, kNN) and 20,000 (radius) would be the better.
+// QK_TUNE_THREAD asks for one thread.  Calls that count nodes keep one thread per query.  So do
+// closest and kNN over ellipsoids, whose 14 steps may end nearer than the boxes around them: which
+// of two such primitives is met first then decides (up to 1 query in 1,000 far outside a scene
+// answers differently on groups), and radius alone does not depend on it.
 constexpr int kFewQueries = 32768;
 constexpr unsigned kScheduleFlags = kSplitFlags | QK_WIDE | QK_TUNE_LEAF4 | QK_TUNE_STASH |
                                     QK_TUNE_TAIL | QK_TUNE_THREAD;
@@ -1787,8 +1798,10 @@ bool use_stash(unsigned flags) {
     return (flags & QK_TUNE_STASH) && !(flags & (kSplitFlags | QK_WIDE));
 }
 
-// lanes per query of the single-pass radius: groups for few queries (one thread -> groups, 8,000 and
-// 32,000 queries on 1 M uniform points, 48 found: 271 -> 223 us, 403 -> 343)
+// lanes per query of the single-pass radius: groups for few queries.  One thread / groups, us, at
+// 2,000, 8,000, 20,000 and 32,000 queries, 48 found: 1 M uniform points 175 / 279, 250 / 290, 307 /
+// 310, 372 / 339; noisy shell 887 / 1,354, 1,214 / 1,362, 1,403 / 1,383, 1,540 / 1,428 (few_flags says
+// why the line lies where it does)
 inline int pool_lanes(unsigned flags, int count) {
     return !(flags & (QK_TUNE_LEAF4 | QK_TUNE_THREAD)) && count <= kFewQueries ? kPoolLanes : 1;
 }

@@ -76,7 +76,8 @@ struct SplitStack {
 // ---------------------------------------------------------------------------------------
 // 32 bytes as four float pairs through the read-only path, in one 256-bit load or two 128-bit
 // ones.  In a divergent warp every lane reads its own node; the ray kernels keep many warps in
-// flight and gain from half as many load instructions (city, 1 M rays: 475 -> 458 us a step),
+// flight, and half as many load instructions pay where nodes come from L2 (1 M rays, city 479 -> 460
+// us) though not where they come from L1 (terrain 519 -> 528; 2,048 rays 23.4 -> 24.2),
 // while the point queries, a few warps per SM bound by the latency of each step, lose more to
 // the longer load (closest of 20,000 points 69 -> 80 us, radius 149 -> 163).  The 256-bit load
 // needs a 32-byte boundary.
