@@ -1471,7 +1471,9 @@ __device__ __forceinline__ void knn_split_one(const BNode* __restrict__ bn,
                 const NodePair nd = load_pair(bn, node);
                 const int lref = nd.lref, rref = nd.rref;
                 float dl, dr;
-                dist2_boxq2<false>(qp, nd.l, nd.r, dl, dr);
+                // a warp per query keeps the schedulers busy enough for the packed form (city, k 16,
+                // 200,000 queries: 5,550 us with scalar distances, 5,491 packed)
+                dist2_boxq2<(G == 32)>(qp, nd.l, nd.r, dl, dr);
                 const bool lfirst = dl <= dr;
                 bool okl = tab.admits(dl);
                 bool okr = tab.admits(dr);
