@@ -1,7 +1,8 @@
 """Benchmark of the B200 spatial-query engine over its five benchmark configurations.
 
 Default run (`python bench.py`): the city configuration is the headline line and the other
-four ride along on the same JSON line under "configs":
+four ride along on the same JSON line under "configs", each with its value and time (the whole
+record, variants and parity counts included, goes to stderr as one JSON line):
   city     131,072 floorless box buildings (1,310,720 triangles) on a 363 x 362 lot grid,
            1,000,000 rays from a plane 50 units above the tallest roof with cosine-weighted
            downward directions, 20,000 kNN (k=8) queries uniform in the bounds
@@ -1834,7 +1835,31 @@ def all_arm(args, world, rank, local):
                 configs[name] = line
     if rank == 0:
         head["configs"] = configs if configs else "the extra configurations run at N = 1"
-        print(json.dumps(head), flush=True)
+        print(json.dumps(head), file=sys.stderr, flush=True)
+        print(json.dumps(short_line(head)), flush=True)
+
+
+def short_line(head: dict) -> dict:
+    """The line of all configurations in under 3 KB (a caller may keep only the end of the output):
+    the headline's fields, and of every other configuration its value, time and end-to-end rate.
+    Everything else (variants, parity counts, rooflines, tuning) is in the full line on stderr."""
+    line = {k: head[k] for k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step",
+                                 "higher_is_better", "scaling", "vs_baseline", "dtype", "data", "config",
+                                 "gpu_launches") if k in head}
+    line["engine"] = {k: head["engine"][k] for k in ("variant", "l2") if k in head.get("engine", {})}
+    line["clocks"] = {k: v for k, v in head.get("clocks", {}).items() if k != "load"}
+    line["e2e"] = {k: head["e2e"][k] for k in ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step")}
+    line["roofline"] = {k: head["roofline"].get(k) for k in ("bound", "achieved", "peak", "unit", "frac",
+                                                             "peak_kind", "kernel", "kernel_ms")}
+    par = head.get("parity") or {}
+    line["mismatches"] = {k: v["mismatches"] for k, v in par.items() if isinstance(v, dict) and "mismatches" in v}
+    if isinstance(head["configs"], dict):
+        line["configs"] = {name: {**{k: c[k] for k in ("value", "unit", "ms_per_step", "gpu_launches") if k in c},
+                                  **({"e2e": c["e2e"].get("value")} if isinstance(c.get("e2e"), dict) else {})}
+                           for name, c in head["configs"].items()}
+    else:
+        line["configs"] = head["configs"]
+    return line
 
 
 def main():

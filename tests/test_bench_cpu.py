@@ -75,3 +75,33 @@ def test_reference_arm_loads_only_checker_libraries_and_matches_the_config():
     import oracle
 
     assert line["config"] == bench.make_workload(oracle.standalone_workloads(), "city", True, 0)[1]
+
+
+def test_the_line_of_all_configurations_is_short():
+    """The default run's line keeps the fields a reader of the headline needs and fits the last
+    3,000 characters of the output."""
+    sys.path.insert(0, str(ROOT))
+    import bench
+
+    e2e = {"value": 1300.04, "unit": "Mrays/s", "h2d_bytes_per_step": 32000000,
+           "d2h_bytes_per_step": 8000000, "path": "p" * 400, "chunks_ms": {"x" * 40: 1.0}}
+    head = {"metric": bench.METRIC, "value": 2104.36, "unit": "Mrays/s", "n_gpus": 1, "steps": 20,
+            "warmup": 5, "ms_per_step": 0.4752, "higher_is_better": True, "scaling": "weak",
+            "vs_baseline": None, "dtype": "f32", "data": "synthetic", "config": {"workload": "city"},
+            "engine": {"variant": "v", "l2": "flushed", "parallelism": "p" * 300},
+            "variants_ms": {f"variant_{i}": 1.0 for i in range(300)},
+            "clocks": {"sm_mhz": 1965.0, "sm_max_mhz": 1965.0, "reasons": [], "load": "l" * 200},
+            "e2e": e2e, "gpu_launches": 100, "roofline": {"bound": "hbm", "frac": 1.0, "bound_met": "b" * 500},
+            "parity": {"against": "port", "rays": {"checked": 10, "mismatches": 0}},
+            "configs": {n: {"value": 1.0, "unit": "u" * 40, "ms_per_step": 1.0, "e2e": e2e, "checks": "c" * 2000}
+                        for n in ("terrain", "points", "grad", "batch")}}
+    line = bench.short_line(head)
+    assert len(json.dumps(line)) < 3000
+    for key in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better",
+                "scaling", "vs_baseline", "dtype", "data", "config", "clocks", "gpu_launches"):
+        assert key in line, key
+    for key in ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step"):
+        assert line["e2e"][key] == e2e[key]
+    assert set(line["configs"]) == {"terrain", "points", "grad", "batch"}
+    assert line["mismatches"] == {"rays": 0}
+    assert bench.short_line({**head, "configs": "the extra configurations run at N = 1"})["configs"]
